@@ -1,13 +1,16 @@
 // ft_mlp.cu -- BF16 tensor-core MLP for the constitutive surrogate: training
-// data from the plain GOH law, forward / backward GEMMs, Adam, prediction.
+// data from the plain GOH law, training steps, in-loop inference, prediction.
 //
-// GEMMs use the warp-level BF16 tensor-core MMA (m16n8k16, FP32 accumulate)
-// with fused epilogues (bias + SiLU, SiLU derivative); every reduction (bias
-// gradients, the batch dimension of weight gradients) runs in a fixed order,
-// so training is bitwise reproducible.
+// Training runs on tcgen05 (ft_train_tc.cuh); a path of one warp-level MMA
+// GEMM (m16n8k16, FP32 accumulate) per product with fused epilogues is kept as
+// its cross-check.  Every reduction (bias gradients, the batch dimension of
+// weight gradients) runs in a fixed order, so training is bitwise
+// reproducible.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -285,21 +288,6 @@ __global__ void k_predict_combine(long long n, const float *Y, double *Slin, con
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int k = 0; k < 6; ++k) Slin[6 * i + k] += scale[i] * double(Y[i * kMlpOut + k]);
-}
-
-// Adam on the FP32 master parameters, then the BF16 weight copies
-__global__ void k_adam(float *P, const float *G, float *Mo, float *V, int n, float lr, float b1,
-                       float b2, float eps, float c1, float c2, bf16 *Wb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float g = G[i];
-  const float m = b1 * Mo[i] + (1.f - b1) * g;
-  const float v = b2 * V[i] + (1.f - b2) * g * g;
-  Mo[i] = m;
-  V[i] = v;
-  const float p = P[i] - lr * (m / c1) / (sqrtf(v / c2) + eps);
-  P[i] = p;
-  Wb[i] = __float2bfloat16_rn(p);
 }
 
 __global__ void k_to_bf16(const float *P, int n, bf16 *Wb) {
@@ -804,7 +792,13 @@ __global__ void __maxnreg__(128)
                  : "memory");
 }
 
-#include "ft_gemm_tc.cuh"
+#include "ft_train_tc.cuh"
+
+// Adam on the FP32 master parameters and the BF16 weight copies (mma.sync path)
+__global__ void k_adam(float *P, const float *G, float *Mo, float *V, bf16 *Wb, const AdamArgs a) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kMlpParams) adam_update(i, G[i], P, Mo, V, Wb, a);
+}
 
 }  // namespace ftgpu
 
@@ -828,15 +822,17 @@ struct ftgpu_surrogate {
        *dZ3 = nullptr;
   long long adam_t = 0;
   int *derr = nullptr;  // device error word of standalone inference calls
-  float *part = nullptr;  // split-K partial tiles of the weight gradients
-  long long part_cap = 0;
-  int tensor_cores = 1;   // training GEMMs: 1 tcgen05 (k_gemm_tc), 0 mma.sync (k_gemm)
+  // tcgen05 path: transposed operand images per 128-row tile, weight-gradient slices
+  unsigned char *tiles = nullptr;
+  float *part = nullptr;
+  long long cap_tc = 0;
+  int tensor_cores = 1;   // training: 1 tcgen05 (ft_train_tc.cuh), 0 mma.sync (k_gemm)
   std::string err;
   ~ftgpu_surrogate() {
     for (void *p : {(void *)P, (void *)G, (void *)Mo, (void *)V, (void *)Wb, (void *)X, (void *)T,
                     (void *)Z1, (void *)Z2, (void *)Z3, (void *)Y, (void *)rowloss, (void *)loss,
                     (void *)H1, (void *)H2, (void *)H3, (void *)dY, (void *)dZ1, (void *)dZ2,
-                    (void *)dZ3, (void *)derr, (void *)part})
+                    (void *)dZ3, (void *)derr, (void *)tiles, (void *)part})
       if (p) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -867,51 +863,44 @@ int dalloc(T **p, size_t n) {
   return 0;
 }
 
+int sm_count(int device) {
+  int sms = 152;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  return sms;
+}
+
+// Buffers of a batch of B rows for the path in use
 int ensure_batch(ftgpu_surrogate *s, long long B) {
-  if (B <= s->cap) return 0;
   int r = 0;
+  if (s->tensor_cores) {
+    if (B <= s->cap_tc) return 0;
+    s->cap_tc = 0;
+    const long long slices = (B + trn::kSlice - 1) / trn::kSlice;
+    r = dalloc(&s->tiles, (B + 127) / 128 * trn::kTileBytes) |
+        dalloc(&s->part, slices * kMlpParams) | dalloc(&s->Y, B * kMlpOut) |
+        dalloc(&s->rowloss, B) | dalloc(&s->loss, 1);
+    s->cap = 0;  // (Y and rowloss are shared with the other path)
+    if (r) return FTGPU_ERR_ALLOC;
+    s->cap_tc = B;
+    return 0;
+  }
+  if (B <= s->cap) return 0;
+  s->cap = s->cap_tc = 0;
   r |= dalloc(&s->Z1, B * kMlpHid) | dalloc(&s->Z2, B * kMlpHid) | dalloc(&s->Z3, B * kMlpHid);
   r |= dalloc(&s->H1, B * kMlpHid) | dalloc(&s->H2, B * kMlpHid) | dalloc(&s->H3, B * kMlpHid);
   r |= dalloc(&s->dZ1, B * kMlpHid) | dalloc(&s->dZ2, B * kMlpHid) | dalloc(&s->dZ3, B * kMlpHid);
   r |= dalloc(&s->Y, B * kMlpOut) | dalloc(&s->dY, B * kMlpOut) | dalloc(&s->rowloss, B);
   r |= dalloc(&s->loss, 1);
-  // split-K partial tiles of the weight gradients: K slices of 256 rows, tiles <= 128 x 128
-  const long long pc = ((B + 255) / 256) * 128 * 128;
-  if (pc > s->part_cap) {
-    r |= dalloc(&s->part, pc);
-    s->part_cap = pc;
-  }
   if (r) return FTGPU_ERR_ALLOC;
   s->cap = B;
   return 0;
 }
 
-// One training GEMM: on the tensor cores (k_gemm_tc: 128-row tiles, weight
-// gradients split over K in slices of 256 batch rows and summed in slice
-// order), or on the warp-level mma.sync kernel (the cross-check path).
+// One training GEMM of the warp-level mma.sync path (the cross-check)
 template <int EPI>
-int gemm(ftgpu_surrogate *s, cudaStream_t st, const GemmArgs &g) {
-  if (!s->tensor_cores) {
-    dim3 grid((unsigned)((g.M + 63) / 64), (unsigned)((g.N + 31) / 32));
-    k_gemm<EPI><<<grid, 128, 0, st>>>(g);
-    return cudaGetLastError() == cudaSuccess ? 0 : FTGPU_ERR_CUDA;
-  }
-  const int Npad = (g.N + 15) / 16 * 16;
-  if (Npad > 128 || g.M <= 0 || g.K <= 0) return FTGPU_ERR_INPUT;
-  const int mt = (g.M + 127) / 128;
-  int slices = 1, kslice = g.K;
-  if (EPI == kEpiStore && mt == 1 && g.K > 512) {
-    kslice = 256;
-    slices = (g.K + kslice - 1) / kslice;
-    if ((long long)slices * g.M * g.N > s->part_cap) return FTGPU_ERR_INPUT;
-  }
-  k_gemm_tc<EPI><<<dim3((unsigned)mt, (unsigned)slices), tcg::kThreads, tcg::kSmem, st>>>(
-      g, Npad, kslice, slices > 1 ? s->part : nullptr, s->derr);
-  if (slices > 1) {
-    const long long n = (long long)g.M * g.N;
-    k_splitk_reduce<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(s->part, slices, g.M, g.N, g.C,
-                                                                g.scm, g.scn);
-  }
+int gemm(cudaStream_t st, const GemmArgs &g) {
+  dim3 grid((unsigned)((g.M + 63) / 64), (unsigned)((g.N + 31) / 32));
+  k_gemm<EPI><<<grid, 128, 0, st>>>(g);
   return cudaGetLastError() == cudaSuccess ? 0 : FTGPU_ERR_CUDA;
 }
 
@@ -923,27 +912,27 @@ GemmArgs ga(int M, int N, int K, const bf16 *A, long long sam, long long sak, co
   return g;
 }
 
-// forward of B rows of X: Z1/H1, Z2/H2, Z3/H3 and Y
-int forward(ftgpu_surrogate *s, const bf16 *X, long long B) {
+// forward of B rows of X (mma.sync path): Z1/H1, Z2/H2, Z3/H3 and Y
+int forward_mma(ftgpu_surrogate *s, const bf16 *X, long long B) {
   const bf16 *W = s->Wb;
   const float *P = s->P;
   GemmArgs g = ga((int)B, kMlpHid, kMlpIn, X, kMlpIn, 1, W + kOffW0, 1, kMlpIn);
   g.bias = P + kOffB0; g.Z = s->Z1; g.H = s->H1;
-  int r = gemm<kEpiBiasSilu>(s, s->stream, g);
+  int r = gemm<kEpiBiasSilu>(s->stream, g);
   g = ga((int)B, kMlpHid, kMlpHid, s->H1, kMlpHid, 1, W + kOffW1, 1, kMlpHid);
   g.bias = P + kOffB1; g.Z = s->Z2; g.H = s->H2;
-  r |= gemm<kEpiBiasSilu>(s, s->stream, g);
+  r |= gemm<kEpiBiasSilu>(s->stream, g);
   g = ga((int)B, kMlpHid, kMlpHid, s->H2, kMlpHid, 1, W + kOffW2, 1, kMlpHid);
   g.bias = P + kOffB2; g.Z = s->Z3; g.H = s->H3;
-  r |= gemm<kEpiBiasSilu>(s, s->stream, g);
+  r |= gemm<kEpiBiasSilu>(s->stream, g);
   g = ga((int)B, kMlpOut, kMlpHid, s->H3, kMlpHid, 1, W + kOffW3, 1, kMlpHid);
   g.bias = P + kOffB3; g.C = s->Y; g.scm = kMlpOut; g.scn = 1;
-  r |= gemm<kEpiBias>(s, s->stream, g);
+  r |= gemm<kEpiBias>(s->stream, g);
   return r;
 }
 
-// loss and all parameter gradients of one batch (X, T) into G
-int backward(ftgpu_surrogate *s, const bf16 *X, const float *T, long long B) {
+// loss and all parameter gradients of one batch (X, T) into G (mma.sync path)
+int backward_mma(ftgpu_surrogate *s, const bf16 *X, const float *T, long long B) {
   const bf16 *W = s->Wb;
   float *G = s->G;
   cudaStream_t st = s->stream;
@@ -953,34 +942,86 @@ int backward(ftgpu_surrogate *s, const bf16 *X, const float *T, long long B) {
   // layer 3: dW3 = dY^T H3, db3, dZ3 = (dY W3) * silu'(Z3)
   GemmArgs g = ga(kMlpOut, kMlpHid, (int)B, s->dY, 1, kMlpOut, s->H3, kMlpHid, 1);
   g.C = G + kOffW3; g.scm = kMlpHid; g.scn = 1;
-  r |= gemm<kEpiStore>(s, st, g);
+  r |= gemm<kEpiStore>(st, g);
   k_colsum<<<kMlpOut, 256, 0, st>>>(s->dY, B, kMlpOut, G + kOffB3);
   g = ga((int)B, kMlpHid, kMlpOut, s->dY, kMlpOut, 1, W + kOffW3, kMlpHid, 1);
   g.Zp = s->Z3; g.dZ = s->dZ3;
-  r |= gemm<kEpiSiluGrad>(s, st, g);
+  r |= gemm<kEpiSiluGrad>(st, g);
   // layer 2
   g = ga(kMlpHid, kMlpHid, (int)B, s->dZ3, 1, kMlpHid, s->H2, kMlpHid, 1);
   g.C = G + kOffW2; g.scm = kMlpHid; g.scn = 1;
-  r |= gemm<kEpiStore>(s, st, g);
+  r |= gemm<kEpiStore>(st, g);
   k_colsum<<<kMlpHid, 256, 0, st>>>(s->dZ3, B, kMlpHid, G + kOffB2);
   g = ga((int)B, kMlpHid, kMlpHid, s->dZ3, kMlpHid, 1, W + kOffW2, kMlpHid, 1);
   g.Zp = s->Z2; g.dZ = s->dZ2;
-  r |= gemm<kEpiSiluGrad>(s, st, g);
+  r |= gemm<kEpiSiluGrad>(st, g);
   // layer 1
   g = ga(kMlpHid, kMlpHid, (int)B, s->dZ2, 1, kMlpHid, s->H1, kMlpHid, 1);
   g.C = G + kOffW1; g.scm = kMlpHid; g.scn = 1;
-  r |= gemm<kEpiStore>(s, st, g);
+  r |= gemm<kEpiStore>(st, g);
   k_colsum<<<kMlpHid, 256, 0, st>>>(s->dZ2, B, kMlpHid, G + kOffB1);
   g = ga((int)B, kMlpHid, kMlpHid, s->dZ2, kMlpHid, 1, W + kOffW1, kMlpHid, 1);
   g.Zp = s->Z1; g.dZ = s->dZ1;
-  r |= gemm<kEpiSiluGrad>(s, st, g);
+  r |= gemm<kEpiSiluGrad>(st, g);
   // layer 0
   g = ga(kMlpHid, kMlpIn, (int)B, s->dZ1, 1, kMlpHid, X, kMlpIn, 1);
   g.C = G + kOffW0; g.scm = kMlpIn; g.scn = 1;
-  r |= gemm<kEpiStore>(s, st, g);
+  r |= gemm<kEpiStore>(st, g);
   k_colsum<<<kMlpHid, 256, 0, st>>>(s->dZ1, B, kMlpHid, G + kOffB0);
   if (cudaGetLastError() != cudaSuccess) return FTGPU_ERR_CUDA;
   return r;
+}
+
+// Shared-memory sizes of the training kernels above the default limit, once
+// per process and device
+int train_attrs(const ftgpu_surrogate *s) {
+  static std::atomic<bool> done[64];
+  const int d = s->device;
+  if (d >= 0 && d < 64 && done[d].load(std::memory_order_acquire)) return 0;
+  const struct {
+    const void *f;
+    uint32_t bytes;
+  } k[] = {{(const void *)k_train_rows<true>, trn::kSmemRows},
+           {(const void *)k_train_rows<false>, trn::kSmemRows},
+           {(const void *)k_train_dw, trn::kSmemDw}};
+  for (const auto &x : k)
+    SCK(cudaFuncSetAttribute(x.f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x.bytes));
+  if (d >= 0 && d < 64) done[d].store(true, std::memory_order_release);
+  return 0;
+}
+
+// Y of B rows of X
+int forward(ftgpu_surrogate *s, const bf16 *X, long long B) {
+  if (!s->tensor_cores) return forward_mma(s, X, B);
+  int r = train_attrs(s);
+  if (r) return r;
+  const unsigned grid = (unsigned)std::min<long long>((B + 127) / 128, sm_count(s->device));
+  k_train_rows<false><<<grid, trn::kThreads, trn::kSmemRows, s->stream>>>(
+      X, nullptr, B, s->Wb, s->P, s->Y, nullptr, nullptr, s->derr);
+  return cudaGetLastError() == cudaSuccess ? 0 : FTGPU_ERR_CUDA;
+}
+
+// loss and gradients of one batch, then (adam.on) the parameter update
+int train_batch(ftgpu_surrogate *s, const bf16 *X, const float *T, long long B,
+                const AdamArgs &adam) {
+  if (!s->tensor_cores) {
+    int r = forward_mma(s, X, B) | backward_mma(s, X, T, B);
+    if (!r && adam.on)
+      k_adam<<<(kMlpParams + 255) / 256, 256, 0, s->stream>>>(s->P, s->G, s->Mo, s->V, s->Wb, adam);
+    return r ? r : (cudaGetLastError() == cudaSuccess ? 0 : FTGPU_ERR_CUDA);
+  }
+  int r = train_attrs(s);
+  if (r) return r;
+  const int rows = train_slice_rows(B);
+  const int slices = (int)((B + rows - 1) / rows);
+  const unsigned grid = (unsigned)std::min<long long>((B + 127) / 128, sm_count(s->device));
+  k_train_rows<true><<<grid, trn::kThreads, trn::kSmemRows, s->stream>>>(
+      X, T, B, s->Wb, s->P, s->Y, s->rowloss, s->tiles, s->derr);
+  k_train_dw<<<dim3((unsigned)slices, 4), trn::kDwThreads, trn::kSmemDw, s->stream>>>(
+      s->tiles, B, s->part, s->derr);
+  k_train_apply<<<kTrnApplyW + kTrnBiases + 1, 256, 0, s->stream>>>(
+      s->tiles, s->part, s->rowloss, B, slices, s->P, s->G, s->Mo, s->V, s->Wb, s->loss, adam);
+  return cudaGetLastError() == cudaSuccess ? 0 : FTGPU_ERR_CUDA;
 }
 
 }  // namespace
@@ -1003,8 +1044,7 @@ int surrogate_infer(ftgpu_surrogate *s, const uint16_t *X, long long n, float *Y
     }
     attr_set[s->device] = true;
   }
-  int sms = 152;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+  const int sms = sm_count(s->device);
   const long long tiles = (n + 127) / 128;
   const long long grid =
       std::max<long long>(1, std::min<long long>((long long)sms, (tiles + tc::kSlots - 1) / tc::kSlots));
@@ -1028,8 +1068,7 @@ int surrogate_infer_mma(ftgpu_surrogate *s, const uint16_t *X, long long n, floa
       return FTGPU_ERR_CUDA;
     attr_set[s->device] = true;
   }
-  int sms = 152;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+  const int sms = sm_count(s->device);
   const long long tiles = (n + 15) / 16;
   long long grid = std::min<long long>((long long)sms * 2, (tiles + 7) / 8);
   if (grid < 1) grid = 1;
@@ -1155,17 +1194,15 @@ int ftgpu_surrogate_train(ftgpu_surrogate *s, int epochs, int batch, double lr,
     for (long long b = 0; b < nb; ++b) {
       const bf16 *X = s->X + b * batch * kMlpIn;
       const float *T = s->T + b * batch * kMlpOut;
-      r = forward(s, X, batch);
-      r |= backward(s, X, T, batch);
-      if (r) return r;
-      ++s->adam_t;
+      const long long at = s->adam_t + 1;
       // cosine-decayed learning rate over the whole run
-      const double frac = double(s->adam_t) / double(total + 1);
+      const double frac = double(at) / double(total + 1);
       const float lr_t = float(lr * 0.5 * (1.0 + cos(3.141592653589793 * std::min(frac, 1.0))));
       const float b1 = 0.9f, b2 = 0.999f;
-      const float c1 = 1.f - powf(b1, (float)s->adam_t), c2 = 1.f - powf(b2, (float)s->adam_t);
-      k_adam<<<(kMlpParams + 255) / 256, 256, 0, s->stream>>>(s->P, s->G, s->Mo, s->V, kMlpParams,
-                                                              lr_t, b1, b2, 1e-8f, c1, c2, s->Wb);
+      const float c1 = 1.f - powf(b1, (float)at), c2 = 1.f - powf(b2, (float)at);
+      r = train_batch(s, X, T, batch, AdamArgs{1, lr_t, b1, b2, 1e-8f, c1, c2});
+      if (r) return r;
+      s->adam_t = at;
       if (b == nb - 1) {
         float hl = 0.f;
         SCK(cudaMemcpyAsync(&hl, s->loss, 4, cudaMemcpyDeviceToHost, s->stream));
@@ -1262,8 +1299,7 @@ int ftgpu_surrogate_gradient(ftgpu_surrogate *s, long long n, const float *x, co
   SCK(cudaMemcpy(dX, xb.data(), n * kMlpIn * 2, cudaMemcpyHostToDevice));
   SCK(cudaMemcpy(dT, t, n * kMlpOut * 4, cudaMemcpyHostToDevice));
   SCK(cudaMemset(s->derr, 0, sizeof(int)));
-  r = forward(s, dX, n);
-  r |= backward(s, dX, dT, n);
+  r = train_batch(s, dX, dT, n, AdamArgs{});
   SCK(cudaStreamSynchronize(s->stream));
   int e = 0;
   SCK(cudaMemcpy(&e, s->derr, sizeof(int), cudaMemcpyDeviceToHost));
