@@ -17,7 +17,8 @@ OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libftgpu.so")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["ft_elem_f32.cu", "ft_elem_f64.cu", "ft_api.cu", "ft_patches.cpp", "ft_noalloc.cu",
+SOURCES = ["ft_elem_f32.cu", "ft_elem_f64.cu", "ft_hexgp_f32.cu", "ft_hexgp_f64.cu", "ft_api.cu",
+           "ft_patches.cpp", "ft_noalloc.cu",
            "ft_mlp.cu", "ft_meshio.cpp", "ft_vtu.cpp", "ft_probe.cu"]
 
 
@@ -31,7 +32,8 @@ def nvcc():
 # The FP32 element kernels use approximate division / square root (their
 # results are checked against the FP64 oracle at the mixed-mode tolerance);
 # every other translation unit keeps IEEE arithmetic.
-EXTRA = {"ft_elem_f32.cu": ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]}
+_FAST32 = ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]
+EXTRA = {"ft_elem_f32.cu": _FAST32, "ft_hexgp_f32.cu": _FAST32}
 
 
 def _compile(src, verbose):

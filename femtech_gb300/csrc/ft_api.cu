@@ -195,7 +195,9 @@ struct ftgpu_model {
   std::vector<int> node_off;
   std::vector<InstParams> inst;
   bool inst_set = false;
-  int patch_elems = 0;
+  int patch_elems = 0;  // requested (0: default)
+  int pe = 128;         // elements per patch, from choose_patches
+  bool hexgp = false;   // C3D8 groups on the eight-lane pass
   int node_threads = 128;  // nodal block (4M block: 0.834 ms/step against 0.839 at 256)
   bool setup_done = false, init_done = false;
   PatchSet ps;
@@ -328,10 +330,31 @@ void drop_graphs(ftgpu_model *m) {
   m->chunk_steps = m->prof_steps = 0;
 }
 
-int max_patch(const ftgpu_model *m) {
+// Mixed-precision models of at most this many C3D8 elements take the
+// eight-lane element pass (ft_hexgp.cuh).
+constexpr int kHexGpMixedMax = 20000;
+
+// The C3D8 pass and the elements per patch of a model (at set-up).  A given
+// patch size stands (FP64: at most 128).  The default is 128, and less where a
+// block per 128 elements would leave SMs idle or uneven: the FP64 and
+// eight-lane passes are bound by the busiest SM, so their patches are halved
+// until every SM has eight blocks (C3D4, a thread per element: four), down to
+// two warps of eight-lane elements or one of tetrahedra.
+void choose_patches(ftgpu_model *m) {
+  long long nh = 0;
+  for (int t : m->etype) nh += t == FTGPU_C3D8;
+  const long long nt = m->nE - nh;
+  m->hexgp = is_fp64(m) || (nh > 0 && nh <= kHexGpMixedMax);
   int pe = m->patch_elems > 0 ? m->patch_elems : 128;
   if (is_fp64(m)) pe = std::min(pe, 128);
-  return std::max(32, std::min(pe, kMaxPatchElems));
+  pe = std::max(32, std::min(pe, kMaxPatchElems));
+  if (m->patch_elems <= 0 && (is_fp64(m) || (m->hexgp && nt == 0))) {
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
+    const int lo = nt > 0 ? 32 : 8, per_sm = nh > 0 ? 8 : 4;
+    while (pe > lo && m->nE < (long long)per_sm * sms * pe) pe /= 2;
+  }
+  m->pe = pe;
 }
 
 template <class R>
@@ -522,7 +545,7 @@ int launch_node(ftgpu_model *m, int mode, int parity) {
 template <class R>
 int launch_groups_t(ftgpu_model *m, int parity, int use_clock, double dt_direct, int gp,
                     int dt_only) {
-  const int PE = max_patch(m);
+  const int PE = m->pe;
   auto active = [&](size_t gi) {
     return m->ps.groups[gi].npatch > 0 &&
            !(gp != kLaunchGaussPoints && gi < m->group_idle.size() && m->group_idle[gi]);
@@ -557,15 +580,21 @@ int launch_groups_t(ftgpu_model *m, int parity, int use_clock, double dt_direct,
     }
     A.use_clock = use_clock;
     A.dt_direct = dt_direct;
-    const size_t smem = elem_smem_bytes_host<R>(g.etype, PE);
+    // one element pass of this group: eight lanes or one thread per element
+    auto elem = [&](int md, int pass) {
+      return g.etype == 0 && m->hexgp
+                 ? launch_hexgp(g.mat, md, g.npatch, hexgp_threads(PE), hexgp_smem_bytes<R>(PE), st,
+                                A, pass)
+                 : launch_elem<R>(g.etype, g.mat, md, g.npatch, PE,
+                                  elem_smem_bytes_host<R>(g.etype, PE), st, A, pass);
+    };
     if (m->surr && g.mat == 7 && dt_only == kPassForce && sizeof(R) == 4) {
       // surrogate: features of every Gauss point, one fused MLP pass, then
       // the force pass reading the network outputs
       const long long base = m->surr_base[gi];
       const long long ngp = (long long)g.nelem * (g.etype == 0 ? 8 : 1);
       A.surr_x = m->surr_x.as<uint16_t>() + base * kMlpIn;
-      int r = launch_elem<R>(g.etype, g.mat, 0, g.npatch, PE, smem, st, A,
-                             kPassSurrogateFeatures);
+      int r = elem(kLaunchPlain, kPassSurrogateFeatures);
       if (r) return r;
       r = surrogate_infer(m->surr, A.surr_x, ngp, m->surr_y.as<float>() + base * kMlpOut,
                           st, m->err.as<int>());
@@ -573,7 +602,7 @@ int launch_groups_t(ftgpu_model *m, int parity, int use_clock, double dt_direct,
       A.surr_x = nullptr;
       A.surr_y = m->surr_y.as<float>() + base * kMlpOut;
     }
-    int r = launch_elem<R>(g.etype, g.mat, mode, g.npatch, PE, smem, st, A, dt_only);
+    int r = elem(mode, dt_only);
     if (r) return r;
   }
   if (split) {
@@ -753,7 +782,7 @@ __global__ void k_principal_strain(const double *E6, long long nE, double *out) 
 
 template <class R>
 int strain_groups_t(ftgpu_model *m, double *E6) {
-  const int PE = max_patch(m);
+  const int PE = m->pe;
   for (size_t gi = 0; gi < m->ps.groups.size(); ++gi) {
     const PatchGroup &g = m->ps.groups[gi];
     const ElemArgs<R> A = elem_args<R>(m, g, (int)gi);
@@ -913,54 +942,8 @@ int upload_bc(ftgpu_model *m) {
 template <class R>
 int upload_materials(ftgpu_model *m) {
   std::vector<MatP<R>> t(m->nPID);
-  for (int p = 0; p < m->nPID; ++p) {
-    const double *pr = &m->props[FTGPU_MAXMATPARAMS * p];
-    MatP<R> q;
-    memset(&q, 0, sizeof(q));
-    for (int k = 0; k < 9; ++k) q.p[k] = R(pr[k]);
-    const double mu = pr[1], lambda = pr[2], rho = pr[0];
-    q.K = R(lambda + 2.0 * mu / 3.0);
-    // CalculateTimeStep.cpp:16-18
-    const double nu = 0.5 * lambda / (lambda + mu);
-    const double ce = std::sqrt(lambda * (1.0 / nu - 1.0) / rho);
-    q.ce = ce;
-    q.inv_ce = R(1.0 / ce);
-    q.mat = m->materialID[p];
-    if (q.mat == 6) {
-      // binomial coefficients of (1+x)^(alpha/2-1), powers 1..n
-      const double a = pr[3];
-      double ba = 1.0;
-      for (int k = 0; k < kOgdenSeries; ++k) {
-        ba *= (a / 2.0 - 1.0 - k) / (k + 1.0);
-        q.ser_a[k] = R(ba);
-      }
-      // FP32 path: the series while |2E|_F < r, r the largest radius (at most
-      // 0.3) whose truncation bound sum_{k > n} |b_a,k| (3 + 2 r) r^k stays
-      // below 1e-7 r (FP32 rounding of the leading term; the 1 + 2 (1 + r)
-      // weighs A itself and tr B = tr(A + M + M A)); FP64 mode keeps the
-      // eigen path
-      auto tail = [&](double r) {
-        double ca = ba, rk = std::pow(r, kOgdenSeries), t = 0.0;
-        for (int k = kOgdenSeries; k < kOgdenSeries + 400; ++k) {
-          ca *= (a / 2.0 - 1.0 - k) / (k + 1.0);
-          rk *= r;
-          t += std::fabs(ca) * (3.0 + 2.0 * r) * rk;
-        }
-        return t;
-      };
-      double lo = 0.0, hi = 0.3;
-      if (tail(hi) <= 1e-7 * hi) {
-        lo = hi;
-      } else {
-        for (int it = 0; it < 60; ++it) {
-          const double mid = 0.5 * (lo + hi);
-          (tail(mid) <= 1e-7 * mid ? lo : hi) = mid;
-        }
-      }
-      q.ser_thr2 = sizeof(R) == 4 ? R(lo * lo) : R(0);
-    }
-    t[p] = q;
-  }
+  for (int p = 0; p < m->nPID; ++p)
+    t[p] = make_matp<R>(m->materialID[p], &m->props[FTGPU_MAXMATPARAMS * p]);
   return m->mats.upload(t.data(), t.size());
 }
 
@@ -984,7 +967,8 @@ int setup_t(ftgpu_model *m) {
     for (int k = m->eptr[e]; k < m->eptr[e + 1]; ++k)
       if (ninst_of[m->conn[k]] != einst[e]) return fail(FTGPU_ERR_INPUT, "element spans instances");
   }
-  const int PE = max_patch(m);
+  choose_patches(m);
+  const int PE = m->pe;
   int rc = build_patches((int)N, E, m->X.data(), m->eptr.data(), m->conn.data(), m->etype.data(),
                          emat.data(), einst.data(), PE, kMaxLocalNodes, m->ps);
   if (rc) return fail(FTGPU_ERR_INPUT, "invalid mesh (element type / node count / node index)");
@@ -1120,22 +1104,23 @@ int setup_t(ftgpu_model *m) {
   CKI(m->rottrig.alloc((size_t)m->ninst * kMaxRotFns * 3 * sizeof(double)));
   CKI(m->err.alloc(sizeof(int)));
   CK(cudaMemset(m->err.p, 0, sizeof(int)));
-  // FP32: reference geometry of every C3D8 Gauss point, once (the element
-  // passes read it instead of rebuilding A^{-1} from the slot coordinates)
+  // reference geometry of every C3D8 Gauss point, once (the element passes
+  // read it instead of rebuilding A^{-1} from the slot coordinates)
   m->geo.clear();
-  if constexpr (sizeof(R) == 4) {
-    for (size_t gi = 0; gi < ps.groups.size(); ++gi) {
-      const PatchGroup &g = ps.groups[gi];
-      if (g.etype != 0 || g.nelem == 0) {
-        m->geo.emplace_back(nullptr);
-        continue;
-      }
-      auto b = std::make_unique<DBuf>();
-      CKI(b->alloc((size_t)80 * g.nelem * sizeof(float)));
-      m->geo.push_back(std::move(b));
-      const ElemArgs<float> A = elem_args<float>(m, g, (int)gi);
-      CK((cudaError_t)launch_geo_f32(g.npatch, m->stream, A, m->geo.back()->as<float>()));
+  for (size_t gi = 0; gi < ps.groups.size(); ++gi) {
+    const PatchGroup &g = ps.groups[gi];
+    if (g.etype != 0 || g.nelem == 0) {
+      m->geo.emplace_back(nullptr);
+      continue;
     }
+    auto b = std::make_unique<DBuf>();
+    CKI(b->alloc((size_t)80 * g.nelem * sizeof(R)));
+    m->geo.push_back(std::move(b));
+    const ElemArgs<R> A = elem_args<R>(m, g, (int)gi);
+    if (m->hexgp)
+      CK((cudaError_t)launch_hexgp_geo(g.npatch, m->stream, A, m->geo.back()->as<R>()));
+    else if constexpr (sizeof(R) == 4)
+      CK((cudaError_t)launch_geo_f32(g.npatch, m->stream, A, m->geo.back()->as<float>()));
   }
   CKI(fill_dtmin(m));
   // lumped mass on the device (FP64), replaces AssembleLumpedMass()

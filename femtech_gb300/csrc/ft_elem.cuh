@@ -159,11 +159,9 @@ __device__ __forceinline__ void goh_parts_surrogate(const MatP<R> &mp, const R (
   Si = Sym6<R>{Slin[0] + scale * R(sy[0]), Slin[1] + scale * R(sy[1]),
                Slin[2] + scale * R(sy[2]), Slin[3] + scale * R(sy[3]),
                Slin[4] + scale * R(sy[4]), Slin[5] + scale * R(sy[5])};
-  const Sym6<R> ce = two_E(D);
-  const Sym6<R> ac = adj_I_plus(ce);
-  const R J = 1 + Jm1;
-  const R Jp = R(0.5) * mp.K * Jm1 * (2 + Jm1) / (J * J);
-  Sv = sym_scale(ac, Jp);
+  const CGreen<R> g = cgreen(D, Jm1);
+  const R Jp = R(0.5) * mp.K * g.jj;
+  Sv = cg_combine(g, Jp + Jp * g.Ca, Jp * g.Cb, Jp * g.Cg);
 }
 
 // hin: the Gauss point's history already loaded into registers (same order
@@ -930,7 +928,7 @@ template <class R, int ET, int MAT, bool GP, bool INJ>
 // INJ: the force pass also updates the brain drivers' per-step injury
 // criteria of its listed elements (CalculateInjuryCriterions, ex5.cpp:
 // 1311-1430, on the F of this pass) and writes the block's extremes.
-__global__ void __launch_bounds__(kElemThreads, ET == 0 ? 2 : 4)
+__global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 : 4)
     k_elem(const ElemArgs<R> A, int pass) {
   constexpr int NC = ET == 0 ? 8 : 4;
   constexpr int NGP = ET == 0 ? 8 : 1;

@@ -46,13 +46,28 @@ inline int launch_strain<double>(int etype, int nblocks, int threads, size_t sme
 // Returns a cudaError_t value.
 int launch_geo_f32(int nblocks, cudaStream_t s, const ElemArgs<float> &A, float *geo);
 
+// The eight-lane C3D8 pass (ft_hexgp.cuh) and its set-up table ([10][8 nelem])
+int launch_hexgp(int mat, int gp, int nblocks, int threads, size_t smem, cudaStream_t s,
+                 const ElemArgs<float> &A, int pass);
+int launch_hexgp(int mat, int gp, int nblocks, int threads, size_t smem, cudaStream_t s,
+                 const ElemArgs<double> &A, int pass);
+int launch_hexgp_geo(int nblocks, cudaStream_t s, const ElemArgs<float> &A, float *geo);
+int launch_hexgp_geo(int nblocks, cudaStream_t s, const ElemArgs<double> &A, double *geo);
+// its block: eight lanes per element, at most 256 threads; slot records and
+// corner forces in shared memory
+inline int hexgp_threads(int PE) { return PE >= 32 ? 256 : (8 * PE + 31) / 32 * 32; }
+template <class R>
+inline size_t hexgp_smem_bytes(int PE) {
+  return sizeof(R) * (8 * (size_t)kMaxLocalNodes + 24 * (size_t)PE);
+}
+
 // Dynamic shared memory of one element block: node X and u records (4
 // values each) for kMaxLocalNodes slots plus NC*3 corner forces per element, or for FP32
 // C3D8 the larger 80-value geometry record per element in the same space.
 template <class R>
 inline size_t elem_smem_bytes_host(int etype, int PE) {
   const int NC = etype == 0 ? 8 : 4;
-  const size_t per_elem = (etype == 0 && sizeof(R) == 4) ? 80 : (size_t)NC * 3;
+  const size_t per_elem = etype == 0 ? 80 : (size_t)NC * 3;
   const size_t slot_words = etype == 0 ? 8 : 6;  // packed records (C3D8) / component arrays
   return sizeof(R) * (slot_words * (size_t)kMaxLocalNodes + per_elem * PE) +
          (etype == 0 ? elem_csr_smem_bytes(NC, PE) : 0);

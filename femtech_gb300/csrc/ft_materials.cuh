@@ -15,6 +15,9 @@
 
 #include <cuda_runtime.h>
 
+#include <cmath>
+#include <cstring>
+
 namespace ftgpu {
 
 template <class R>
@@ -22,7 +25,21 @@ struct Sym6 {
   R xx, yy, zz, yz, xz, xy;
 };
 
-constexpr int kOgdenSeries = 9;  // terms of the small-strain Ogden series
+// Terms of the small-strain Ogden series: FP32 always sums 9; FP64 the
+// smallest of the listed counts that reaches its rounding at the strain at hand
+template <class R> struct OgdenSeries;
+template <> struct OgdenSeries<float> {
+  static constexpr int kMax = 9, kSteps = 1;
+  static constexpr int n[kSteps] = {9};
+};
+template <> struct OgdenSeries<double> {
+  static constexpr int kMax = 32, kSteps = 5;
+  static constexpr int n[kSteps] = {8, 12, 16, 24, 32};
+};
+// Terms of the binomial series of J^(-alpha/3) in J - 1
+template <class R> struct JPowSeries;
+template <> struct JPowSeries<float> { static constexpr int kMax = 6; };
+template <> struct JPowSeries<double> { static constexpr int kMax = 11; };
 
 template <class R>
 struct MatP {  // per-part material parameters, precomputed on the host
@@ -32,13 +49,87 @@ struct MatP {  // per-part material parameters, precomputed on the host
   double ce;   // dilatational wave speed in FP64
   int mat;     // material ID
   int pad;
-  // Ogden: binomial coefficients binom(alpha/2 - 1, k), k = 1..kOgdenSeries,
-  // and the squared Frobenius bound on 2E below which the series is used
-  // (0 = always the eigen-decomposition; set on the host from the series'
-  // truncation bound for this alpha)
-  R ser_a[kOgdenSeries];
-  R ser_thr2;
+  // Ogden: binomial coefficients binom(alpha/2 - 1, k), k = 1.., and for each
+  // count of terms the largest spectral radius of 2E at which that many reach
+  // the type's rounding (0: never; beyond the last, the eigen-decomposition);
+  // binom(-alpha/3, k) and the largest |J - 1| for their series
+  R og_c;      // 2 mu / alpha
+  R ser_a[OgdenSeries<R>::kMax];
+  float ser_r[OgdenSeries<R>::kSteps];
+  R jpow[JPowSeries<R>::kMax];
+  float jpow_x;
 };
+
+// A part's parameters from the reference's property array (host)
+template <class R>
+inline MatP<R> make_matp(int mat, const double *pr) {
+  MatP<R> q;
+  memset(&q, 0, sizeof(q));
+  for (int k = 0; k < 9; ++k) q.p[k] = R(pr[k]);
+  const double mu = pr[1], lambda = pr[2], rho = pr[0];
+  q.K = R(lambda + 2.0 * mu / 3.0);
+  // CalculateTimeStep.cpp:16-18
+  const double nu = 0.5 * lambda / (lambda + mu);
+  const double ce = std::sqrt(lambda * (1.0 / nu - 1.0) / rho);
+  q.ce = ce;
+  q.inv_ce = R(1.0 / ce);
+  q.mat = mat;
+  if (mat != 6) return q;
+  const double a = pr[3];
+  q.og_c = R(2.0 * mu / a);
+  const double eps = sizeof(R) == 4 ? 1e-7 : 5e-17;
+  double ba = 1.0;
+  int step = 0;
+  for (int k = 0; k < OgdenSeries<R>::kMax; ++k) {
+    ba *= (a / 2.0 - 1.0 - k) / (k + 1.0);
+    q.ser_a[k] = R(ba);
+    const int n = k + 1;
+    if (n != OgdenSeries<R>::n[step]) continue;
+    // n terms while the spectral radius of 2E is below r, r the largest (at
+    // most 0.3 in FP32, 0.5 in FP64) whose truncation bound
+    // sum_{j > n} |b_j| (3 + 2 r) r^j stays below eps r (rounding of the leading
+    // term; the 1 + 2 (1 + r) weighs A itself and tr B = tr(A + M + M A))
+    auto tail = [&](double r) {
+      double ca = ba, rk = std::pow(r, n), t = 0.0;
+      for (int j = n; j < n + 400; ++j) {
+        ca *= (a / 2.0 - 1.0 - j) / (j + 1.0);
+        rk *= r;
+        t += std::fabs(ca) * (3.0 + 2.0 * r) * rk;
+      }
+      return t;
+    };
+    double lo = 0.0, hi = sizeof(R) == 4 ? 0.3 : 0.5;
+    if (tail(hi) <= eps * hi) {
+      lo = hi;
+    } else {
+      for (int it = 0; it < 60; ++it) {
+        const double mid = 0.5 * (lo + hi);
+        (tail(mid) <= eps * mid ? lo : hi) = mid;
+      }
+    }
+    q.ser_r[step++] = float(lo * (1.0 - 1e-6));
+  }
+  // J^(-alpha/3): |J - 1| up to 1/32, less where the tail would show
+  double c = 1.0;
+  const int nj = JPowSeries<R>::kMax;
+  for (int k = 0; k < nj; ++k) {
+    c *= (-a / 3.0 - k) / (k + 1.0);
+    q.jpow[k] = R(c);
+  }
+  auto jtail = [&](double x) {
+    double ca = c, xk = std::pow(x, nj), t = 0.0;
+    for (int k = nj; k < nj + 100; ++k) {
+      ca *= (-a / 3.0 - k) / (k + 1.0);
+      xk *= x;
+      t += std::fabs(ca) * xk;
+    }
+    return t;
+  };
+  double x = 1.0 / 32.0;
+  while (x > 1e-6 && !(jtail(x) <= (sizeof(R) == 4 ? 1e-8 : 2e-17))) x *= 0.5;
+  q.jpow_x = float(x > 1e-6 ? x : 0.0);
+  return q;
+}
 
 template <class R> __device__ __forceinline__ R d_log1p(R x);
 template <> __device__ __forceinline__ float d_log1p<float>(float x) { return log1pf(x); }
@@ -78,19 +169,6 @@ __device__ __forceinline__ Sym6<R> two_E(const R (&D)[3][3]) {
   return e;
 }
 
-// 2e = B - I = D + D^T + D D^T
-template <class R>
-__device__ __forceinline__ Sym6<R> two_e_left(const R (&D)[3][3]) {
-  Sym6<R> e;
-  e.xx = 2 * D[0][0] + (D[0][0] * D[0][0] + D[0][1] * D[0][1] + D[0][2] * D[0][2]);
-  e.yy = 2 * D[1][1] + (D[1][0] * D[1][0] + D[1][1] * D[1][1] + D[1][2] * D[1][2]);
-  e.zz = 2 * D[2][2] + (D[2][0] * D[2][0] + D[2][1] * D[2][1] + D[2][2] * D[2][2]);
-  e.yz = D[1][2] + D[2][1] + (D[1][0] * D[2][0] + D[1][1] * D[2][1] + D[1][2] * D[2][2]);
-  e.xz = D[0][2] + D[2][0] + (D[0][0] * D[2][0] + D[0][1] * D[2][1] + D[0][2] * D[2][2]);
-  e.xy = D[0][1] + D[1][0] + (D[0][0] * D[1][0] + D[0][1] * D[1][1] + D[0][2] * D[1][2]);
-  return e;
-}
-
 // adj(C) for C = I + e (symmetric): C^{-1} = adj(C) / det(C) = adj(C) / J^2
 template <class R>
 __device__ __forceinline__ Sym6<R> adj_I_plus(const Sym6<R> &e) {
@@ -121,51 +199,131 @@ __device__ __forceinline__ void adj_F(const R (&D)[3][3], R (&A)[3][3]) {
   A[2][2] = f00 * f11 - f01 * f10;
 }
 
-// s * M * W * M^T for symmetric W (upper triangle returned)
+// |x| < bound for a positive bound, and a < b for b > 0: FP64 by the bit
+// patterns (positive doubles order as integers), so that a test does not take a
+// slot of the FP64 pipe, which issues one warp instruction in 16 cycles
+__device__ __forceinline__ bool abs_below(float x, float bound) { return fabsf(x) < bound; }
+__device__ __forceinline__ bool abs_below(double x, double bound) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffll) < __double_as_longlong(bound);
+}
+__device__ __forceinline__ bool below_pos(float a, float b) { return a < b; }
+__device__ __forceinline__ bool below_pos(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ bool above_zero(float x) { return x > 0.f; }
+__device__ __forceinline__ bool above_zero(double x) { return __double_as_longlong(x) > 0; }
+// |x| in FP32 to within 2^-23 of it (bits; FP32-range overflow gives inf)
+__device__ __forceinline__ float approx_abs(float x) { return fabsf(x); }
+__device__ __forceinline__ float approx_abs(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  const unsigned lo = (unsigned)__double2loint(x);
+  if (hi < (897u << 20)) return 0.f;
+  if (hi >= (1151u << 20)) return __int_as_float(0x7f800000);
+  return __uint_as_float(((hi - (896u << 20)) << 3) | (lo >> 29));
+}
+
+// ln(1 + x) and exp(y) for the small arguments of nearly incompressible
+// tissue (|J - 1| << 1): Taylor polynomials for |x|, |y| < 1/32 (FP32 degree 6
+// and 5, truncation below 2^-40 relative; FP64 degree 11 and 9, below 2^-56),
+// else the library functions.  In FP64 a third of the library call's
+// operations.
 template <class R>
-__device__ __forceinline__ Sym6<R> congruence(const R (&M)[3][3], const Sym6<R> &W, R s) {
-  R w[3][3] = {{W.xx, W.xy, W.xz}, {W.xy, W.yy, W.yz}, {W.xz, W.yz, W.zz}};
-  R T[3][3];
+__device__ __forceinline__ R log1p_small(R x) {
+  if (abs_below(x, R(0.03125))) {
+    if (sizeof(R) == 4)
+      return x * (R(1) + x * (R(-0.5) + x * (R(1.0 / 3.0) + x * (R(-0.25) +
+                  x * (R(0.2) + x * R(-1.0 / 6.0))))));
+    R s = R(1.0 / 11.0);
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+    for (int k = 10; k >= 1; --k) s = R((k & 1) ? 1.0 / k : -1.0 / k) + x * s;
+    return x * s;
+  }
+  return d_log1p(x);
+}
+template <class R>
+__device__ __forceinline__ R exp_small(R y) {
+  if (abs_below(y, R(0.03125))) {
+    if (sizeof(R) == 4)
+      return R(1) + y * (R(1) + y * (R(0.5) + y * (R(1.0 / 6.0) + y * (R(1.0 / 24.0) +
+                  y * R(1.0 / 120.0)))));
+    R s = R(1.0 / 362880.0);
+    constexpr double f[9] = {1.0, 1.0, 0.5, 1.0 / 6.0, 1.0 / 24.0, 1.0 / 120.0, 1.0 / 720.0,
+                             1.0 / 5040.0, 1.0 / 40320.0};
 #pragma unroll
-    for (int j = 0; j < 3; ++j) T[i][j] = M[i][0] * w[0][j] + M[i][1] * w[1][j] + M[i][2] * w[2][j];
+    for (int k = 8; k >= 0; --k) s = R(f[k]) + y * s;
+    return s;
+  }
+  return d_exp(y);
+}
+
+// symmetric product of two commuting symmetric matrices (powers of one matrix)
+template <class R>
+__device__ __forceinline__ Sym6<R> sym_mul(const Sym6<R> &a, const Sym6<R> &b) {
   Sym6<R> r;
-  r.xx = s * (T[0][0] * M[0][0] + T[0][1] * M[0][1] + T[0][2] * M[0][2]);
-  r.yy = s * (T[1][0] * M[1][0] + T[1][1] * M[1][1] + T[1][2] * M[1][2]);
-  r.zz = s * (T[2][0] * M[2][0] + T[2][1] * M[2][1] + T[2][2] * M[2][2]);
-  r.yz = s * (T[1][0] * M[2][0] + T[1][1] * M[2][1] + T[1][2] * M[2][2]);
-  r.xz = s * (T[0][0] * M[2][0] + T[0][1] * M[2][1] + T[0][2] * M[2][2]);
-  r.xy = s * (T[0][0] * M[1][0] + T[0][1] * M[1][1] + T[0][2] * M[1][2]);
+  r.xx = a.xx * b.xx + a.xy * b.xy + a.xz * b.xz;
+  r.yy = a.xy * b.xy + a.yy * b.yy + a.yz * b.yz;
+  r.zz = a.xz * b.xz + a.yz * b.yz + a.zz * b.zz;
+  r.yz = a.xy * b.xz + a.yy * b.yz + a.yz * b.zz;
+  r.xz = a.xx * b.xz + a.xy * b.yz + a.xz * b.zz;
+  r.xy = a.xx * b.xy + a.xy * b.yy + a.xz * b.yz;
   return r;
 }
 
+// M = C - I with its square and invariants, and C^{-1} - I = Ca I + Cb M +
+// Cg M^2, exact by Cayley-Hamilton for C = I + M:
+//   C^{-1} - I = (-I3 I - (1 + I1) M + M^2) / (1 + I1 + I2 + I3),
+// without the cancellation of adj(C) / det C - I.  Every law below is a
+// combination of I, M, M^2 (and the fibre's a0 x a0), so one product M M
+// replaces adjugates, left Cauchy-Green tensors and pull-backs.
+// 1 + I1 + I2 + I3 = J^2 = 1 + jj with jj = (J - 1)(J + 1).  I3 is the
+// determinant in FP32; in FP64 jj - I1 - I2, whose rounding is that of M
+// itself and five operations fewer.
 template <class R>
-__device__ __forceinline__ Sym6<R> sym_scale(const Sym6<R> &a, R s) {
-  return Sym6<R>{a.xx * s, a.yy * s, a.zz * s, a.yz * s, a.xz * s, a.xy * s};
+struct CGreen {
+  Sym6<R> M, M2;
+  R I1, trM2, I2, I3, jj, Ca, Cb, Cg;
+};
+template <class R>
+__device__ __forceinline__ CGreen<R> cgreen(const R (&D)[3][3], R Jm1) {
+  CGreen<R> g;
+  g.M = two_E(D);
+  g.M2 = sym_mul(g.M, g.M);
+  g.I1 = g.M.xx + g.M.yy + g.M.zz;
+  g.trM2 = g.M2.xx + g.M2.yy + g.M2.zz;
+  g.I2 = R(0.5) * (g.I1 * g.I1 - g.trM2);
+  g.jj = Jm1 * (2 + Jm1);
+  if (sizeof(R) == 4)
+    g.I3 = g.M.xx * (g.M.yy * g.M.zz - g.M.yz * g.M.yz) -
+           g.M.xy * (g.M.xy * g.M.zz - g.M.yz * g.M.xz) +
+           g.M.xz * (g.M.xy * g.M.yz - g.M.yy * g.M.xz);
+  else
+    g.I3 = g.jj - g.I1 - g.I2;
+  g.Cg = R(1) / (1 + g.jj);
+  g.Ca = -g.I3 * g.Cg;
+  g.Cb = -(1 + g.I1) * g.Cg;
+  return g;
+}
+// a I + b M + c M^2
+template <class R>
+__device__ __forceinline__ Sym6<R> cg_combine(const CGreen<R> &g, R a, R b, R c) {
+  Sym6<R> S;
+  S.xx = a + b * g.M.xx + c * g.M2.xx;
+  S.yy = a + b * g.M.yy + c * g.M2.yy;
+  S.zz = a + b * g.M.zz + c * g.M2.zz;
+  S.yz = b * g.M.yz + c * g.M2.yz;
+  S.xz = b * g.M.xz + c * g.M2.xz;
+  S.xy = b * g.M.xy + c * g.M2.xy;
+  return S;
 }
 
 // ---- 1: compressible Neo-Hookean, CompressibleNeoHookean.cpp:15-55 ----
-// S = mu (I - C^-1) + lambda ln J C^-1 = C^-1 (mu 2E + lambda ln J I)
+// S = mu (I - C^-1) + lambda ln J C^-1 = t I + (t - mu) (C^-1 - I), t = lambda ln J
 template <class R>
 __device__ __forceinline__ Sym6<R> mat_neohookean(const MatP<R> &m, const R (&D)[3][3], R Jm1) {
-  R mu = m.p[1], lam = m.p[2];
-  Sym6<R> e = two_E(D);
-  Sym6<R> a = adj_I_plus(e);
-  R J = 1 + Jm1;
-  R iJ2 = 1 / (J * J);
-  R t = lam * d_log1p(Jm1);
-  // T = mu*2E + t I
-  R txx = mu * e.xx + t, tyy = mu * e.yy + t, tzz = mu * e.zz + t;
-  R tyz = mu * e.yz, txz = mu * e.xz, txy = mu * e.xy;
-  Sym6<R> S;
-  S.xx = iJ2 * (a.xx * txx + a.xy * txy + a.xz * txz);
-  S.yy = iJ2 * (a.xy * txy + a.yy * tyy + a.yz * tyz);
-  S.zz = iJ2 * (a.xz * txz + a.yz * tyz + a.zz * tzz);
-  S.yz = iJ2 * (a.xy * txz + a.yy * tyz + a.yz * tzz);
-  S.xz = iJ2 * (a.xx * txz + a.xy * tyz + a.xz * tzz);
-  S.xy = iJ2 * (a.xx * txy + a.xy * tyy + a.xz * tyz);
-  return S;
+  const CGreen<R> g = cgreen(D, Jm1);
+  const R t = m.p[2] * log1p_small(Jm1);
+  const R w = t - m.p[1];
+  return cg_combine(g, t + w * g.Ca, w * g.Cb, w * g.Cg);
 }
 
 // ---- 2: St. Venant-Kirchhoff, StVenantKirchhoff.cpp:16-54 ----
@@ -202,77 +360,69 @@ __device__ __forceinline__ Sym6<R> mat_linear(const MatP<R> &m, const R (&D)[3][
   return S;
 }
 
-// Isochoric Cauchy-type tensor of the HGO family pulled back to PK2:
-//   S_iso = J F^-1 [ (c1 dev(Bbar) + c4 dev(abar x abar)) / J ] F^-T,
-// with Bbar = J^-2/3 B, abar = J^-1/3 F a0.  c4 = 0 drops the fibre term.
-template <class R>
-__device__ __forceinline__ Sym6<R> hgo_iso_pk2(const R (&D)[3][3], R J, R Jm23,
-                                               const Sym6<R> &eB, R c1, R c4, const R (&a)[3]) {
-  R t3 = (eB.xx + eB.yy + eB.zz) * R(1.0 / 3.0);  // dev(B) = dev(2e)
-  R aa3 = (a[0] * a[0] + a[1] * a[1] + a[2] * a[2]) * R(1.0 / 3.0);
-  R s = Jm23;
-  Sym6<R> W;
-  W.xx = s * (c1 * (eB.xx - t3) + c4 * (a[0] * a[0] - aa3));
-  W.yy = s * (c1 * (eB.yy - t3) + c4 * (a[1] * a[1] - aa3));
-  W.zz = s * (c1 * (eB.zz - t3) + c4 * (a[2] * a[2] - aa3));
-  W.yz = s * (c1 * eB.yz + c4 * a[1] * a[2]);
-  W.xz = s * (c1 * eB.xz + c4 * a[0] * a[2]);
-  W.xy = s * (c1 * eB.xy + c4 * a[0] * a[1]);
-  // J F^-1 (W/J) F^-T = adj(F) W adj(F)^T / J^2
-  return W;
-}
-
 // ---- 4/5/7: HGO family (HGOIsotropic.cpp:21-115, HGOIsotropicViscoelastic.cpp:27-168) ----
 // Returns the isochoric PK2 part (which is also the reference's "Sdev") and the
 // volumetric part separately so the viscoelastic update can use S_iso.
-// J^{-2/3} - 1 from x = J - 1: in FP32 for |x| < 1/32 the binomial series
-// of (1 + x)^{-2/3} to degree 7 (truncation below 2^-40 relative), else
-// expm1(-2/3 log1p(x)); FP64 always the library functions.
+// J^{-2/3} - 1 from x = J - 1: for |x| < 1/32 the binomial series of
+// (1 + x)^{-2/3} (FP32 degree 7, truncation below 2^-40 relative; FP64 degree
+// 11, below 2^-56), else expm1(-2/3 log1p(x)).
 template <class R>
 __device__ __forceinline__ R jm23m1_of(R x) {
-  if (sizeof(R) == 4 && fabs(x) < R(0.03125)) {
-    // binom(-2/3, k): -2/3, 5/9, -40/81, 110/243, -308/729, 2618/6561, -7480/19683
-    return x * (R(-2.0 / 3.0) + x * (R(5.0 / 9.0) + x * (R(-40.0 / 81.0) +
-                x * (R(110.0 / 243.0) + x * (R(-308.0 / 729.0) + x * (R(2618.0 / 6561.0) +
-                x * R(-7480.0 / 19683.0)))))));
+  if (abs_below(x, R(0.03125))) {
+    // binom(-2/3, k), k = 1..11
+    constexpr double b[11] = {-2.0 / 3.0, 5.0 / 9.0, -40.0 / 81.0, 110.0 / 243.0, -308.0 / 729.0,
+                              2618.0 / 6561.0, -7480.0 / 19683.0, 21505.0 / 59049.0,
+                              -559130.0 / 1594323.0, 1621477.0 / 4782969.0, -4717024.0 / 14348907.0};
+    constexpr int n = sizeof(R) == 4 ? 7 : 11;
+    R s = R(b[n - 1]);
+#pragma unroll
+    for (int k = n - 2; k >= 0; --k) s = R(b[k]) + x * s;
+    return x * s;
   }
   return d_expm1(R(-2.0 / 3.0) * d_log1p(x));
 }
+// With Bbar = J^-2/3 B, abar = J^-1/3 F a0 the family's isochoric Kirchhoff-type
+// tensor c1 dev(Bbar) + c4 dev(abar x abar) pulls back term by term
+// (F^-1 B F^-T = I, F^-1 F^-T = C^-1, F^-1 a a F^-T = a0 x a0) to
+//   S_iso = J^-2/3 [c1 (I - tr B / 3 C^-1) + c4 (a0 x a0 - |F a0|^2 / 3 C^-1)],
+// and with C^-1 = I + Ci, tr B = 3 + I1, |F a0|^2 = 1 + q nothing of order one
+// cancels at small strain: I - tr B / 3 C^-1 = -I1/3 I - (1 + I1/3) Ci.
 template <class R, bool FIBER>
 __device__ __forceinline__ void mat_hgo_parts(const MatP<R> &m, const R (&D)[3][3], R Jm1,
                                               const R (&a0)[3], Sym6<R> &Siso, Sym6<R> &Svol) {
-  R mu = m.p[1], k1 = m.p[3], k2 = m.p[4];
-  R kappa = FIBER ? m.p[7] : R(1.0 / 3.0);
-  R J = 1 + Jm1;
-  R Jm23m1 = jm23m1_of(Jm1);
-  R Jm23 = 1 + Jm23m1;
-  Sym6<R> eB = two_e_left(D);
-  R I1m3 = 3 * Jm23m1 + Jm23 * (eB.xx + eB.yy + eB.zz);
-  R a[3] = {R(0), R(0), R(0)};
-  R Ea = kappa * I1m3;
+  const R mu = m.p[1], k1 = m.p[3], k2 = m.p[4];
+  const R kappa = FIBER ? m.p[7] : R(1.0 / 3.0);
+  const CGreen<R> g = cgreen(D, Jm1);
+  const R Jm23m1 = jm23m1_of(Jm1);
+  const R Jm23 = 1 + Jm23m1;
+  R Ea = kappa * (3 * Jm23m1 + Jm23 * g.I1);  // kappa (I1bar - 3)
+  Sym6<R> aa = {R(0), R(0), R(0), R(0), R(0), R(0)};
+  R q = 0;
   if (FIBER) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) a[i] = a0[i] + D[i][0] * a0[0] + D[i][1] * a0[1] + D[i][2] * a0[2];
-    R da0 = a[0] * a0[0] + a[1] * a0[1] + a[2] * a0[2] - 1;  // a0 . D a0
-    R Da2 = (a[0] - a0[0]) * (a[0] - a0[0]) + (a[1] - a0[1]) * (a[1] - a0[1]) +
-            (a[2] - a0[2]) * (a[2] - a0[2]);
-    R q = 2 * da0 + Da2;  // |F a0|^2 - 1
-    R I4m1 = Jm23m1 + Jm23 * q;
-    Ea += (1 - 3 * kappa) * I4m1;
+    aa = Sym6<R>{a0[0] * a0[0], a0[1] * a0[1], a0[2] * a0[2], a0[1] * a0[2], a0[0] * a0[2],
+                 a0[0] * a0[1]};
+    q = aa.xx * g.M.xx + aa.yy * g.M.yy + aa.zz * g.M.zz +
+        2 * (aa.yz * g.M.yz + aa.xz * g.M.xz + aa.xy * g.M.xy);  // |F a0|^2 - 1
+    Ea += (1 - 3 * kappa) * (Jm23m1 + Jm23 * q);
   }
-  R dW = Ea > 0 ? k1 * Ea * d_exp(k2 * Ea * Ea) : R(0);  // dW_f/dE_alpha
-  R c1 = mu + 2 * dW * kappa;
-  R c4 = FIBER ? 2 * dW * (1 - 3 * kappa) : R(0);
-  Sym6<R> W = hgo_iso_pk2(D, J, Jm23, eB, c1, c4, a);
-  R A[3][3];
-  adj_F(D, A);
-  R iJ2 = 1 / (J * J);
-  Siso = congruence(A, W, iJ2);
+  const R dW = above_zero(Ea) ? k1 * Ea * exp_small(k2 * Ea * Ea) : R(0);  // dW_f/dE_alpha
+  const R third = R(1.0 / 3.0);
+  const R c1 = Jm23 * (mu + 2 * dW * kappa);
+  const R c4 = FIBER ? Jm23 * (2 * dW * (1 - 3 * kappa)) : R(0);
+  const R i = c1 * (third * g.I1) + (FIBER ? c4 * (third + third * q) : R(0));
+  const R w = -(c1 + i);
+  Siso = cg_combine(g, w * g.Ca - i, w * g.Cb, w * g.Cg);
+  if (FIBER) {
+    Siso.xx += c4 * aa.xx;
+    Siso.yy += c4 * aa.yy;
+    Siso.zz += c4 * aa.zz;
+    Siso.yz += c4 * aa.yz;
+    Siso.xz += c4 * aa.xz;
+    Siso.xy += c4 * aa.xy;
+  }
   // S_vol = J p C^-1, p = K (J^2 - 1) / (2 J)  (HGOIsotropic.cpp:47)
-  Sym6<R> ce = two_E(D);
-  Sym6<R> ac = adj_I_plus(ce);
-  R Jp = R(0.5) * m.K * Jm1 * (2 + Jm1);
-  Svol = sym_scale(ac, Jp * iJ2);
+  const R Jp = R(0.5) * m.K * g.jj;
+  Svol = cg_combine(g, Jp + Jp * g.Ca, Jp * g.Cb, Jp * g.Cg);
 }
 
 // ---- 6: one-term Ogden (new): W = 2mu/alpha^2 sum(lbar_i^alpha - 1) + K/2((J^2-1)/2 - ln J) ----
@@ -351,122 +501,33 @@ __device__ __forceinline__ void jacobi_sym3(Sym6<R> A, R (&w)[3], R (&V)[3][3]) 
     for (int j = 0; j < 3; ++j) V[i][j] = v[i][j];
 }
 
-// symmetric product of two commuting symmetric matrices (powers of one matrix)
+// Isochoric stress plus volumetric part through the principal directions of
+// M = 2E (large strains)
 template <class R>
-__device__ __forceinline__ Sym6<R> sym_mul(const Sym6<R> &a, const Sym6<R> &b) {
-  Sym6<R> r;
-  r.xx = a.xx * b.xx + a.xy * b.xy + a.xz * b.xz;
-  r.yy = a.xy * b.xy + a.yy * b.yy + a.yz * b.yz;
-  r.zz = a.xz * b.xz + a.yz * b.yz + a.zz * b.zz;
-  r.yz = a.xy * b.xz + a.yy * b.yz + a.yz * b.zz;
-  r.xz = a.xx * b.xz + a.xy * b.yz + a.xz * b.zz;
-  r.xy = a.xx * b.xy + a.xy * b.yy + a.xz * b.yz;
-  return r;
-}
-
-// ln(1 + x) and exp(y) for the small arguments of nearly incompressible
-// tissue (|J - 1| << 1): in FP32 the Taylor polynomials to degree 6 and 5
-// (truncation below 2^-40 relative for |x|, |y| < 1/32), else the library
-// functions; FP64 always the library functions.
-template <class R>
-__device__ __forceinline__ R log1p_small(R x) {
-  if (sizeof(R) == 4 && fabs(x) < R(0.03125))
-    return x * (R(1) + x * (R(-0.5) + x * (R(1.0 / 3.0) + x * (R(-0.25) +
-                x * (R(0.2) + x * R(-1.0 / 6.0))))));
-  return d_log1p(x);
-}
-template <class R>
-__device__ __forceinline__ R exp_small(R y) {
-  if (sizeof(R) == 4 && fabs(y) < R(0.03125))
-    return R(1) + y * (R(1) + y * (R(0.5) + y * (R(1.0 / 6.0) + y * (R(1.0 / 24.0) +
-                y * R(1.0 / 120.0)))));
-  return d_exp(y);
-}
-
-template <class R>
-__device__ __forceinline__ Sym6<R> mat_ogden(const MatP<R> &m, const R (&D)[3][3], R Jm1) {
-  R mu = m.p[1], alpha = m.p[3];
-  Sym6<R> e = two_E(D);
-  R lnJ = log1p_small(Jm1);
+__device__ __forceinline__ Sym6<R> ogden_eigen(const MatP<R> &m, const Sym6<R> &e, R Jm1) {
+  const R mu = m.p[1], alpha = m.p[3];
+  const R lnJ = log1p_small(Jm1);
   Sym6<R> S;
-  const R n2 = e.xx * e.xx + e.yy * e.yy + e.zz * e.zz +
-               2 * (e.yz * e.yz + e.xz * e.xz + e.xy * e.xy);
-  if (n2 < m.ser_thr2) {
-    // Small strain: with M = 2E = C - I the isochoric stress is
-    //   S_iso = (2 mu/alpha) J^{-alpha/3} [C^{alpha/2-1} - tr(C^{alpha/2})/3 C^{-1}]
-    //         = c [A - Ci - tr(B)/3 (I + Ci)],
-    // A = (I+M)^{alpha/2-1} - I, a binomial series in powers of M (exact to
-    // FP32 rounding below the host's bound on |M|_F, no eigenvectors, no
-    // cancellation of O(1) terms), and B = (I+M)^{alpha/2} - I = A + M + M A
-    // (exact: (I+M)^{alpha/2} = (I+M)(I+A)).  By Cayley-Hamilton every power
-    // is M^p = a I + b M + c M^2 with
-    //   M^{p+1}: (a, b, c) <- (c I3, a - c I2, b + c I1),
-    // so the series reduces to scalar coefficients of I, M and M^2, and
-    //   tr B = I1 + tr A + tr(M A),  tr M^3 = I1 tr M^2 - I2 I1 + 3 I3.
-    // Ci = (I+M)^{-1} - I is exact by Cayley-Hamilton for C = I + M:
-    //   C^{-1} = (C^2 - I1(C) C + I2(C) I) / I3(C)
-    //   => Ci = (-I3 I - (1 + I1) M + M^2) / (1 + I1 + I2 + I3)
-    // (I1..I3: invariants of M; no cancellation).
-    const Sym6<R> M2 = sym_mul(e, e);
-    const R I1 = e.xx + e.yy + e.zz;
-    const R trM2 = M2.xx + M2.yy + M2.zz;
-    const R I2 = R(0.5) * (I1 * I1 - trM2);
-    const R I3 = e.xx * (e.yy * e.zz - e.yz * e.yz) - e.xy * (e.xy * e.zz - e.yz * e.xz) +
-                 e.xz * (e.xy * e.yz - e.yy * e.xz);
-    // power 1: (0, 1, 0)
-    R pa = 0, pb = 1, pc = 0;
-    R Aa = 0, Ab = m.ser_a[0], Ag = 0;  // A  = Aa I + Ab M + Ag M^2
+  R w[3], V[3][3];
+  jacobi_sym3<R, sizeof(R) == 4 ? 4 : 6>(e, w, V);
+  R em[3], mean = 0;
 #pragma unroll
-    for (int k = 1; k < kOgdenSeries; ++k) {
-      const R na = pc * I3, nb = pa - pc * I2, nc = pb + pc * I1;
-      pa = na;
-      pb = nb;
-      pc = nc;
-      const R sa = m.ser_a[k];
-      Aa += sa * pa;
-      Ab += sa * pb;
-      Ag += sa * pc;
-    }
-    const R trM3 = I1 * (trM2 - I2) + R(3) * I3;
-    const R trB = I1 + (R(3) * Aa + Ab * I1 + Ag * trM2) + (Aa * I1 + Ab * trM2 + Ag * trM3);
-    const R iC3 = R(1) / (1 + I1 + I2 + I3);  // Ci = Ca I + Cb M + Cg M^2
-    const R Ca = -I3 * iC3, Cb = -(1 + I1) * iC3, Cg = iC3;
-    const R c = 2 * mu / alpha * exp_small(-alpha * R(1.0 / 3.0) * lnJ);
-    const R t = trB * R(1.0 / 3.0);
-    // the volumetric part J p C^{-1} in the same basis: C^{-1} = I + Ci, and
-    // J p = K (J^2 - 1) / 2 (HGOIsotropic.cpp:47 form) -- no second inverse
-    const R Jp = R(0.5) * m.K * Jm1 * (2 + Jm1);
-    const R ka = c * (Aa - Ca - t * (1 + Ca)) + Jp * (1 + Ca),
-            kb = c * (Ab - Cb - t * Cb) + Jp * Cb, kg = c * (Ag - Cg - t * Cg) + Jp * Cg;
-    S.xx = ka + kb * e.xx + kg * M2.xx;
-    S.yy = ka + kb * e.yy + kg * M2.yy;
-    S.zz = ka + kb * e.zz + kg * M2.zz;
-    S.yz = kb * e.yz + kg * M2.yz;
-    S.xz = kb * e.xz + kg * M2.xz;
-    S.xy = kb * e.xy + kg * M2.xy;
-    return S;
-  } else {
-    R w[3], V[3][3];
-    jacobi_sym3<R, sizeof(R) == 4 ? 4 : 6>(e, w, V);
-    R em[3], mean = 0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      R y = R(0.5) * alpha * (d_log1p(w[i]) - R(2.0 / 3.0) * lnJ);  // (alpha/2) ln lbar_i^2
-      em[i] = d_expm1(y);
-      mean += em[i];
-    }
-    mean *= R(1.0 / 3.0);
-    R c = 2 * mu / alpha;
-    R f[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) f[i] = c * (em[i] - mean) / (1 + w[i]);
-    S.xx = f[0] * V[0][0] * V[0][0] + f[1] * V[0][1] * V[0][1] + f[2] * V[0][2] * V[0][2];
-    S.yy = f[0] * V[1][0] * V[1][0] + f[1] * V[1][1] * V[1][1] + f[2] * V[1][2] * V[1][2];
-    S.zz = f[0] * V[2][0] * V[2][0] + f[1] * V[2][1] * V[2][1] + f[2] * V[2][2] * V[2][2];
-    S.yz = f[0] * V[1][0] * V[2][0] + f[1] * V[1][1] * V[2][1] + f[2] * V[1][2] * V[2][2];
-    S.xz = f[0] * V[0][0] * V[2][0] + f[1] * V[0][1] * V[2][1] + f[2] * V[0][2] * V[2][2];
-    S.xy = f[0] * V[0][0] * V[1][0] + f[1] * V[0][1] * V[1][1] + f[2] * V[0][2] * V[1][2];
+  for (int i = 0; i < 3; ++i) {
+    R y = R(0.5) * alpha * (d_log1p(w[i]) - R(2.0 / 3.0) * lnJ);  // (alpha/2) ln lbar_i^2
+    em[i] = d_expm1(y);
+    mean += em[i];
   }
+  mean *= R(1.0 / 3.0);
+  R c = 2 * mu / alpha;
+  R f[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) f[i] = c * (em[i] - mean) / (1 + w[i]);
+  S.xx = f[0] * V[0][0] * V[0][0] + f[1] * V[0][1] * V[0][1] + f[2] * V[0][2] * V[0][2];
+  S.yy = f[0] * V[1][0] * V[1][0] + f[1] * V[1][1] * V[1][1] + f[2] * V[1][2] * V[1][2];
+  S.zz = f[0] * V[2][0] * V[2][0] + f[1] * V[2][1] * V[2][1] + f[2] * V[2][2] * V[2][2];
+  S.yz = f[0] * V[1][0] * V[2][0] + f[1] * V[1][1] * V[2][1] + f[2] * V[1][2] * V[2][2];
+  S.xz = f[0] * V[0][0] * V[2][0] + f[1] * V[0][1] * V[2][1] + f[2] * V[0][2] * V[2][2];
+  S.xy = f[0] * V[0][0] * V[1][0] + f[1] * V[0][1] * V[1][1] + f[2] * V[0][2] * V[1][2];
   Sym6<R> ac = adj_I_plus(e);
   R J = 1 + Jm1;
   R Jp = R(0.5) * m.K * Jm1 * (2 + Jm1) / (J * J);
@@ -477,6 +538,71 @@ __device__ __forceinline__ Sym6<R> mat_ogden(const MatP<R> &m, const R (&D)[3][3
   S.xz += Jp * ac.xz;
   S.xy += Jp * ac.xy;
   return S;
+}
+
+// Horner steps X <- M X + s_k I, k = K1 - 1 .. K0 (coefficient index), on
+// X = a I + b M + c M^2: M^3 = I1 M^2 - I2 M + I3 I
+template <int K0, int K1, class R>
+__device__ __forceinline__ void ogden_horner(const MatP<R> &m, const CGreen<R> &g, R &a, R &b,
+                                             R &c) {
+#pragma unroll
+  for (int k = K1 - 1; k >= K0; --k) {
+    const R na = c * g.I3 + m.ser_a[k], nb = a - c * g.I2, nc = b + c * g.I1;
+    a = na;
+    b = nb;
+    c = nc;
+  }
+}
+
+// ---- 6: small strain: with M = 2E = C - I the isochoric stress is
+//   S_iso = (2 mu/alpha) J^{-alpha/3} [C^{alpha/2-1} - tr(C^{alpha/2})/3 C^{-1}]
+//         = c [A - Ci - tr(B)/3 (I + Ci)],
+// A = (I+M)^{alpha/2-1} - I, a binomial series in powers of M (to the type's
+// rounding below the host's bound on the spectral radius, no eigenvectors, no
+// cancellation of O(1) terms), and B = (I+M)^{alpha/2} - I = A + M + M A
+// (exact: (I+M)^{alpha/2} = (I+M)(I+A)).  By Cayley-Hamilton the series is
+// Horner's scheme on the three coefficients of I, M and M^2 (three FMAs per
+// term; carrying the powers themselves takes six), and
+//   tr B = I1 + tr A + tr(M A),  tr M^3 = I1 (tr M^2 - I2) + 3 I3.
+// The spectral radius is at most |I1|/3 + sqrt(2/3 tr M^2).
+template <class R>
+__device__ __forceinline__ Sym6<R> mat_ogden(const MatP<R> &m, const R (&D)[3][3], R Jm1) {
+  const CGreen<R> g = cgreen(D, Jm1);
+  const float i1 = approx_abs(g.I1) * (1.f / 3.f), f2 = approx_abs(g.trM2) * (2.f / 3.f);
+  auto within = [&](int k) {
+    const float t = m.ser_r[k] - i1;
+    return t > 0.f && f2 < t * t;
+  };
+  if (!within(OgdenSeries<R>::kSteps - 1)) return ogden_eigen(m, g.M, Jm1);
+  R a = 0, b = 0, c = 0;
+  if constexpr (sizeof(R) == 4) {
+    ogden_horner<0, 9>(m, g, a, b, c);
+  } else {
+    if (!within(3)) ogden_horner<24, 32>(m, g, a, b, c);
+    if (!within(2)) ogden_horner<16, 24>(m, g, a, b, c);
+    if (!within(1)) ogden_horner<12, 16>(m, g, a, b, c);
+    if (!within(0)) ogden_horner<8, 12>(m, g, a, b, c);
+    ogden_horner<0, 8>(m, g, a, b, c);
+  }
+  const R Aa = c * g.I3, Ab = a - c * g.I2, Ag = b + c * g.I1;  // A = M X
+  const R trM3 = g.I1 * (g.trM2 - g.I2) + R(3) * g.I3;
+  const R trB = g.I1 + Aa * (R(3) + g.I1) + Ab * (g.I1 + g.trM2) + Ag * (g.trM2 + trM3);
+  R jp;  // J^(-alpha/3)
+  if (abs_below(Jm1, R(m.jpow_x))) {
+    jp = m.jpow[JPowSeries<R>::kMax - 1];
+#pragma unroll
+    for (int k = JPowSeries<R>::kMax - 2; k >= 0; --k) jp = m.jpow[k] + Jm1 * jp;
+    jp = R(1) + Jm1 * jp;
+  } else {
+    jp = d_exp(-m.p[3] * R(1.0 / 3.0) * d_log1p(Jm1));
+  }
+  const R k0 = m.og_c * jp;
+  const R t = trB * R(1.0 / 3.0);
+  // the volumetric part J p C^{-1} in the same basis: C^{-1} = I + Ci, and
+  // J p = K (J^2 - 1) / 2 (HGOIsotropic.cpp:47 form)
+  const R Jp = R(0.5) * m.K * g.jj;
+  const R w = Jp - k0 * (1 + t);
+  return cg_combine(g, k0 * (Aa - t) + Jp + w * g.Ca, k0 * Ab + w * g.Cb, k0 * Ag + w * g.Cg);
 }
 
 }  // namespace ftgpu

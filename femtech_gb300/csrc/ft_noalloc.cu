@@ -133,14 +133,8 @@ extern "C" int ftgpu_hex8_force_noalloc(int nNodes, int nelements, const double 
     scratch = g_noalloc_ptr[dev];
     bad = g_noalloc_bad_ptr[dev];
   }
-  // Parameters as the model's set-up builds them for FP64 mode; Ogden in
-  // FP64 always takes the eigen-decomposition (ser_thr2 = 0, no series).
-  MatP<double> mp;
-  memset(&mp, 0, sizeof(mp));
-  for (int k = 0; k < 9; ++k) mp.p[k] = properties[k];
-  mp.K = properties[2] + 2.0 * properties[1] / 3.0;
-  mp.mat = materialID;
-  mp.ser_thr2 = 0.0;
+  // parameters as the model's set-up builds them for FP64 mode
+  const MatP<double> mp = make_matp<double>(materialID, properties);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(bad, 0, sizeof(int), s) != cudaSuccess) return FTGPU_ERR_CUDA;
   const int th = 128, nb = (nelements + th - 1) / th;
