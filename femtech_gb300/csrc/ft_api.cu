@@ -586,7 +586,7 @@ int launch_groups_t(ftgpu_model *m, int parity, int use_clock, double dt_direct,
                  ? launch_hexgp(g.mat, md, g.npatch, hexgp_threads(PE), hexgp_smem_bytes<R>(PE), st,
                                 A, pass)
                  : launch_elem<R>(g.etype, g.mat, md, g.npatch, PE,
-                                  elem_smem_bytes_host<R>(g.etype, PE), st, A, pass);
+                                  elem_smem_bytes_host<R>(g.etype, g.mat, PE), st, A, pass);
     };
     if (m->surr && g.mat == 7 && dt_only == kPassForce && sizeof(R) == 4) {
       // surrogate: features of every Gauss point, one fused MLP pass, then

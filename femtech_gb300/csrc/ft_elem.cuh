@@ -164,13 +164,28 @@ __device__ __forceinline__ void goh_parts_surrogate(const MatP<R> &mp, const R (
   Sv = cg_combine(g, Jp + Jp * g.Ca, Jp * g.Cb, Jp * g.Cg);
 }
 
-// hin: the Gauss point's history already loaded into registers (same order
-// as hist[c * hs]), or nullptr to read it from hist
-template <class R, int MAT>
+// where a Gauss point's history is read: component k from global memory
+// (where it is also written), or from this thread's column of a staged copy
+template <class R>
+struct HistGlobal {
+  const R *p;
+  long long stride;
+  __device__ __forceinline__ R operator()(int k) const { return p[k * stride]; }
+};
+template <class R>
+struct HistShared {
+  const R *p;
+  int stride;
+  __device__ __forceinline__ R operator()(int k) const { return p[k * stride]; }
+};
+// history components of a law per Gauss point
+__host__ __device__ constexpr int hist_comps(int mat) { return mat == 5 ? 18 : (mat == 7 ? 12 : 0); }
+
+template <class R, int MAT, class HIN>
 __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][3], R Jm1,
                                              const R (&a0)[3], R *hist, long long hs,
                                              const R (&pc)[4], const float *sy,
-                                             const SurrogateLaw &law, const R *hin = nullptr) {
+                                             const SurrogateLaw &law, const HIN &hin) {
   Sym6<R> S;
   if (MAT == 0) {
     S = Sym6<R>{0, 0, 0, 0, 0, 0};
@@ -188,6 +203,13 @@ __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][
   } else if (MAT == 6) {
     S = mat_ogden(mp, D, Jm1);
   } else {  // 5 / 7: HGO family + Prony series (HGOIsotropicViscoelastic.cpp:98-159)
+    constexpr int NT = MAT == 5 ? 2 : 1, NH = 6 * (NT + 1);
+    // the point's whole history first: behind the stores of one component the
+    // loads of the next could not start (they might alias), six round trips
+    // to memory per point instead of one that the law's arithmetic covers
+    R h[NH];
+#pragma unroll
+    for (int k = 0; k < NH; ++k) h[k] = hin(k);
     Sym6<R> Si, Sv;
     if (MAT == 7 && sy != nullptr)
       goh_parts_surrogate(mp, D, Jm1, a0, sy, law, Si, Sv);
@@ -195,17 +217,15 @@ __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][
       mat_hgo_parts<R, MAT == 7>(mp, D, Jm1, a0, Si, Sv);
     R sd[6] = {Si.xx, Si.yy, Si.zz, Si.yz, Si.xz, Si.xy};
     R sv[6] = {Sv.xx, Sv.yy, Sv.zz, Sv.yz, Sv.xz, Sv.xy};
-    constexpr int NT = MAT == 5 ? 2 : 1;
     R out[6];
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-      R s0 = hin ? hin[NT * 6 + c] : hist[(NT * 6 + c) * hs];
-      R dS = sd[c] - s0;
-      R h1 = pc[0] * (hin ? hin[c] : hist[c * hs]) + pc[1] * dS;
+      const R dS = sd[c] - h[NT * 6 + c];
+      const R h1 = pc[0] * h[c] + pc[1] * dS;
       hist[c * hs] = h1;
       R acc = sd[c] + sv[c] + h1;
       if (NT == 2) {
-        R h2 = pc[2] * (hin ? hin[6 + c] : hist[(6 + c) * hs]) + pc[3] * dS;
+        const R h2 = pc[2] * h[6 + c] + pc[3] * dS;
         hist[(6 + c) * hs] = h2;
         acc += h2;
       }
@@ -370,6 +390,37 @@ __device__ __forceinline__ float face_pair_area_max(const float (&h)[7][3], int 
   return fmaxf(ax, ay);
 }
 
+// The Gauss points' inputs of one element of the FP32 C3D8 pass, in this
+// thread's columns of shared memory by its own asynchronous copies (no
+// barrier: nobody else reads them).  Laws without history stage all 20 rows of
+// the geometry before the loop (40 KB per 128 elements; streaming them two
+// points at a time took 834 instead of 811 us a step on the 4M block, the
+// waits and address steps in the loop).  Laws with a history stream both: the
+// geometry of two points at a time (five rows of 16 bytes, two buffers), the
+// history one point ahead (two buffers), so that no point waits for memory and
+// four blocks still fit an SM (238k elements of material 5: step 156 us with
+// the history loaded at each point's start, 114 us streamed).
+struct HexStream {
+  float *geo;        // shared: [pairs held][5 rows][elements] x 4, this thread's first value
+  float *hist;       // shared: [2][components][elements], this thread's value
+  const float *src;  // global: this element's value 0 of row 0
+  long long nelem;
+  int rs;            // 4 x elements per patch: row stride in shared memory
+  int mask;          // pairs held - 1 (3: all four, 1: two)
+  __device__ __forceinline__ void geo_pair(int q) const {
+    const float *s = src + 20ll * q * nelem;
+    float *d = geo + (q & mask) * 5 * rs;
+#pragma unroll
+    for (int r = 0; r < 5; ++r) cp_async16(d + r * rs, s + 4ll * r * nelem);
+  }
+  template <int NH>
+  __device__ __forceinline__ void hist_point(int g, const float *h, long long hs) const {
+    float *d = hist + (g & 1) * NH * (rs / 4);
+#pragma unroll
+    for (int k = 0; k < NH; ++k) cp_async_small<4>(d + k * (rs / 4), h + k * hs);
+  }
+};
+
 template <int MAT, bool GP>
 __device__ __forceinline__ void hex_gauss_loop_x2(const float2 (&hp)[7], const float (&hz)[7],
                                                   const MatP<float> &mp,
@@ -378,8 +429,10 @@ __device__ __forceinline__ void hex_gauss_loop_x2(const float2 (&hp)[7], const f
                                                   int pass, float &vol, float2 (&mc)[7],
                                                   float (&mz)[7], int &bad,
                                                   const ElemArgs<float> &A, long long gpo,
-                                                  const float *gb, int rs) {
+                                                  const HexStream &st) {
   const bool dt_only = pass == kPassDt;
+  const int rs = st.rs;
+  const float *gn = st.geo;  // the next point's values (all rows staged)
 #pragma unroll
   for (int k = 0; k < 7; ++k) {
     mc[k] = make_float2(0.f, 0.f);
@@ -390,14 +443,23 @@ __device__ __forceinline__ void hex_gauss_loop_x2(const float2 (&hp)[7], const f
     float xi, et, ze;
     hex_gauss_point(g, xi, et, ze);
     const float ez = et * ze, xz = xi * ze, xe = xi * et;
+    if (hist_comps(MAT) > 0) {
+      if (g > 0) cp_async_wait_all();  // this point's inputs, on their way since the last one
+      if (!(g & 1) && g < 6) st.geo_pair(g / 2 + 1);
+      if (g < 7 && pass == kPassForce)
+        st.template hist_point<hist_comps(MAT)>(g + 1, hist + (g + 1) * gs, hs);
+    }
     // A^{-1} (Q) and det A: values 10g .. 10g+9 as five pairs
+    const float *gb = hist_comps(MAT) > 0
+                          ? st.geo + ((g >> 1) & 1) * 5 * rs + ((g & 1) ? 2 * rs + 2 : 0)
+                          : gn;
     const int o1 = (g & 1) ? rs - 2 : 2;
     const float2 q0 = *reinterpret_cast<const float2 *>(gb),
                  q1 = *reinterpret_cast<const float2 *>(gb + o1),
                  q2 = *reinterpret_cast<const float2 *>(gb + rs),
                  q3 = *reinterpret_cast<const float2 *>(gb + rs + o1),
                  q4 = *reinterpret_cast<const float2 *>(gb + 2 * rs);
-    gb += (g & 1) ? 3 * rs - 2 : 2 * rs + 2;
+    if (hist_comps(MAT) == 0) gn += (g & 1) ? 3 * rs - 2 : 2 * rs + 2;
     const float Q[3][3] = {{q0.x, q0.y, q1.x}, {q1.y, q2.x, q2.y}, {q3.x, q3.y, q4.x}};
     const float detA = q4.y;
     // H[d][i] = du_d / dxi_i: column i, rows 0-1 paired, row 2 scalar
@@ -427,7 +489,9 @@ __device__ __forceinline__ void hex_gauss_loop_x2(const float2 (&hp)[7], const f
       continue;
     }
     const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
-    const Sym6<float> S = stress_at<float, MAT>(mp, D, Jm1, a0, hist + g * gs, hs, pc, sy, A.law);
+    const Sym6<float> S = stress_at<float, MAT>(
+        mp, D, Jm1, a0, hist + g * gs, hs, pc, sy, A.law,
+        HistShared<float>{st.hist + (g & 1) * hist_comps(MAT) * (rs / 4), rs / 4});
     if (GP) {
       const long long q = gpo + g;
 #pragma unroll
@@ -508,80 +572,86 @@ __device__ __forceinline__ void hex_inverse_transform(const T (&m)[7], T (&f)[8]
   f[7] = mul2(q, sub2(Qpp, Ppp));
 }
 
-// GEO: the Gauss points' A^{-1} and det A come from the setup-time table
+// FP32: the Gauss points' A^{-1} and det A come from the setup-time table
 // (k_elem_geo; the reference likewise evaluates dN/dX and det J once, at
 // initialisation, ShapeFunctions.cpp:197-215) instead of being rebuilt from
-// the reference coordinates: `geo` is this element's column of the block's
-// shared-memory copy, value k of the 80-value record at geo[(k/4)*rs + k%4].
-template <class R, int MAT, bool GP, bool GEO>
+// the reference coordinates.  The characteristic length on the current
+// geometry first (volume / max face area,
+// CalculateCharacteristicLength_C3D8.cpp:6-29) so that the nodal values are
+// dead before the Gauss loop; the 2x2x2 Gauss sum of det(dx/dxi) is the exact
+// volume of the trilinear hexahedron.
+template <int MAT, bool GP>
+__device__ __forceinline__ void hex_element_f32(const float (&x)[8][3], const float (&u)[8][3],
+                                                const MatP<float> &mp, const float (&pc)[4],
+                                                const float (&a0)[3], float *hist, long long hs,
+                                                long long gs, int pass, float (&f)[8][3],
+                                                float &le, int &bad, const ElemArgs<float> &A,
+                                                long long gpo, const HexStream &st) {
+  float vol = 0;
+  // FP32: corners as (x, y) pairs + z; the current geometry's Hadamard
+  // coefficients give the six face areas as three opposite-face pairs
+  float2 xp[8], up[8];
+  float xz[8], uz[8];
+#pragma unroll
+  for (int a = 0; a < 8; ++a) {
+    up[a] = make_float2(u[a][0], u[a][1]);
+    uz[a] = u[a][2];
+    xp[a] = __fadd2_rn(make_float2(x[a][0], x[a][1]), up[a]);
+    xz[a] = x[a][2] + u[a][2];
+  }
+  float hcx[7][3];
+  {
+    float2 hcp[7];
+    float hcz[7];
+    hex_hadamard_x2(xp, xz, hcp, hcz);
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      hcx[k][0] = hcp[k].x;
+      hcx[k][1] = hcp[k].y;
+      hcx[k][2] = hcz[k];
+    }
+  }
+  // (0123, 4567): c1 = h0 -+ h4, c2 = h1 -+ h5, cD = h3 -+ h6;
+  // (0374, 1265): h1 -+ h3, h2 -+ h4, h5 -+ h6; (0154, 3267): h0 -+ h3, h2 -+ h5, h4 -+ h6
+  float amax = face_pair_area_max(hcx, 0, 4, 1, 5, 3, 6);
+  amax = fmaxf(amax, face_pair_area_max(hcx, 1, 3, 2, 4, 5, 6));
+  amax = fmaxf(amax, face_pair_area_max(hcx, 0, 3, 2, 5, 4, 6));
+  float2 hp[7], mc[7];
+  float hz[7], mz[7];
+  hex_hadamard_x2(up, uz, hp, hz);
+#pragma unroll
+  for (int k = 0; k < 7; ++k) {
+    mc[k] = make_float2(0.f, 0.f);
+    mz[k] = 0.f;
+  }
+  hex_gauss_loop_x2<MAT, GP>(hp, hz, mp, pc, a0, hist, hs, gs, pass, vol, mc, mz, bad, A, gpo,
+                             st);
+  le = vol / amax;
+  if (pass == kPassForce) {
+    float2 fp[8];
+    float fz[8];
+    hex_inverse_transform(mc, fp);
+    hex_inverse_transform(mz, fz);
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      f[a][0] = fp[a].x;
+      f[a][1] = fp[a].y;
+      f[a][2] = fz[a];
+    }
+  }
+}
+
+// The same in any precision with the Jacobian rebuilt at each Gauss point (the
+// allocation-free entry point, which keeps no table).
+template <class R, int MAT, bool GP>
 __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][3],
                                             const MatP<R> &mp, const R (&pc)[4],
                                             const R (&a0)[3], R *hist, long long hs,
                                             long long gs, int pass, R (&f)[8][3], R &le,
-                                            int &bad, const ElemArgs<R> &A, long long gpo,
-                                            const R *geo, int rs) {
+                                            int &bad, const ElemArgs<R> &A, long long gpo) {
   const bool dt_only = pass == kPassDt;
-  // characteristic length on the current geometry first (volume / max face
-  // area, CalculateCharacteristicLength_C3D8.cpp:6-29) so that the nodal
-  // values are dead before the Gauss loop; the 2x2x2 Gauss sum of
-  // det(dx/dxi) below is the exact volume of the trilinear hexahedron.
   R vol = 0;
   R m[7][3];
-  const R *gb = geo;
-  if constexpr (GEO && sizeof(R) == 4) {
-    // FP32: corners as (x, y) pairs + z; the current geometry's Hadamard
-    // coefficients give the six face areas as three opposite-face pairs
-    float2 xp[8], up[8];
-    float xz[8], uz[8];
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      up[a] = make_float2(u[a][0], u[a][1]);
-      uz[a] = u[a][2];
-      xp[a] = __fadd2_rn(make_float2(x[a][0], x[a][1]), up[a]);
-      xz[a] = x[a][2] + u[a][2];
-    }
-    float hcx[7][3];
-    {
-      float2 hcp[7];
-      float hcz[7];
-      hex_hadamard_x2(xp, xz, hcp, hcz);
-#pragma unroll
-      for (int k = 0; k < 7; ++k) {
-        hcx[k][0] = hcp[k].x;
-        hcx[k][1] = hcp[k].y;
-        hcx[k][2] = hcz[k];
-      }
-    }
-    // (0123, 4567): c1 = h0 -+ h4, c2 = h1 -+ h5, cD = h3 -+ h6;
-    // (0374, 1265): h1 -+ h3, h2 -+ h4, h5 -+ h6; (0154, 3267): h0 -+ h3, h2 -+ h5, h4 -+ h6
-    float amax = face_pair_area_max(hcx, 0, 4, 1, 5, 3, 6);
-    amax = fmaxf(amax, face_pair_area_max(hcx, 1, 3, 2, 4, 5, 6));
-    amax = fmaxf(amax, face_pair_area_max(hcx, 0, 3, 2, 5, 4, 6));
-    float2 hp[7], mc[7];
-    float hz[7], mz[7];
-    hex_hadamard_x2(up, uz, hp, hz);
-#pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      mc[k] = make_float2(0.f, 0.f);
-      mz[k] = 0.f;
-    }
-    hex_gauss_loop_x2<MAT, GP>(hp, hz, mp, pc, a0, hist, hs, gs, pass, vol, mc, mz, bad, A, gpo,
-                               gb, rs);
-    le = vol / amax;
-    if (pass == kPassForce) {
-      float2 fp[8];
-      float fz[8];
-      hex_inverse_transform(mc, fp);
-      hex_inverse_transform(mz, fz);
-#pragma unroll
-      for (int a = 0; a < 8; ++a) {
-        f[a][0] = fp[a].x;
-        f[a][1] = fp[a].y;
-        f[a][2] = fz[a];
-      }
-    }
-    return;
-  } else {
   R amax;
   {
     R xc[8][3];
@@ -597,12 +667,10 @@ __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][
     amax = fmax(amax, hex_face_area(xc, 3, 2, 6, 7));
   }
   R hx[7][3], hu[7][3];
-  if (!GEO) hex_hadamard(x, hx);
+  hex_hadamard(x, hx);
   hex_hadamard(u, hu);
 #pragma unroll
   for (int i = 0; i < 7; ++i) m[i][0] = m[i][1] = m[i][2] = 0;
-  // first pair of the current Gauss point in the geometry rows: value 10 g,
-  // at column 0 of a row for even g and column 2 for odd g
   // The loop is not unrolled: one Gauss point's code stays in the
   // instruction cache and its temporaries are the only ones live.
 #pragma unroll 1
@@ -611,21 +679,7 @@ __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][
     hex_gauss_point(g, xi, et, ze);
     const R ez = et * ze, xz = xi * ze, xe = xi * et;
     R Q[3][3], detA;  // Q = A^{-1}, A[i][d] = dX_d / dxi_i
-    if (GEO) {
-      typedef typename Pair<R>::T P2;
-      // values 10g .. 10g+9 as five pairs (a pair never straddles a row)
-      const int o1 = (g & 1) ? rs - 2 : 2;
-      const P2 q0 = *reinterpret_cast<const P2 *>(gb),
-               q1 = *reinterpret_cast<const P2 *>(gb + o1),
-               q2 = *reinterpret_cast<const P2 *>(gb + rs),
-               q3 = *reinterpret_cast<const P2 *>(gb + rs + o1),
-               q4 = *reinterpret_cast<const P2 *>(gb + 2 * rs);
-      gb += (g & 1) ? 3 * rs - 2 : 2 * rs + 2;
-      Q[0][0] = q0.x; Q[0][1] = q0.y; Q[0][2] = q1.x;
-      Q[1][0] = q1.y; Q[1][1] = q2.x; Q[1][2] = q2.y;
-      Q[2][0] = q3.x; Q[2][1] = q3.y; Q[2][2] = q4.x;
-      detA = q4.y;
-    } else {
+    {
       R Am[3][3], Ad[3][3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
@@ -664,7 +718,8 @@ __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][
       continue;
     }
     const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
-    Sym6<R> S = stress_at<R, MAT>(mp, D, Jm1, a0, hist + g * gs, hs, pc, sy, A.law);
+    Sym6<R> S = stress_at<R, MAT>(mp, D, Jm1, a0, hist + g * gs, hs, pc, sy, A.law,
+                                  HistGlobal<R>{hist + g * gs, hs});
     if (GP) {
       long long q = gpo + g;
 #pragma unroll
@@ -704,7 +759,6 @@ __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][
     }
   }
   le = vol / amax;
-  }
   if (pass == kPassForce) {
     // inverse transform: f_a = 1/8 sum_k sign_k(a) m_k
 #pragma unroll
@@ -734,7 +788,8 @@ __device__ __forceinline__ void tet_element(const R (&x)[4][3], const R (&u)[4][
                                             const MatP<R> &mp, const R (&pc)[4],
                                             const R (&a0)[3], R *hist, long long hs,
                                             int pass, R (&f)[4][3], R &le, int &bad,
-                                            const ElemArgs<R> &A, long long gpo, const R *hin) {
+                                            const ElemArgs<R> &A, long long gpo,
+                                            const HistShared<R> &hin) {
   const bool dt_only = pass != kPassForce;
   R Am[3][3], H[3][3];
 #pragma unroll
@@ -944,14 +999,15 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
   Slot4<R> *shU = shX + kMaxLocalNodes;
   R *shXs = reinterpret_cast<R *>(smem_raw);
   R *shUs = shXs + 3 * kMaxLocalNodes;
-  // [NC*3][blockDim] corner forces; FP32 C3D8: first the elements' reference
-  // geometry, [20][blockDim] x 4 values, in the same space (a barrier
-  // separates the last geometry read from the first corner-force write)
+  // [NC*3][blockDim] corner forces; C3D8: first the reference geometry (and
+  // history) as HexStream holds it in the same space (a barrier separates the
+  // last read from the first corner-force write)
   R *shF = PACK ? reinterpret_cast<R *>(shU + kMaxLocalNodes) : shUs + 3 * kMaxLocalNodes;
-  constexpr bool GEO = ET == 0 && sizeof(R) == 4;
+  constexpr bool GEO = ET == 0;  // (FP32: FP64 C3D8 elements run on k_hexgp)
+  constexpr int kStream = hist_comps(MAT) > 0 ? 40 + 2 * hist_comps(MAT) : 80;  // per element
   const int PE = blockDim.x;
   // the local CSR of the in-block assembly: offsets, then entries
-  uint16_t *shLp = reinterpret_cast<uint16_t *>(shF + (GEO ? 80 : NC * 3) * PE);
+  uint16_t *shLp = reinterpret_cast<uint16_t *>(shF + (GEO ? kStream : NC * 3) * PE);
   uint16_t *shLe = shLp + kMaxLocalNodes + 8;
   const int t = threadIdx.x;
   const int p = A.patch_begin + blockIdx.x;
@@ -964,13 +1020,18 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
   const int e = e0 + (act ? t : 0);
   const long long el = e - A.elem_begin;
   const long long gs = A.nelem, hs = (long long)NGP * A.nelem;
-  if (GEO && act) {
-    // 20 rows of 16 bytes, coalesced across the block, landing while the
-    // per-element loads and the slot staging below are in flight
-    const R *src = A.geo + 4 * el;
-    R *dst = shF + 4 * t;
-#pragma unroll 4
-    for (int r = 0; r < 20; ++r) cp_async16(dst + 4 * r * PE, src + 4 * r * gs);
+  // the first Gauss points' geometry (and the first one's history), landing
+  // while the per-element loads and the slot staging below are in flight
+  HexStream stream;
+  if constexpr (GEO) {
+    constexpr bool kHist = hist_comps(MAT) > 0;
+    stream = HexStream{shF + 4 * t, shF + 40 * PE + t, A.geo + 4 * el, gs, 4 * PE, kHist ? 1 : 3};
+    if (act) {
+#pragma unroll
+      for (int q = 0; q < (kHist ? 1 : 4); ++q) stream.geo_pair(q);
+      if (kHist && pass == kPassForce)
+        stream.template hist_point<hist_comps(MAT)>(0, A.hist + el, hs);
+    }
   }
   uint4 cv = make_uint4(0u, 0u, 0u, 0u);
   int pw = 0;
@@ -1076,16 +1137,11 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
     R *hist = A.hist ? A.hist + el : nullptr;
     R le;
     const long long gpo = A.gpbase + el * NGP;
-    if (ET == 0)
-      hex_element<R, MAT, GP, GEO>(
-          reinterpret_cast<const R(&)[8][3]>(x), reinterpret_cast<const R(&)[8][3]>(u), mp, pc,
-          a0, hist, hs, gs, pass, reinterpret_cast<R(&)[8][3]>(f), le, bad, A, gpo, shF + 4 * t,
-          4 * PE);
+    if constexpr (ET == 0)
+      hex_element_f32<MAT, GP>(x, u, mp, pc, a0, hist, hs, gs, pass, f, le, bad, A, gpo, stream);
     else
-      tet_element<R, MAT, GP>(reinterpret_cast<const R(&)[4][3]>(x),
-                              reinterpret_cast<const R(&)[4][3]>(u), mp, pc, a0, hist, hs,
-                              pass, reinterpret_cast<R(&)[4][3]>(f), le, bad, A, gpo,
-                              NH > 1 ? hin : nullptr);
+      tet_element<R, MAT, GP>(x, u, mp, pc, a0, hist, hs, pass, f, le, bad, A, gpo,
+                              HistShared<R>{hin, 1});
     if (!GEO && pass == kPassForce) {
 #pragma unroll
       for (int a = 0; a < NC; ++a)
@@ -1310,12 +1366,6 @@ __global__ void __launch_bounds__(kElemThreads) k_elem_strain(const ElemArgs<R> 
   element_green_strain<R, ET>(x, u, Es);
 #pragma unroll
   for (int k = 0; k < 6; ++k) Eout[6 * (long long)e + k] = double(Es[k]);
-}
-
-template <class R>
-size_t elem_smem_bytes(int ET, int PE) {
-  const int NC = ET == 0 ? 8 : 4;
-  return sizeof(R) * (6 * (size_t)kMaxLocalNodes + (size_t)NC * 3 * PE);
 }
 
 }  // namespace ftgpu

@@ -14,7 +14,7 @@ static int go(int gp, int nb, int th, size_t sm, cudaStream_t s, const ElemArgs<
   if (ET == 0 && (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64))
     return (int)cudaErrorInvalidDevice;
   if (ET == 0 && !opted[dev]) {
-    const int mx = (int)elem_smem_bytes_host<float>(0, kMaxPatchElems);
+    const int mx = (int)elem_smem_bytes_host<float>(0, MAT, kMaxPatchElems);
     for (cudaError_t e : {cudaFuncSetAttribute(k_elem<float, ET, MAT, true, false>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, mx),
                           cudaFuncSetAttribute(k_elem<float, ET, MAT, false, true>,

@@ -278,7 +278,8 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
       if ((MAT == 5 || MAT == 7) && !act)  // (its history is another element's)
         S = Sym6<R>{0, 0, 0, 0, 0, 0};
       else
-        S = stress_at<R, MAT>(mp, D, Jm1, a0, A.hist ? A.hist + sg : nullptr, GS, pc, sy, A.law);
+        S = stress_at<R, MAT>(mp, D, Jm1, a0, A.hist + sg, GS, pc, sy, A.law,
+                              HistGlobal<R>{A.hist + sg, GS});
       if (GP && act) {
         const long long q = A.gpbase + 8 * el + gp;
 #pragma unroll

@@ -61,13 +61,15 @@ inline size_t hexgp_smem_bytes(int PE) {
   return sizeof(R) * (8 * (size_t)kMaxLocalNodes + 24 * (size_t)PE);
 }
 
-// Dynamic shared memory of one element block: node X and u records (4
-// values each) for kMaxLocalNodes slots plus NC*3 corner forces per element, or for FP32
-// C3D8 the larger 80-value geometry record per element in the same space.
+// Dynamic shared memory of one element block: node X and u records (4 values
+// each) for kMaxLocalNodes slots plus NC*3 corner forces per element, or for
+// C3D8 (FP32) the larger geometry of all Gauss points, or of two pairs with
+// two points' history, in the same space.
 template <class R>
-inline size_t elem_smem_bytes_host(int etype, int PE) {
+inline size_t elem_smem_bytes_host(int etype, int mat, int PE) {
   const int NC = etype == 0 ? 8 : 4;
-  const size_t per_elem = etype == 0 ? 80 : (size_t)NC * 3;
+  const size_t hist = mat == 5 ? 18 : (mat == 7 ? 12 : 0);
+  const size_t per_elem = etype == 0 ? (hist ? 40 + 2 * hist : 80) : (size_t)NC * 3;
   const size_t slot_words = etype == 0 ? 8 : 6;  // packed records (C3D8) / component arrays
   return sizeof(R) * (slot_words * (size_t)kMaxLocalNodes + per_elem * PE) +
          (etype == 0 ? elem_csr_smem_bytes(NC, PE) : 0);
