@@ -319,8 +319,8 @@ struct ftgpu_model {
   int inj_n = 0;
   std::vector<int> inj_upos;  // compact index -> position in the caller's list
   std::vector<int> inj_group_n;  // listed elements per group (groups with none are skipped)
-  DBuf inj_cidx, inj_upos_d, inj_eref, inj_ps_old, inj_psxsr, inj_flags, inj_part, inj_part2,
-      inj_done, inj_state, inj_hist;
+  DBuf inj_cidx, inj_upos_d, inj_eref, inj_ps_old, inj_psxsr, inj_flags, inj_part, inj_state,
+      inj_run, inj_cand;
   // energy balance of the explicit loop (CheckEnergy), single instance only
   bool energy_on = false;
   DBuf du, fprev, epart, estate;
@@ -667,6 +667,9 @@ int launch_groups_t(ftgpu_model *m, int parity, int use_clock, double dt_direct,
         A.inj_ps_old = m->inj_ps_old.as<R>();
         A.inj_psxsr = m->inj_psxsr.as<R>();
         A.inj_part = m->inj_part.p;
+        A.inj_run = m->inj_run.as<InjuryRun>();
+        A.inj_cand = m->inj_cand.as<R>();
+        A.inj_n = m->inj_n;
       } else {
         mode = kLaunchPlain;
       }
@@ -878,14 +881,15 @@ __global__ void k_principal_strain(const double *E6, const int *order, long long
   shear[el] = 0.5 * (mx - mn);
 }
 
-// The listed elements' flags and last MPS in the caller's order
+// The listed elements' flags (with the last step's percentile lists) and last
+// MPS in the caller's order
 template <class R>
-__global__ void k_injury_out(const uint8_t *flags, const R *ps, const int *upos, int n, double *ps_out,
-                             int *flags_out) {
+__global__ void k_injury_out(const InjuryRun *run, const uint8_t *flags, const R *ps, const R *psxsr,
+                             const int *upos, int n, double *ps_out, int *flags_out) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const int j = upos[c];
-  flags_out[j] = flags[c];
+  flags_out[j] = inj_list_flags<R>(run, flags[c], ps[c], psxsr[c]);
   ps_out[j] = double(ps[c]);
 }
 
@@ -1293,50 +1297,24 @@ int ensure_gp(ftgpu_model *m) {
   return 0;
 }
 
-// One chunk: BEGIN, K x (element groups, node), the last node pass FINISH.
-// With prof, event-record nodes bracket every element pass and node pass
-// (events 2k / 2k+1 / 2k+2 around step k).
-constexpr int kInjHistWords = 2 * 8 * kRadixBins + 2;  // histograms + two counters
-
-template <class R>
-InjuryArgs<R> injury_args(ftgpu_model *m, int parity) {
-  InjuryArgs<R> A;
-  A.cidx = m->inj_cidx.as<int>();
-  A.upos = m->inj_upos_d.as<int>();
-  A.eref = m->inj_eref.as<int>();
-  A.ps_old = m->inj_ps_old.as<R>();
-  A.psxsr = m->inj_psxsr.as<R>();
-  A.flags = m->inj_flags.as<uint8_t>();
-  A.part = m->inj_part.as<InjuryPart>();
-  A.part2 = m->inj_part2.as<InjuryPart>();
-  A.done_blocks = m->inj_done.as<unsigned>();
-  A.state = m->inj_state.as<InjuryState>();
-  A.clock = m->clock.as<Clock>();
-  A.hist = m->inj_hist.as<unsigned>();
-  A.count = A.hist + 2 * 8 * kRadixBins;
-  A.n = m->inj_n;
-  A.parity = parity;
-  int np = 0;
-  for (auto &g : m->ps.groups) np += g.npatch;
-  A.npart = np;
-  return A;
-}
-
-// One step of the injury criteria after the element pass (whose force
-// launches of groups with listed elements updated the per-element criteria
-// and left each block's extremes, launch mode kLaunchInjury): the step's
-// extremes (which also clears the histograms), the radix passes of both
-// selections, the element lists and the running maxima.  Partials of patches
-// without listed elements keep their sentinel values.
+// The end of a step's injury criteria after the element pass (whose force
+// launches of groups with listed elements updated the per-element criteria,
+// left each block's extremes and appended the candidates of the percentiles).
+// Partials of patches without listed elements keep their sentinel values.
 template <class R>
 int launch_injury_t(ftgpu_model *m, int parity) {
-  const InjuryArgs<R> J = injury_args<R>(m, parity);
-  k_injury_reduce<R><<<(J.npart + kInjReduceSpan - 1) / kInjReduceSpan, 256, 0, m->stream>>>(J);
-  const int hb = std::min((m->inj_n + kInjThreads - 1) / kInjThreads, 512);
-  for (int pass = 0; pass < (int)sizeof(R); ++pass)
-    k_radix_hist<R><<<dim3(hb, 2), kInjThreads, 0, m->stream>>>(J, pass);
-  k_radix_list<R><<<hb, kInjThreads, 0, m->stream>>>(J);
-  k_radix_final<R><<<1, kRadixBins, 0, m->stream>>>(J);
+  InjuryArgs<R> A;
+  A.eref = m->inj_eref.as<int>();
+  A.cand = m->inj_cand.as<R>();
+  A.part = m->inj_part.as<InjuryPart>();
+  A.run = m->inj_run.as<InjuryRun>();
+  A.state = m->inj_state.as<InjuryState>();
+  A.clock = m->clock.as<Clock>();
+  A.n = m->inj_n;
+  A.parity = parity;
+  A.npart = 0;
+  for (auto &g : m->ps.groups) A.npart += g.npatch;
+  k_injury_select<R><<<3 * kInjCluster, kInjThreads, kInjSelectSmem, m->stream>>>(A);
   CK(cudaGetLastError());
   return 0;
 }
@@ -1345,6 +1323,9 @@ int launch_injury(ftgpu_model *m, int parity) {
   return is_fp64(m) ? launch_injury_t<double>(m, parity) : launch_injury_t<float>(m, parity);
 }
 
+// One chunk: BEGIN, K x (element groups, node), the last node pass FINISH.
+// With prof, event-record nodes bracket every element pass and node pass
+// (events 2k / 2k+1 / 2k+2 around step k).
 // Steps per chunk graph (even: the clock slots alternate with the step
 // parity, so a graph of an even number of steps fits any starting step).
 constexpr int kChunkSteps = 16;
@@ -1879,6 +1860,7 @@ int ftgpu_init_explicit(ftgpu_model *m, double reduction, double failure_dt, dou
     CK(cudaMemsetAsync(m->inj_psxsr.p, 0, m->inj_n * rb, m->stream));
     CK(cudaMemsetAsync(m->inj_flags.p, 0, m->inj_n, m->stream));
     CK(cudaMemsetAsync(m->inj_state.p, 0, sizeof(InjuryState), m->stream));
+    CK(cudaMemsetAsync(m->inj_run.p, 0, sizeof(InjuryRun), m->stream));
   }
   if (m->energy_on) {  // CheckEnergy's works start from zero with the loop
     CK(cudaMemsetAsync(m->du.p, 0, m->du.bytes, m->stream));
@@ -1954,8 +1936,7 @@ int ftgpu_launches_per_step(ftgpu_model *m) {
   if (m->surr)
     for (auto &x : m->ps.groups) g += 2 * (x.npatch > 0 && x.mat == 7);
   int inj = 0;
-  if (m->injury_on)  // (element work rides on the force pass) reduce, radix passes, list, final
-    inj = 1 + (is_fp64(m) ? 8 : 4) + 2;
+  if (m->injury_on) inj = 1;  // k_injury_select (element work rides on the force pass)
   // mixed precision without the energy balance: the node pass is
   // k_node_free plus k_node_step over the rest list (when it has nodes)
   const int split = (m->nkind.p && !m->energy_on && m->rest_n > 0) ? 1 : 0;
@@ -2048,9 +2029,12 @@ int ftgpu_set_injury(ftgpu_model *m, int n, const int *element_ids) {
   CKI(m->inj_psxsr.alloc(n * rb));
   CKI(m->inj_flags.alloc(n));
   CKI(m->inj_part.alloc(np * sizeof(InjuryPart)));
-  CKI(m->inj_part2.alloc(((np + kInjReduceSpan - 1) / kInjReduceSpan) * sizeof(InjuryPart)));
-  CKI(m->inj_done.alloc(sizeof(unsigned)));
-  CK(cudaMemset(m->inj_done.p, 0, sizeof(unsigned)));
+  CKI(m->inj_run.alloc(sizeof(InjuryRun)));
+  CK(cudaMemset(m->inj_run.p, 0, sizeof(InjuryRun)));
+  CKI(m->inj_cand.alloc(2 * (size_t)n * rb));
+  CK(cudaFuncSetAttribute(is_fp64(m) ? (const void *)k_injury_select<double>
+                                     : (const void *)k_injury_select<float>,
+                          cudaFuncAttributeMaxDynamicSharedMemorySize, kInjSelectSmem));
   {  // sentinel partials (no element) for the patches of groups never launched
     std::vector<InjuryPart> sp(np);
     for (auto &q : sp)
@@ -2067,7 +2051,6 @@ int ftgpu_set_injury(ftgpu_model *m, int n, const int *element_ids) {
     for (int k = 0; k < g.nelem; ++k) m->inj_group_n[gi] += cidx[g.elem_begin + k] >= 0;
   }
   CKI(m->inj_state.alloc(sizeof(InjuryState)));
-  CKI(m->inj_hist.alloc(kInjHistWords * sizeof(unsigned)));
   CK(cudaMemset(m->inj_ps_old.p, 0, n * rb));
   CK(cudaMemset(m->inj_psxsr.p, 0, n * rb));
   CK(cudaMemset(m->inj_flags.p, 0, n));
@@ -2087,12 +2070,13 @@ int ftgpu_get_injury(ftgpu_model *m, ftgpu_injury *out, int *flags, double *ps) 
   CKI(m->inj_out.bytes >= n * 12ull ? 0 : m->inj_out.alloc(n * 12ull));
   double *po = m->inj_out.as<double>();
   int *fo = reinterpret_cast<int *>(po + n);
-  if (is_fp64(m))
-    k_injury_out<double><<<(n + 255) / 256, 256, 0, m->stream>>>(
-        m->inj_flags.as<uint8_t>(), m->inj_ps_old.as<double>(), m->inj_upos_d.as<int>(), n, po, fo);
-  else
-    k_injury_out<float><<<(n + 255) / 256, 256, 0, m->stream>>>(
-        m->inj_flags.as<uint8_t>(), m->inj_ps_old.as<float>(), m->inj_upos_d.as<int>(), n, po, fo);
+  auto collect = [&](auto real) {
+    typedef decltype(real) R;
+    k_injury_out<R><<<(n + 255) / 256, 256, 0, m->stream>>>(
+        m->inj_run.as<InjuryRun>(), m->inj_flags.as<uint8_t>(), m->inj_ps_old.as<R>(),
+        m->inj_psxsr.as<R>(), m->inj_upos_d.as<int>(), n, po, fo);
+  };
+  is_fp64(m) ? collect(0.0) : collect(0.f);
   CK(cudaGetLastError());
   const HostDrain::Part parts[] = {{flags, fo, n * sizeof(int)}, {ps, po, n * sizeof(double)}};
   return m->drain.copy(m->device, m->stream, parts, 2);

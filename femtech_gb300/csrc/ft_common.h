@@ -69,6 +69,8 @@ enum { kErrInverted = 1, kErrDt = 2, kErrIndex = 4, kErrWait = 8 };
 
 constexpr int kSlotCsr = -2;  // NodeArgs::slot4 marker: more slots than the records hold
 
+struct InjuryRun;  // ft_injury.cuh
+
 template <class Real>
 struct ElemArgs {
   // patches
@@ -120,6 +122,9 @@ struct ElemArgs {
   uint8_t *inj_flags;         // [listed]
   Real *inj_ps_old, *inj_psxsr;
   void *inj_part;             // [patches] InjuryPart block extremes
+  InjuryRun *inj_run;         // running percentiles, last update, candidate counts
+  Real *inj_cand;             // [2][inj_n] values above the running percentiles
+  int inj_n;
 };
 
 enum { kPassForce = 0, kPassDt = 1, kPassSurrogateFeatures = 2 };

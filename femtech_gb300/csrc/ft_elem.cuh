@@ -181,7 +181,8 @@ struct HistShared {
 // history components of a law per Gauss point
 __host__ __device__ constexpr int hist_comps(int mat) { return mat == 5 ? 18 : (mat == 7 ? 12 : 0); }
 
-template <class R, int MAT, class HIN>
+// FFORM: the HGO family through F (FP32 tetrahedra, see mat_hgo_parts_f)
+template <class R, int MAT, bool FFORM = false, class HIN>
 __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][3], R Jm1,
                                              const R (&a0)[3], R *hist, long long hs,
                                              const R (&pc)[4], const float *sy,
@@ -197,7 +198,10 @@ __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][
     S = mat_linear(mp, D, Jm1);
   } else if (MAT == 4) {
     Sym6<R> Si, Sv;
-    mat_hgo_parts<R, false>(mp, D, Jm1, a0, Si, Sv);
+    if (FFORM)
+      mat_hgo_parts_f<R, false>(mp, D, Jm1, a0, Si, Sv);
+    else
+      mat_hgo_parts<R, false>(mp, D, Jm1, a0, Si, Sv);
     S = Sym6<R>{Si.xx + Sv.xx, Si.yy + Sv.yy, Si.zz + Sv.zz, Si.yz + Sv.yz, Si.xz + Sv.xz,
                 Si.xy + Sv.xy};
   } else if (MAT == 6) {
@@ -213,6 +217,8 @@ __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][
     Sym6<R> Si, Sv;
     if (MAT == 7 && sy != nullptr)
       goh_parts_surrogate(mp, D, Jm1, a0, sy, law, Si, Sv);
+    else if (FFORM)
+      mat_hgo_parts_f<R, MAT == 7>(mp, D, Jm1, a0, Si, Sv);
     else
       mat_hgo_parts<R, MAT == 7>(mp, D, Jm1, a0, Si, Sv);
     R sd[6] = {Si.xx, Si.yy, Si.zz, Si.yz, Si.xz, Si.xy};
@@ -836,7 +842,8 @@ __device__ __forceinline__ void tet_element(const R (&x)[4][3], const R (&u)[4][
   }
   if (!dt_only) {
     const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
-    Sym6<R> S = stress_at<R, MAT>(mp, D, Jm1, a0, hist, hs, pc, sy, A.law, hin);
+    Sym6<R> S =
+        stress_at<R, MAT, sizeof(R) == 4>(mp, D, Jm1, a0, hist, hs, pc, sy, A.law, hin);
     if (GP) {
 #pragma unroll
       for (int i = 0; i < 3; ++i)
@@ -893,18 +900,22 @@ __device__ __forceinline__ void element_green_strain(const R (&x)[ET == 0 ? 8 : 
                                                      R (&Es)[6]);
 
 // One listed element's injury update (the body of the reference's per-element
-// loop, ex5.cpp:1330-1383): principal strains of the averaged Green strain,
-// the sticky flags, the principal strain rate against the previous step, and
-// the thread's extremes.
+// loop, ex5.cpp:1330-1383): the list flags of the previous step's percentiles,
+// principal strains of the averaged Green strain, the sticky flags, the
+// principal strain rate against the previous step, the thread's extremes and
+// whether the two values (v[0], v[3]) exceed the running percentiles.
 template <class R>
 __device__ __forceinline__ void injury_element(const ElemArgs<R> &A, int c, const R (&Es)[6],
-                                               R dt, R (&v)[4], int (&jj)[4], int (&cc)[4]) {
+                                               R dt, R (&v)[4], int (&jj)[4], int (&cc)[4],
+                                               bool (&above)[2]) {
+  const InjuryRun *q = A.inj_run;
   R mx, mn, sh;
   principal_strains<R>(Es[0], Es[1], Es[2], Es[3], Es[4], Es[5], mx, mn, sh);
-  uint8_t f = A.inj_flags[c];
+  const R old = A.inj_ps_old[c];
+  uint8_t f = inj_list_flags<R>(q, A.inj_flags[c], old, q->upd[1] ? A.inj_psxsr[c] : R(0));
   if (mx > R(0.15)) f |= kInjMps15;
   if (mx > R(0.30)) f |= kInjMps30;
-  const R psr = (mx - A.inj_ps_old[c]) / dt;
+  const R psr = (mx - old) / dt;
   const R psxsr = mx * psr;
   if (psr > R(120)) f |= kInjPsr120;
   if (psxsr > R(28)) f |= kInjPsxsr28;
@@ -918,6 +929,21 @@ __device__ __forceinline__ void injury_element(const ElemArgs<R> &A, int c, cons
   const int up = A.inj_upos[c];
   jj[0] = jj[1] = jj[2] = jj[3] = up;
   cc[0] = cc[1] = cc[2] = cc[3] = c;
+  above[0] = mx > inj_run<R>(q, 0);
+  above[1] = psxsr > inj_run<R>(q, 1);
+}
+
+// A warp's values above a running percentile into the step's candidates (in
+// any order: only the values are selected from).  Every lane calls it.
+template <class R>
+__device__ __forceinline__ void injury_append(const ElemArgs<R> &A, int sel, bool has, R v) {
+  const unsigned b = __ballot_sync(0xffffffffu, has);
+  if (!b) return;
+  const int lane = threadIdx.x & 31, lead = __ffs(b) - 1;
+  unsigned at = 0;
+  if (lane == lead) at = atomicAdd(&A.inj_run->count[sel][0], (unsigned)__popc(b));
+  at = __shfl_sync(0xffffffffu, at, lead) + __popc(b & ((1u << lane) - 1u));
+  if (has && at < (unsigned)A.inj_n) A.inj_cand[(long long)sel * A.inj_n + at] = v;
 }
 
 // The block's injury extremes into *out: a butterfly per warp, then the warps
@@ -1103,6 +1129,7 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
   // max shear, max MPS x rate, with list position and compact index
   R iv[4] = {-r_inf<R>(), r_inf<R>(), -r_inf<R>(), -r_inf<R>()};
   int ij[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff}, ic[4] = {-1, -1, -1, -1};
+  bool above[2] = {false, false};  // of the running percentiles
   R f[NC][3];
   if (act) {
     int lc[NC];
@@ -1149,7 +1176,11 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
         for (int d = 0; d < 3; ++d) shF[(a * 3 + d) * PE + t] = f[a][d];
     }
     if (!skip) dte = dt_of<R>(le, mp);
-    if (INJ && ci >= 0) injury_element<R>(A, ci, Es, dt, iv, ij, ic);
+    if (INJ && ci >= 0) injury_element<R>(A, ci, Es, dt, iv, ij, ic, above);
+  }
+  if (INJ && pass == kPassForce) {
+    injury_append<R>(A, 0, above[0], iv[0]);
+    injury_append<R>(A, 1, above[1], iv[3]);
   }
   if (GEO && pass == kPassForce) {
     __syncthreads();  // every thread is done with its geometry rows

@@ -256,10 +256,11 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
         Es[k] = R(0.0625) * (Es[k] + shx(Es[k], 4));
       }
       const int ci = act && l8 == 0 ? A.inj_cidx[e] : -1;
+      R v[4] = {0, 0, 0, 0};
+      bool above[2] = {false, false};
       if (ci >= 0) {
-        R v[4];
         int vj[4], vc[4];
-        injury_element<R>(A, ci, Es, dt, v, vj, vc);
+        injury_element<R>(A, ci, Es, dt, v, vj, vc, above);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           if (inj_better(k, v[k], vj[k], iv[k], ij[k])) {
@@ -268,6 +269,8 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
             ic[k] = vc[k];
           }
       }
+      injury_append<R>(A, 0, above[0], v[0]);
+      injury_append<R>(A, 1, above[1], v[3]);
     }
     R G[3][3];
     {

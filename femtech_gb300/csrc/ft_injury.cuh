@@ -1,10 +1,21 @@
 // ft_injury.cuh -- per-step injury criteria of the brain drivers on the GPU
 // (examples/ex5/ex5.cpp:1311-1430, CalculateInjuryCriterions): principal
 // strains of the listed elements, running extremes, sticky threshold flags and
-// the largest 95th percentiles of MPS and of MPS x strain rate, by an exact
-// radix selection.
+// the largest 95th percentiles of MPS and of MPS x strain rate.
+//
+// Only a step whose percentile exceeds the running maximum changes anything,
+// and then the percentile is one of the values above that maximum.  So the
+// force pass, which forms the values, appends those above it to a candidate
+// list (some 5 % of the elements while a percentile grows, none while it does
+// not, all at a run's first step), and one launch ends the step:
+// k_injury_select takes the percentile's rank among the candidates by an exact
+// radix selection, a cluster of eight blocks per selection, and the extremes
+// from the patches' partials.  The
+// elements' list flags follow in the next force pass, which has the step's
+// values at hand (k_injury_out applies them when they are read).
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -36,8 +47,25 @@ struct InjuryPart {
   int c[4];     // compact index
 };
 
-constexpr int kInjThreads = 256;
-constexpr int kRadixBins = 256;
+// The running maxima of the two percentiles as the force pass compares with
+// them, and the last step's update: upd[sel] set when it took a new maximum v
+// (both also in FP32, exactly: they are values of the element precision)
+struct InjuryRun {
+  double run[2], v[2];
+  float runf[2], vf[2];
+  int upd[2];
+  unsigned count[2][32];  // candidates of the step ([sel][0]; a line each)
+};
+template <class R> __device__ __forceinline__ R inj_run(const InjuryRun *q, int sel);
+template <> __device__ __forceinline__ float inj_run<float>(const InjuryRun *q, int sel) { return q->runf[sel]; }
+template <> __device__ __forceinline__ double inj_run<double>(const InjuryRun *q, int sel) { return q->run[sel]; }
+template <class R> __device__ __forceinline__ R inj_thr(const InjuryRun *q, int sel);
+template <> __device__ __forceinline__ float inj_thr<float>(const InjuryRun *q, int sel) { return q->vf[sel]; }
+template <> __device__ __forceinline__ double inj_thr<double>(const InjuryRun *q, int sel) { return q->v[sel]; }
+
+constexpr int kInjThreads = 512;
+constexpr int kInjCluster = 8;            // blocks per selection
+constexpr int kInjSelectSmem = 96 << 10;  // a block's candidate keys on the chip
 
 // The listed elements are kept in group order ("compact" index c): element e
 // (group order) is listed when cidx[e] >= 0; upos[c] is its position in the
@@ -45,18 +73,12 @@ constexpr int kRadixBins = 256;
 // and eref[c] its reference id.
 template <class R>
 struct InjuryArgs {
-  const int *cidx;       // [E] compact index or -1
-  const int *upos;       // [n]
   const int *eref;       // [n]
-  R *ps_old, *psxsr;     // [n] compact order
-  uint8_t *flags;        // [n] compact order
-  InjuryPart *part;      // [patches] block extremes of the step
-  InjuryPart *part2;     // [reduction blocks] second level
-  unsigned *done_blocks; // finished reduction blocks (reset by the last one)
+  const R *cand;         // [2][n] the step's candidates
+  const InjuryPart *part;  // [patches] block extremes of the step
+  InjuryRun *run;
   InjuryState *state;
   const Clock *clock;    // clock[0] of the step (single instance)
-  unsigned *hist;        // [2 selections][passes][256], then [2] counters
-  unsigned *count;       // [2] elements at or above a new maximum
   int n, parity, npart;
 };
 
@@ -115,263 +137,215 @@ __device__ __forceinline__ bool inj_better(int k, V bv, int bj, V av, int aj) {
   return (k == 1) ? (bv < av || (bv == av && bj < aj)) : (bv > av || (bv == av && bj < aj));
 }
 
-// Best of each extreme over a range of partials, then over the threads of a
-// block (fixed tree); the result in slot 0 of the shared arrays.
-__device__ __forceinline__ void inj_block_best(const InjuryPart *part, int lo, int hi,
-                                               double (*sv)[256], int (*sj)[256],
-                                               int (*sc)[256]) {
-  double v[4] = {-1e300, 1e300, -1e300, -1e300};
-  int jj[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff}, cc[4] = {-1, -1, -1, -1};
-  for (int b = lo + threadIdx.x; b < hi; b += blockDim.x) {
-    const InjuryPart p = part[b];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (inj_better(k, p.v[k], p.j[k], v[k], jj[k])) {
-        v[k] = p.v[k];
-        jj[k] = p.j[k];
-        cc[k] = p.c[k];
+// The list flags of an element after the last step's update
+template <class R>
+__device__ __forceinline__ uint8_t inj_list_flags(const InjuryRun *q, uint8_t f, R ps, R psxsr) {
+  if (q->upd[0])
+    f = ps >= inj_thr<R>(q, 0) ? (f | kInjInMps95) : (f & (uint8_t)~kInjInMps95);
+  if (q->upd[1])
+    f = psxsr >= inj_thr<R>(q, 1) ? (f | kInjInMpsxsr95) : (f & (uint8_t)~kInjInMpsxsr95);
+  return f;
+}
+
+// The value of rank k = (int)(0.95 n) - 1 (rank 0 if negative) of a selection,
+// when it exceeds the running maximum: the n - count values at or below the
+// maximum come before every candidate.  Eight bits per pass over the
+// candidates' keys, each block of the cluster on its share; lanes with the
+// same bin add once (the strains of one tissue share their top bits), and
+// every block sums the eight histograms through distributed shared memory, so
+// one cluster barrier per pass suffices (the other buffer is cleared
+// meanwhile: its readers passed the barrier before).
+template <class R>
+__device__ __forceinline__ void injury_select(const InjuryArgs<R> &A, int sel, double time,
+                                              unsigned char *sm) {
+  typedef typename std::conditional<sizeof(R) == 8, uint64_t, uint32_t>::type K;
+  constexpr int KB = sizeof(K) * 8;
+  __shared__ unsigned hist[2][256], total[256];
+  __shared__ unsigned s_digit, s_below;
+  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int t = threadIdx.x, lane = t & 31;
+  const unsigned rank = cl.block_rank();
+  InjuryRun *q = A.run;
+  const unsigned c = min(q->count[sel][0], (unsigned)A.n);
+  const int k = max((int)(A.n * 0.95) - 1, 0), before = A.n - (int)c;
+  if (t < 256) hist[0][t] = 0;
+  cl.sync();  // every block has read the count
+  if (rank == 0 && t == 0) q->count[sel][0] = 0;
+  if (c == 0 || k < before) {  // (the same in every block)
+    if (rank == 0 && t == 0) q->upd[sel] = 0;
+    return;
+  }
+  const unsigned share = (c + kInjCluster - 1) / kInjCluster, lo = min(c, rank * share),
+                 cnt = min(c, lo + share) - lo;
+  const R *cand = A.cand + (long long)sel * A.n + lo;
+  K *keys = reinterpret_cast<K *>(sm);
+  const bool held = share * sizeof(K) <= (size_t)kInjSelectSmem;
+  if (held)  // (a thread reads back its own entries only)
+    for (unsigned j = t; j < cnt; j += kInjThreads) keys[j] = fkey(cand[j]);
+  unsigned krem = (unsigned)(k - before);
+  K prefix = 0;
+  for (int b = KB - 8, p = 0; b >= 0; b -= 8, p ^= 1) {
+    // the same trip count for every lane of a warp (for __match_any_sync)
+    for (unsigned j0 = 0; j0 < cnt; j0 += kInjThreads) {
+      const unsigned j = j0 + t;
+      unsigned bin = 256u;
+      if (j < cnt) {
+        const K key = held ? keys[j] : fkey(cand[j]);
+        if (b == KB - 8 || ((key ^ prefix) >> (b + 8)) == 0) bin = (unsigned)(key >> b) & 0xffu;
       }
-  }
+      if (__all_sync(0xffffffffu, bin == 256u)) continue;
+      const unsigned peers = __match_any_sync(0xffffffffu, bin);
+      if (bin < 256u && lane == __ffs(peers) - 1) atomicAdd(&hist[p][bin], __popc(peers));
+    }
+    cl.sync();
+    if (t < 256) {
+      unsigned x = 0;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    sv[k][threadIdx.x] = v[k];
-    sj[k][threadIdx.x] = jj[k];
-    sc[k][threadIdx.x] = cc[k];
-  }
-  __syncthreads();
-  for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h)
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (inj_better(k, sv[k][threadIdx.x + h], sj[k][threadIdx.x + h], sv[k][threadIdx.x],
-                       sj[k][threadIdx.x])) {
-          sv[k][threadIdx.x] = sv[k][threadIdx.x + h];
-          sj[k][threadIdx.x] = sj[k][threadIdx.x + h];
-          sc[k][threadIdx.x] = sc[k][threadIdx.x + h];
-        }
+      for (int r = 0; r < kInjCluster; ++r) x += *cl.map_shared_rank(&hist[p][t], r);
+      total[t] = x;
+      hist[p ^ 1][t] = 0;
+    }
     __syncthreads();
+    if (t < 32) {  // eight bins per lane: the bin that holds the remaining rank
+      unsigned h[8], sum = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        h[i] = total[8 * lane + i];
+        sum += h[i];
+      }
+      unsigned x = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      unsigned at = x - sum;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (krem >= at && krem < at + h[i]) {
+          s_digit = 8 * lane + i;
+          s_below = at;
+        }
+        at += h[i];
+      }
+    }
+    __syncthreads();
+    prefix |= (K)s_digit << b;
+    krem -= s_below;
+    __syncthreads();  // (s_digit, s_below before the next pass writes them)
+  }
+  cl.sync();  // no block leaves while another reads its histogram
+  if (rank != 0 || t != 0) return;
+  const double v = double(fkey_inv(prefix));
+  q->upd[sel] = 1;
+  q->v[sel] = q->run[sel] = v;
+  q->vf[sel] = q->runf[sel] = float(v);
+  const int count = (int)(c - ((unsigned)(k - before) - krem));  // candidates not below it
+  InjuryState *s = A.state;
+  if (sel == 0) {
+    s->mps95 = v;
+    s->mps95_time = time;
+    s->mps95_count = count;
+  } else {
+    s->mpsxsr95 = v;
+    s->mpsxsr95_time = time;
+    s->mpsxsr95_count = count;
   }
 }
 
-constexpr int kInjReduceSpan = 256;  // partials per reduction block
-
-// The step's extremes from the per-patch partials into the running state: each
-// block reduces kInjReduceSpan partials into part2[block]; the last block to
-// finish (counter in count[2]) reduces those in block order and updates the
-// state: a strictly better value takes the element and the time (the
-// reference's ordered loop with strict comparisons).  The last block also
-// clears the radix histograms and counters of the step.
+// The step's extremes from the per-patch partials into the running state: a
+// strictly better value takes the element and the time (the reference's
+// ordered loop with strict comparisons).  Values are compared as
+// order-preserving integers (FP64 compares issue once in 16 cycles).
 template <class R>
-__global__ void __launch_bounds__(256) k_injury_reduce(const InjuryArgs<R> A) {
-  __shared__ double sv[4][256];
-  __shared__ int sj[4][256], sc[4][256];
-  __shared__ bool last;
-  const int lo = blockIdx.x * kInjReduceSpan, hi = min(lo + kInjReduceSpan, A.npart);
-  inj_block_best(A.part, lo, hi, sv, sj, sc);
-  if (threadIdx.x == 0) {
-    InjuryPart q;
+__device__ __forceinline__ void injury_extremes(const InjuryArgs<R> &A, double time) {
+  uint64_t key[4] = {0, 0, 0, 0};
+  int jj[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff}, cc[4] = {-1, -1, -1, -1};
+  auto take = [&](int k, uint64_t x, int j, int c) {
+    if (x > key[k] || (x == key[k] && j < jj[k])) {
+      key[k] = x;
+      jj[k] = j;
+      cc[k] = c;
+    }
+  };
+  for (int b = threadIdx.x; b < A.npart; b += kInjThreads) {
+    const InjuryPart p = A.part[b];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      q.v[k] = sv[k][0];
-      q.j[k] = sj[k][0];
-      q.c[k] = sc[k][0];
+      // (a NaN -- the trigonometric roots just outside acos' domain -- is no extreme)
+      const uint64_t a = (uint64_t)__double_as_longlong(p.v[k]) & 0x7fffffffffffffffull;
+      if (a > 0x7ff0000000000000ull) continue;
+      const uint64_t x = fkey(p.v[k]);
+      take(k, k == 1 ? ~x : x, p.j[k], p.c[k]);
     }
-    A.part2[blockIdx.x] = q;
-    __threadfence();
-    last = atomicAdd(A.done_blocks, 1u) == gridDim.x - 1;
+  }
+  constexpr int NW = kInjThreads / 32;
+  __shared__ uint64_t sk[4][NW];
+  __shared__ int sj[4][NW], sc[4][NW];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  auto warp_best = [&]() {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t x = __shfl_xor_sync(0xffffffffu, key[k], o);
+        const int j = __shfl_xor_sync(0xffffffffu, jj[k], o);
+        const int c = __shfl_xor_sync(0xffffffffu, cc[k], o);
+        take(k, x, j, c);
+      }
+  };
+  warp_best();
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      sk[k][w] = key[k];
+      sj[k][w] = jj[k];
+      sc[k][w] = cc[k];
+    }
   }
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  inj_block_best(A.part2, 0, gridDim.x, sv, sj, sc);
-  for (int i = threadIdx.x; i < 2 * 8 * kRadixBins + 2; i += blockDim.x) A.hist[i] = 0;
-  if (threadIdx.x != 0) return;
-  *A.done_blocks = 0;
-  const Clock ck = A.clock[A.parity];
-  if (ck.done) return;
-  const double t = ck.time + ck.dt;
-  InjuryState s = *A.state;
-  double *val[4] = {&s.max_strain, &s.min_strain, &s.max_shear, &s.max_psxsr};
-  double *tim[4] = {&s.max_strain_time, &s.min_strain_time, &s.max_shear_time,
-                    &s.max_psxsr_time};
-  int *el[4] = {&s.max_strain_elem, &s.min_strain_elem, &s.max_shear_elem, &s.max_psxsr_elem};
+  if (w != 0) return;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int c = sc[k][0];
-    if (c < 0) continue;
-    const bool upd = (k == 1) ? (*val[k] > sv[k][0]) : (*val[k] < sv[k][0]);
+    key[k] = sk[k][lane % NW];  // (twice is once for a maximum)
+    jj[k] = sj[k][lane % NW];
+    cc[k] = sc[k][lane % NW];
+  }
+  warp_best();
+  if (lane != 0) return;
+  InjuryState *s = A.state;
+  double *val[4] = {&s->max_strain, &s->min_strain, &s->max_shear, &s->max_psxsr};
+  double *tim[4] = {&s->max_strain_time, &s->min_strain_time, &s->max_shear_time,
+                    &s->max_psxsr_time};
+  int *el[4] = {&s->max_strain_elem, &s->min_strain_elem, &s->max_shear_elem, &s->max_psxsr_elem};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (cc[k] < 0) continue;
+    const double v = fkey_inv(k == 1 ? ~key[k] : key[k]);
+    const bool upd = (k == 1) ? (*val[k] > v) : (*val[k] < v);
     if (upd) {
-      *val[k] = sv[k][0];
-      *el[k] = A.eref[c];
-      *tim[k] = t;
+      *val[k] = v;
+      *el[k] = A.eref[cc[k]];
+      *tim[k] = time;
     }
   }
-  ++s.steps;
-  *A.state = s;
+  ++s->steps;
 }
 
-// Radix selection of the value of rank k = (int)(0.95 n) - 1 (rank 0 if
-// negative) of sel = 0: ps_old, 1: psxsr, 8 bits per pass from the most
-// significant byte.  Every pass first recovers the digits fixed so far from
-// the histograms of the previous passes (the same in every block).
-// The digits fixed by the first `pass` histograms of a selection, recovered
-// by every block (blockDim.x == kRadixBins: thread t owns bin t): per pass a
-// block-wide scan of the 256 counts finds the bin holding the remaining rank
-// (the first bin whose cumulative count exceeds it).  The result is in
-// *prefix after the final barrier; `stage` is unused scratch kept for the
-// callers' layout.
-template <class K>
-__device__ __forceinline__ void block_radix_prefix(const unsigned *hist, int pass, int n,
-                                                   unsigned *stage, K *prefix) {
-  (void)stage;
-  constexpr int KB = sizeof(K) * 8;
-  __shared__ unsigned wsum[kRadixBins / 32];
-  __shared__ unsigned s_krem, s_below;
-  __shared__ int s_d;
-  __shared__ K s_pref;
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  if (t == 0) {
-    int k = (int)(n * 0.95) - 1;
-    if (k < 0) k = 0;
-    s_krem = (unsigned)k;
-    s_pref = 0;
-  }
-  for (int q = 0; q < pass; ++q) {
-    const unsigned c = hist[q * kRadixBins + t];
-    unsigned x = c;  // inclusive scan within the warp
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[w] = x;
-    if (t == 0) {
-      s_d = 0;
-      s_below = 0;
-    }
-    __syncthreads();
-    unsigned off = 0;
-#pragma unroll
-    for (int v = 0; v < kRadixBins / 32; ++v) off += v < w ? wsum[v] : 0u;
-    const unsigned incl = x + off, excl = incl - c, krem = s_krem;
-    if (excl <= krem && krem < incl) {
-      s_d = t;
-      s_below = excl;
-    }
-    __syncthreads();
-    if (t == 0) {
-      s_krem = krem - s_below;
-      s_pref |= (K)s_d << (KB - 8 * (q + 1));
-    }
-    __syncthreads();
-  }
-  if (t == 0) *prefix = s_pref;
-  __syncthreads();
-}
-
-// Histogram of the next digit of the keys that share the digits fixed so far.
-// The values cluster (strains of one tissue), so most keys fall into a few
-// bins: lanes of a warp with the same bin are merged (__match_any_sync) and one
-// of them adds the count to its warp's own sub-histogram.
+// The end of a step's criteria: clusters 0 and 1 the two percentiles, the
+// first block of cluster 2 the extremes.
 template <class R>
-__global__ void __launch_bounds__(kInjThreads) k_radix_hist(const InjuryArgs<R> A, int pass) {
-  const int sel = blockIdx.y;  // 0: MPS, 1: MPS x rate
-  typedef typename std::conditional<sizeof(R) == 8, uint64_t, uint32_t>::type K;
-  constexpr int KB = sizeof(K) * 8;
-  constexpr int kWarps = kInjThreads / 32;
-  if (A.clock[A.parity].done) return;
-  unsigned *hist = A.hist + (sel * (KB / 8)) * kRadixBins;
-  __shared__ unsigned sh[kWarps][kRadixBins];
-  __shared__ unsigned stage[(KB / 8) * kRadixBins];
-  __shared__ K s_prefix;
-  for (int i = threadIdx.x; i < kWarps * kRadixBins; i += blockDim.x) (&sh[0][0])[i] = 0;
-  block_radix_prefix<K>(hist, pass, A.n, stage, &s_prefix);  // digits fixed so far
-  const K prefix = s_prefix;
-  const R *val = sel == 0 ? A.ps_old : A.psxsr;
-  const K mask = pass == 0 ? K(0) : (K)(~K(0)) << (KB - 8 * pass);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // the same trip count for every lane of a warp (for __match_any_sync)
-  for (long long base = (long long)blockIdx.x * blockDim.x; base < A.n;
-       base += (long long)gridDim.x * blockDim.x) {
-    const long long j = base + threadIdx.x;
-    unsigned bin = 0xffffffffu;
-    if (j < A.n) {
-      const K key = fkey(val[j]);
-      if ((key & mask) == prefix) bin = (unsigned)(key >> (KB - 8 * (pass + 1))) & 0xffu;
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, bin);
-    if (bin != 0xffffffffu && lane == __ffs(peers) - 1) atomicAdd(&sh[warp][bin], __popc(peers));
-  }
-  __syncthreads();
-  unsigned *out = hist + pass * kRadixBins;
-  for (int i = threadIdx.x; i < kRadixBins; i += blockDim.x) {
-    unsigned c = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) c += sh[w][i];
-    if (c) atomicAdd(&out[i], c);
-  }
-}
-
-// The selected values; where one beats its running maximum, the listed
-// elements at or above it are marked (flag bit) and counted.  Both selections
-// in one pass per element, so each flag byte is written by one thread.
-template <class R>
-__global__ void __launch_bounds__(kInjThreads) k_radix_list(const InjuryArgs<R> A) {
-  typedef typename std::conditional<sizeof(R) == 8, uint64_t, uint32_t>::type K;
-  constexpr int KB = sizeof(K) * 8;
-  if (A.clock[A.parity].done) return;
-  __shared__ unsigned stage[(KB / 8) * kRadixBins];
-  __shared__ K s_prefix[2];
-  for (int sel = 0; sel < 2; ++sel)
-    block_radix_prefix<K>(A.hist + (sel * (KB / 8)) * kRadixBins, KB / 8, A.n, stage,
-                          &s_prefix[sel]);
-  const R v0 = fkey_inv(s_prefix[0]), v1 = fkey_inv(s_prefix[1]);
-  const bool up0 = double(v0) > A.state->mps95, up1 = double(v1) > A.state->mpsxsr95;
-  if (!up0 && !up1) return;
-  unsigned c0 = 0, c1 = 0;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < A.n; j += gridDim.x * blockDim.x) {
-    uint8_t f = A.flags[j];
-    if (up0) {
-      const bool in = A.ps_old[j] >= v0;
-      f = in ? (f | kInjInMps95) : (f & (uint8_t)~kInjInMps95);
-      c0 += in;
-    }
-    if (up1) {
-      const bool in = A.psxsr[j] >= v1;
-      f = in ? (f | kInjInMpsxsr95) : (f & (uint8_t)~kInjInMpsxsr95);
-      c1 += in;
-    }
-    A.flags[j] = f;
-  }
-  if (c0) atomicAdd(&A.count[0], c0);
-  if (c1) atomicAdd(&A.count[1], c1);
-}
-
-// Running maxima of the two percentiles (after k_radix_list of both).
-template <class R>
-__global__ void __launch_bounds__(kRadixBins) k_radix_final(const InjuryArgs<R> A) {
-  typedef typename std::conditional<sizeof(R) == 8, uint64_t, uint32_t>::type K;
-  constexpr int KB = sizeof(K) * 8;
+__global__ void __cluster_dims__(kInjCluster, 1, 1) __launch_bounds__(kInjThreads)
+    k_injury_select(const InjuryArgs<R> A) {
+  extern __shared__ __align__(16) unsigned char inj_sm[];
   const Clock ck = A.clock[A.parity];
   if (ck.done) return;
-  __shared__ unsigned stage[(KB / 8) * kRadixBins];
-  __shared__ K s_prefix[2];
-  for (int sel = 0; sel < 2; ++sel)
-    block_radix_prefix<K>(A.hist + (sel * (KB / 8)) * kRadixBins, KB / 8, A.n, stage,
-                          &s_prefix[sel]);
-  if (threadIdx.x != 0) return;
-  const double t = ck.time + ck.dt;
-  InjuryState s = *A.state;
-  for (int sel = 0; sel < 2; ++sel) {
-    const double v = double(fkey_inv(s_prefix[sel]));
-    double &mx = sel == 0 ? s.mps95 : s.mpsxsr95;
-    if (v > mx) {
-      mx = v;
-      (sel == 0 ? s.mps95_time : s.mpsxsr95_time) = t;
-      (sel == 0 ? s.mps95_count : s.mpsxsr95_count) = (int)A.count[sel];
-    }
-  }
-  *A.state = s;
+  const double time = ck.time + ck.dt;
+  const int job = blockIdx.x / kInjCluster;
+  if (job < 2)
+    injury_select<R>(A, job, time, inj_sm);
+  else if (blockIdx.x % kInjCluster == 0)
+    injury_extremes<R>(A, time);
 }
 
 }  // namespace ftgpu
