@@ -286,8 +286,10 @@ struct ftgpu_model {
   std::vector<InstParams> inst;
   bool inst_set = false;
   int patch_elems = 0;  // requested (0: default)
+  int sms = 152;
   int pe = 128;         // elements per patch, from choose_patches
   bool hexgp = false;   // C3D8 groups on the eight-lane pass
+  int step_pdl = 0;     // while capturing: the step is one chain of dependent launches
   int node_threads = 128;  // nodal block (4M block: 0.834 ms/step against 0.839 at 256)
   bool setup_done = false, init_done = false;
   PatchSet ps;
@@ -371,7 +373,8 @@ struct ftgpu_model {
   int prof_steps = 0;
   std::vector<cudaEvent_t> prof_ev;
   Clock *h_clock = nullptr;  // pinned
-  int *h_err = nullptr;
+  int *h_err = nullptr;          // [2] pinned
+  cudaEvent_t run_ev[2] = {};    // the clocks of a run's last two graphs are in h_clock
   // learned surrogate for material-7 groups
   ftgpu_surrogate *surr = nullptr;
   SurrogateLaw surr_law{};
@@ -388,6 +391,8 @@ struct ftgpu_model {
     for (cudaEvent_t e : prof_ev) cudaEventDestroy(e);
     if (h_clock) cudaFreeHost(h_clock);
     if (h_err) cudaFreeHost(h_err);
+    for (cudaEvent_t e : run_ev)
+      if (e) cudaEventDestroy(e);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (stream2) cudaStreamDestroy(stream2);
@@ -424,8 +429,11 @@ void drop_graphs(ftgpu_model *m) {
 }
 
 // Mixed-precision models of at most this many C3D8 elements take the
-// eight-lane element pass (ft_hexgp.cuh).
+// eight-lane element pass (ft_hexgp.cuh).  Step of an Ogden block, eight lanes
+// against one thread per element, us: 3,927 elements 10.9 / 16.1, 15,000 15.7 /
+// 16.6, 18,000 16.1 / 16.5, 22,500 19.4 / 18.2, 32,000 23.4 / 19.0.
 constexpr int kHexGpMixedMax = 20000;
+
 
 // The C3D8 pass and the elements per patch of a model (at set-up).  A given
 // patch size stands (FP64: at most 128).  The default is 128, and less where a
@@ -437,15 +445,14 @@ void choose_patches(ftgpu_model *m) {
   long long nh = 0;
   for (int t : m->etype) nh += t == FTGPU_C3D8;
   const long long nt = m->nE - nh;
+  cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
   m->hexgp = is_fp64(m) || (nh > 0 && nh <= kHexGpMixedMax);
   int pe = m->patch_elems > 0 ? m->patch_elems : 128;
   if (is_fp64(m)) pe = std::min(pe, 128);
   pe = std::max(32, std::min(pe, kMaxPatchElems));
   if (m->patch_elems <= 0 && (is_fp64(m) || (m->hexgp && nt == 0))) {
-    int sms = 152;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
     const int lo = nt > 0 ? 32 : 8, per_sm = nh > 0 ? 8 : 4;
-    while (pe > lo && m->nE < (long long)per_sm * sms * pe) pe /= 2;
+    while (pe > lo && m->nE < (long long)per_sm * m->sms * pe) pe /= 2;
   }
   m->pe = pe;
 }
@@ -548,11 +555,9 @@ NodeArgs node_args(ftgpu_model *m, int mode, int parity) {
 }
 
 template <class R, bool EN>
-void node_step_launch(long long nb, int th, cudaStream_t st, const NodeArgs &A) {
-  if (A.node_list)
-    k_node_step<R, EN, true><<<(unsigned)nb, th, 0, st>>>(A);
-  else
-    k_node_step<R, EN, false><<<(unsigned)nb, th, 0, st>>>(A);
+int node_step_launch(int pdl, long long nb, int th, cudaStream_t st, const NodeArgs &A) {
+  if (A.node_list) return launch_pdl(0, k_node_step<R, EN, true>, nb, th, 0, st, A);
+  return launch_pdl(pdl, k_node_step<R, EN, false>, nb, th, 0, st, A);
 }
 
 int launch_node(ftgpu_model *m, int mode, int parity) {
@@ -562,20 +567,20 @@ int launch_node(ftgpu_model *m, int mode, int parity) {
   const bool step = mode == kNodeFused || mode == kNodeFinish;
   const bool en = step && m->energy_on;
   const bool f64 = is_fp64(m);
-  auto node_step = [&](long long blocks, cudaStream_t st, const NodeArgs &B) {
+  auto node_step = [&](int pdl, long long blocks, cudaStream_t st, const NodeArgs &B) {
     if (f64)
-      en ? node_step_launch<double, true>(blocks, th, st, B)
-         : node_step_launch<double, false>(blocks, th, st, B);
-    else
-      en ? node_step_launch<float, true>(blocks, th, st, B)
-         : node_step_launch<float, false>(blocks, th, st, B);
+      return en ? node_step_launch<double, true>(pdl, blocks, th, st, B)
+                : node_step_launch<double, false>(pdl, blocks, th, st, B);
+    return en ? node_step_launch<float, true>(pdl, blocks, th, st, B)
+              : node_step_launch<float, false>(pdl, blocks, th, st, B);
   };
   const bool fork = step && m->rig_nodes > 0 && m->stream2;
+  const int pdl = m->step_pdl;
   if (step) {  // (with the fork, the rotation trigonometry moves to k_driven_step)
     NodeArgs S = A;
     if (fork) S.nrot = 0;
-    const long long nth = std::max<long long>(m->ninst, A.nkind ? (long long)m->fns.size() : 0);
-    k_step_scalars<<<(unsigned)((nth + 127) / 128), 128, 0, m->stream>>>(S);
+    const long long nth = step_scalar_fn0(m->ninst) + (A.nkind ? (long long)m->fns.size() : 0);
+    CKI(launch_pdl(pdl, k_step_scalars, (nth + 127) / 128, 128, 0, m->stream, S));
   }
   if (fork) {
     // fork: the driven nodes' motion (rigid bodies' integrator, rotation
@@ -590,17 +595,17 @@ int launch_node(ftgpu_model *m, int mode, int parity) {
     CK(cudaEventRecord(m->ev_fork, m->stream));
     CK(cudaStreamWaitEvent(m->stream2, m->ev_fork, 0));
     k_driven_step<<<(unsigned)m->ninst, 32, 0, m->stream2>>>(B);
-    node_step(nbr, m->stream2, B);
+    CKI(node_step(0, nbr, m->stream2, B));
     if (!f64 && !en && A.nkind) {  // every other node: the split, as below
       k_node_free<<<(unsigned)nb, th, 0, m->stream>>>(A);
       if (m->rest_n > 0) {
         NodeArgs C = A;
         C.node_list = m->rest_list.as<int>();
         C.nlist = m->rest_n;
-        node_step((m->rest_n + th - 1) / th, m->stream, C);
+        CKI(node_step(0, (m->rest_n + th - 1) / th, m->stream, C));
       }
     } else {
-      node_step(nb, m->stream, A);
+      CKI(node_step(0, nb, m->stream, A));
     }
     CK(cudaEventRecord(m->ev_join, m->stream2));
     CK(cudaStreamWaitEvent(m->stream, m->ev_join, 0));
@@ -613,15 +618,15 @@ int launch_node(ftgpu_model *m, int mode, int parity) {
     }
     if (!f64 && !en && A.nkind) {
       // free nodes on their lean kernel, the rest through k_node_step's list
-      k_node_free<<<(unsigned)nb, th, 0, m->stream>>>(A);
+      CKI(launch_pdl(pdl, k_node_free, nb, th, 0, m->stream, A));
       if (m->rest_n > 0) {
         NodeArgs B = A;
         B.node_list = m->rest_list.as<int>();
         B.nlist = m->rest_n;
-        node_step((m->rest_n + th - 1) / th, m->stream, B);
+        CKI(node_step(0, (m->rest_n + th - 1) / th, m->stream, B));
       }
     } else {
-      node_step(nb, m->stream, A);
+      CKI(node_step(pdl, nb, m->stream, A));
     }
   } else {
     if (mode == kNodeBegin && m->rigid_on)
@@ -676,6 +681,12 @@ int launch_groups_t(ftgpu_model *m, int parity, int use_clock, double dt_direct,
     }
     A.use_clock = use_clock;
     A.dt_direct = dt_direct;
+    // (A grid of one or two blocks per SM is not launched early: beside the
+    // node pass' blocks its own land unevenly, 30.4 against 24.3 us a step for
+    // 15,000 elements; from three per SM on it gains, 28.4 against 30.7 us for
+    // 64,000.  The eight-lane pass' many small blocks gain at every size.)
+    A.pdl = m->step_pdl && !m->surr &&
+            ((g.etype == 0 && m->hexgp) || g.npatch >= 3 * m->sms);
     // one element pass of this group: eight lanes or one thread per element
     auto elem = [&](int md, int pass) {
       return g.etype == 0 && m->hexgp
@@ -1281,7 +1292,7 @@ int setup_t(ftgpu_model *m) {
   if (m->h_clock) cudaFreeHost(m->h_clock);
   m->h_clock = nullptr;
   CK(cudaMallocHost((void **)&m->h_clock, sizeof(Clock) * std::max(2 * m->ninst, 2)));
-  if (!m->h_err) CK(cudaMallocHost((void **)&m->h_err, sizeof(int)));
+  if (!m->h_err) CK(cudaMallocHost((void **)&m->h_err, 2 * sizeof(int)));
   m->setup_done = true;
   m->init_done = false;
   drop_graphs(m);
@@ -1356,6 +1367,14 @@ int capture_chunk(ftgpu_model *m, int K, bool prof, bool open = true) {
     m->prof_ev.assign(2 * K + 1, nullptr);
     for (auto &e : m->prof_ev) CK(cudaEventCreate(&e));
   }
+  // Programmatic dependent launches where a step is one chain on the stream
+  // (no timing events, no second stream within it)
+  {
+    int nact = 0;
+    for (size_t gi = 0; gi < m->ps.groups.size(); ++gi)
+      nact += m->ps.groups[gi].npatch > 0 && !m->group_idle[gi];
+    m->step_pdl = !prof && nact == 1 && m->rig_nodes == 0 && !m->rigid_on;
+  }
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   int r = open ? launch_node(m, kNodeBegin, 0) : 0;
@@ -1369,6 +1388,7 @@ int capture_chunk(ftgpu_model *m, int K, bool prof, bool open = true) {
   }
   if (prof && !r) r = (int)cudaEventRecordWithFlags(m->prof_ev[2 * K], m->stream, cudaEventRecordExternal);
   cudaError_t ce = cudaStreamEndCapture(m->stream, &g);
+  m->step_pdl = 0;
   if (r) return fail(FTGPU_ERR_CUDA, std::string("capture launch: ") + cudaGetErrorString((cudaError_t)r));
   if (ce != cudaSuccess) return fail(FTGPU_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
   ce = cudaGraphInstantiate(&exec, g, 0);
@@ -1422,61 +1442,75 @@ int run_impl(ftgpu_model *m, int max_steps, int *steps_done, bool prof, double *
     CK(cudaEventCreate(&e1));
     CK(cudaEventRecord(e0, m->stream));
   }
-  // every launch advances each running instance by its steps (or ends it)
-  const long long max_chunks = (max_steps + 1) / 2 + 2;
+  // Every launch advances each running instance by its steps (or ends it).  Up
+  // to two graphs are on their way: the next one is launched before the host
+  // has read the clocks of the one before (a graph of an ended run moves
+  // nothing), so the GPU does not wait for the host between graphs.  The
+  // timing graph is read back one at a time.
+  const int deep = prof ? 1 : 2;
+  for (int k = 0; k < 2; ++k)
+    if (!m->run_ev[k]) CK(cudaEventCreateWithFlags(&m->run_ev[k], cudaEventDisableTiming));
   int rc = FTGPU_OK;
   long long prev = start0;
-  long long left = max_steps;  // most steps any running instance still has
-  for (long long c = 0; c < max_chunks; ++c) {
-    // the run's first graph opens with the half-step, the others continue
-    const bool open = c == 0;
-    cudaGraphExec_t g = prof ? m->prof_exec : open ? m->chunk_exec : m->cont_exec;
-    if (!prof && left < K) {
-      // the end of the run: the shortest even graph that covers it
-      const int Kt = (int)std::max<long long>(2, (left + 1) & ~1ll);
-      if (Kt < K) {
-        CKI(capture_chunk(m, Kt, false, open));
-        g = open ? m->tail_exec[Kt / 2] : m->tailc_exec[Kt / 2];
+  long long left = max_steps;  // most steps any running instance will still have
+  long long launched = 0, read = 0;
+  bool stop = false;
+  const Clock *last = m->h_clock;  // the newest clocks read
+  while (true) {
+    while (!stop && left > 0 && launched - read < deep) {
+      // the run's first graph opens with the half-step, the others continue
+      const bool open = launched == 0;
+      cudaGraphExec_t g = prof ? m->prof_exec : open ? m->chunk_exec : m->cont_exec;
+      int steps = K;
+      if (!prof && left < K) {
+        // the end of the run: the shortest even graph that covers it
+        const int Kt = (int)std::max<long long>(2, (left + 1) & ~1ll);
+        if (Kt < K) {
+          CKI(capture_chunk(m, Kt, false, open));
+          g = open ? m->tail_exec[Kt / 2] : m->tailc_exec[Kt / 2];
+          steps = Kt;
+        }
       }
+      const int k = (int)(launched & 1);
+      CK(cudaGraphLaunch(g, m->stream));
+      CK(cudaMemcpyAsync(m->h_clock + (size_t)k * ni, m->clock.p, sizeof(Clock) * ni,
+                         cudaMemcpyDeviceToHost, m->stream));
+      CK(cudaMemcpyAsync(m->h_err + k, m->err.p, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+      CK(cudaEventRecord(m->run_ev[k], m->stream));
+      ++launched;
+      left -= steps;
     }
-    CK(cudaGraphLaunch(g, m->stream));
-    CK(cudaMemcpyAsync(m->h_clock, m->clock.p, sizeof(Clock) * ni, cudaMemcpyDeviceToHost,
-                       m->stream));
-    CK(cudaMemcpyAsync(m->h_err, m->err.p, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
-    CK(cudaStreamSynchronize(m->stream));
+    if (read == launched) break;
+    const int k = (int)(read++ & 1);
+    CK(cudaEventSynchronize(m->run_ev[k]));
+    const Clock *ck = last = m->h_clock + (size_t)k * ni;
     if (prof) {
-      const long long taken = m->h_clock[0].step - prev;
-      for (long long k = 0; k < std::min<long long>(taken, K); ++k) {
+      const long long taken = ck[0].step - prev;
+      for (long long j = 0; j < std::min<long long>(taken, K); ++j) {
         float a = 0.f, b = 0.f;
-        CK(cudaEventElapsedTime(&a, m->prof_ev[2 * k], m->prof_ev[2 * k + 1]));
-        CK(cudaEventElapsedTime(&b, m->prof_ev[2 * k + 1], m->prof_ev[2 * k + 2]));
+        CK(cudaEventElapsedTime(&a, m->prof_ev[2 * j], m->prof_ev[2 * j + 1]));
+        CK(cudaEventElapsedTime(&b, m->prof_ev[2 * j + 1], m->prof_ev[2 * j + 2]));
         if (elem_ms) *elem_ms += a;
         if (node_ms) *node_ms += b;
       }
     }
-    prev = m->h_clock[0].step;
-    left = 0;
-    for (int i = 0; i < ni; ++i)
-      if (!m->h_clock[i].done)
-        left = std::max<long long>(left, m->inst[i].step_limit - m->h_clock[i].step);
-    if (*m->h_err & kErrInverted) {
-      rc = fail(FTGPU_ERR_INVERTED, "non-positive or non-finite Jacobian");
-      break;
-    }
-    if (*m->h_err & kErrWait) {
-      rc = fail(FTGPU_ERR_CUDA, "tensor-core inference gave up waiting");
-      break;
-    }
+    prev = ck[0].step;
+    if (stop) continue;  // (a graph behind the one that ended the run)
     bool all = true, dterr = false;
+    long long most = 0;
     for (int i = 0; i < ni; ++i) {
-      all &= m->h_clock[i].done != 0;
-      dterr |= (m->h_clock[i].done & 4) != 0;
+      all &= ck[i].done != 0;
+      dterr |= (ck[i].done & 4) != 0;
+      if (!ck[i].done) most = std::max<long long>(most, m->inst[i].step_limit - ck[i].step);
     }
-    if (dterr) {
+    if (m->h_err[k] & kErrInverted)
+      rc = fail(FTGPU_ERR_INVERTED, "non-positive or non-finite Jacobian");
+    else if (m->h_err[k] & kErrWait)
+      rc = fail(FTGPU_ERR_CUDA, "tensor-core inference gave up waiting");
+    else if (dterr)
       rc = fail(FTGPU_ERR_DT, "time step below FailureTimeStep");
-      break;
-    }
-    if (all) break;
+    stop = rc != FTGPU_OK || all;
+    if (launched == read) left = most;
   }
   if (device_ms) {
     CK(cudaEventRecord(e1, m->stream));
@@ -1487,7 +1521,7 @@ int run_impl(ftgpu_model *m, int max_steps, int *steps_done, bool prof, double *
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
   }
-  if (steps_done) *steps_done = (int)(m->h_clock[0].step - start0);
+  if (steps_done) *steps_done = (int)(last[0].step - start0);
   return rc;
 }
 

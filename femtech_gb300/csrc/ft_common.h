@@ -71,6 +71,16 @@ constexpr int kSlotCsr = -2;  // NodeArgs::slot4 marker: more slots than the rec
 
 struct InjuryRun;  // ft_injury.cuh
 
+// Programmatic dependent launch within a step: a kernel that may be launched
+// before its predecessor in the stream has ended calls step_wait() before it
+// reads what the predecessor writes, and only then step_release(), after which
+// its own successor may be launched.  So a successor's loads before its wait
+// run beside the predecessor alone: everything older has ended.
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void step_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <class Real>
 struct ElemArgs {
   // patches
@@ -108,6 +118,7 @@ struct ElemArgs {
   int ninst, parity;
   int patch_begin, npatch, elem_begin, nelem;
   int use_clock;              // 1: dt and done flags from the clock; 0: dt_direct
+  int pdl;                    // (host) launch as a programmatic dependent
   double dt_direct;
   long long gpbase;
   // learned surrogate of the material-7 isochoric stress (null when off):

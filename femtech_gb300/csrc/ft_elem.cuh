@@ -140,8 +140,9 @@ __device__ __forceinline__ void write_surrogate_features(const R (&D)[3][3], con
 }
 
 // Material 7 isochoric stress from the surrogate's output sy (inside the trust
-// region |E|_F^2 <= trust_e2), else from the plain law; volumetric part exact.
-template <class R>
+// region |E|_F^2 <= trust_e2), else from the plain law in the caller's form;
+// volumetric part exact.
+template <class R, bool FFORM>
 __device__ __forceinline__ void goh_parts_surrogate(const MatP<R> &mp, const R (&D)[3][3], R Jm1,
                                                     const R (&a0)[3], const float *sy,
                                                     const SurrogateLaw &law, Sym6<R> &Si,
@@ -151,7 +152,10 @@ __device__ __forceinline__ void goh_parts_surrogate(const MatP<R> &mp, const R (
   const R e2 = E[0] * E[0] + E[1] * E[1] + E[2] * E[2] +
                R(2) * (E[3] * E[3] + E[4] * E[4] + E[5] * E[5]);
   if (!(e2 <= R(law.trust_e2))) {
-    mat_hgo_parts<R, true>(mp, D, Jm1, a0, Si, Sv);
+    if (FFORM)
+      mat_hgo_parts_f<R, true>(mp, D, Jm1, a0, Si, Sv);
+    else
+      mat_hgo_parts<R, true>(mp, D, Jm1, a0, Si, Sv);
     return;
   }
   float x[kMlpUsedIn];
@@ -181,12 +185,14 @@ struct HistShared {
 // history components of a law per Gauss point
 __host__ __device__ constexpr int hist_comps(int mat) { return mat == 5 ? 18 : (mat == 7 ? 12 : 0); }
 
+// part: where the Ogden law's longer FP32 series finds its coefficients.
 // FFORM: the HGO family through F (FP32 tetrahedra, see mat_hgo_parts_f)
-template <class R, int MAT, bool FFORM = false, class HIN>
+template <class R, int MAT, bool FFORM = false, class HIN, class PART>
 __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][3], R Jm1,
                                              const R (&a0)[3], R *hist, long long hs,
                                              const R (&pc)[4], const float *sy,
-                                             const SurrogateLaw &law, const HIN &hin) {
+                                             const SurrogateLaw &law, const HIN &hin,
+                                             const PART &part) {
   Sym6<R> S;
   if (MAT == 0) {
     S = Sym6<R>{0, 0, 0, 0, 0, 0};
@@ -205,7 +211,7 @@ __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][
     S = Sym6<R>{Si.xx + Sv.xx, Si.yy + Sv.yy, Si.zz + Sv.zz, Si.yz + Sv.yz, Si.xz + Sv.xz,
                 Si.xy + Sv.xy};
   } else if (MAT == 6) {
-    S = mat_ogden(mp, D, Jm1);
+    S = mat_ogden(mp, D, Jm1, part);
   } else {  // 5 / 7: HGO family + Prony series (HGOIsotropicViscoelastic.cpp:98-159)
     constexpr int NT = MAT == 5 ? 2 : 1, NH = 6 * (NT + 1);
     // the point's whole history first: behind the stores of one component the
@@ -216,7 +222,7 @@ __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][
     for (int k = 0; k < NH; ++k) h[k] = hin(k);
     Sym6<R> Si, Sv;
     if (MAT == 7 && sy != nullptr)
-      goh_parts_surrogate(mp, D, Jm1, a0, sy, law, Si, Sv);
+      goh_parts_surrogate<R, FFORM>(mp, D, Jm1, a0, sy, law, Si, Sv);
     else if (FFORM)
       mat_hgo_parts_f<R, MAT == 7>(mp, D, Jm1, a0, Si, Sv);
     else
@@ -497,7 +503,8 @@ __device__ __forceinline__ void hex_gauss_loop_x2(const float2 (&hp)[7], const f
     const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
     const Sym6<float> S = stress_at<float, MAT>(
         mp, D, Jm1, a0, hist + g * gs, hs, pc, sy, A.law,
-        HistShared<float>{st.hist + (g & 1) * hist_comps(MAT) * (rs / 4), rs / 4});
+        HistShared<float>{st.hist + (g & 1) * hist_comps(MAT) * (rs / 4), rs / 4},
+        PartOfThread<float>{A.mats, A.epid, A.patch_elem_off, A.patch_begin});
     if (GP) {
       const long long q = gpo + g;
 #pragma unroll
@@ -725,7 +732,7 @@ __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][
     }
     const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
     Sym6<R> S = stress_at<R, MAT>(mp, D, Jm1, a0, hist + g * gs, hs, pc, sy, A.law,
-                                  HistGlobal<R>{hist + g * gs, hs});
+                                  HistGlobal<R>{hist + g * gs, hs}, PartAt<R>{&mp});
     if (GP) {
       long long q = gpo + g;
 #pragma unroll
@@ -843,7 +850,8 @@ __device__ __forceinline__ void tet_element(const R (&x)[4][3], const R (&u)[4][
   if (!dt_only) {
     const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
     Sym6<R> S =
-        stress_at<R, MAT, sizeof(R) == 4>(mp, D, Jm1, a0, hist, hs, pc, sy, A.law, hin);
+        stress_at<R, MAT, sizeof(R) == 4>(mp, D, Jm1, a0, hist, hs, pc, sy, A.law, hin,
+                                          PartOfThread<R>{A.mats, A.epid, A.patch_elem_off, A.patch_begin});
     if (GP) {
 #pragma unroll
       for (int i = 0; i < 3; ++i)
@@ -1086,6 +1094,8 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
     }
   }
   const Clock *ck = A.clock + A.parity * A.ninst + inst;
+  step_wait();  // the displacements and the clock are the node pass'
+  step_release();
   // the slot records go to shared memory by asynchronous copies, in flight
   // together (and with the C3D8 geometry rows) until the one wait below; the
   // padding word of a C3D8 coordinate record is never read

@@ -25,12 +25,10 @@ static int go(int gp, int nb, int th, size_t sm, cudaStream_t s, const ElemArgs<
     opted[dev] = true;
   }
   if (gp == kLaunchGaussPoints)
-    k_elem<float, ET, MAT, true, false><<<nb, th, sm, s>>>(A, dto);
-  else if (gp == kLaunchInjury)
-    k_elem<float, ET, MAT, false, true><<<nb, th, sm, s>>>(A, dto);
-  else
-    k_elem<float, ET, MAT, false, false><<<nb, th, sm, s>>>(A, dto);
-  return (int)cudaGetLastError();
+    return launch_pdl(A.pdl, k_elem<float, ET, MAT, true, false>, nb, th, sm, s, A, dto);
+  if (gp == kLaunchInjury)
+    return launch_pdl(A.pdl, k_elem<float, ET, MAT, false, true>, nb, th, sm, s, A, dto);
+  return launch_pdl(A.pdl, k_elem<float, ET, MAT, false, false>, nb, th, sm, s, A, dto);
 }
 
 template <int ET>

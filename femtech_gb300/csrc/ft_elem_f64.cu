@@ -8,12 +8,10 @@ namespace ftgpu {
 template <int MAT>
 static int go(int gp, int nb, int th, size_t sm, cudaStream_t s, const ElemArgs<double> &A, int dto) {
   if (gp == kLaunchGaussPoints)
-    k_elem<double, 1, MAT, true, false><<<nb, th, sm, s>>>(A, dto);
-  else if (gp == kLaunchInjury)
-    k_elem<double, 1, MAT, false, true><<<nb, th, sm, s>>>(A, dto);
-  else
-    k_elem<double, 1, MAT, false, false><<<nb, th, sm, s>>>(A, dto);
-  return (int)cudaGetLastError();
+    return launch_pdl(A.pdl, k_elem<double, 1, MAT, true, false>, nb, th, sm, s, A, dto);
+  if (gp == kLaunchInjury)
+    return launch_pdl(A.pdl, k_elem<double, 1, MAT, false, true>, nb, th, sm, s, A, dto);
+  return launch_pdl(A.pdl, k_elem<double, 1, MAT, false, false>, nb, th, sm, s, A, dto);
 }
 
 int launch_strain_f64(int etype, int nblocks, int threads, size_t smem, cudaStream_t s,

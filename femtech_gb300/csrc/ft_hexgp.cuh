@@ -162,13 +162,17 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
   const int s0 = A.patch_node_off[p], ns = A.patch_node_off[p + 1] - s0;
   const Clock *ck = A.clock + A.parity * A.ninst + inst;
   for (int i = t; i < ns; i += T) {
+    cp_async_small<sizeof(R)>(&shX[i].x, A.sX + s0 + i);
+    cp_async_small<sizeof(R)>(&shX[i].y, A.sX + A.S + s0 + i);
+    cp_async_small<sizeof(R)>(&shX[i].z, A.sX + 2 * A.S + s0 + i);
+  }
+  step_wait();  // the displacements and the clock are the node pass'
+  step_release();
+  for (int i = t; i < ns; i += T) {
     const R *us = A.sU + 4ll * (s0 + i);
 #pragma unroll
     for (int h = 0; h < (int)sizeof(Slot4<R>) / 16; ++h)
       cp_async16(reinterpret_cast<char *>(shU + i) + 16 * h, us + h * (16 / sizeof(R)));
-    cp_async_small<sizeof(R)>(&shX[i].x, A.sX + s0 + i);
-    cp_async_small<sizeof(R)>(&shX[i].y, A.sX + A.S + s0 + i);
-    cp_async_small<sizeof(R)>(&shX[i].z, A.sX + 2 * A.S + s0 + i);
   }
   // lane l of the element: bits, corner and Gauss point of these signs
   const int l8 = t & 7;
@@ -282,7 +286,7 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
         S = Sym6<R>{0, 0, 0, 0, 0, 0};
       else
         S = stress_at<R, MAT>(mp, D, Jm1, a0, A.hist + sg, GS, pc, sy, A.law,
-                              HistGlobal<R>{A.hist + sg, GS});
+                              HistGlobal<R>{A.hist + sg, GS}, PartAt<R>{&mp});
       if (GP && act) {
         const long long q = A.gpbase + 8 * el + gp;
 #pragma unroll
@@ -421,12 +425,10 @@ static_assert(8 * (8 * kMaxLocalNodes + 24 * 128) <= 48 * 1024,
 template <class R, int MAT>
 int hexgp_go(int gp, int nb, int th, size_t sm, cudaStream_t s, const ElemArgs<R> &A, int pass) {
   if (gp == kLaunchGaussPoints)
-    k_hexgp<R, MAT, true, false><<<nb, th, sm, s>>>(A, pass);
-  else if (gp == kLaunchInjury)
-    k_hexgp<R, MAT, false, true><<<nb, th, sm, s>>>(A, pass);
-  else
-    k_hexgp<R, MAT, false, false><<<nb, th, sm, s>>>(A, pass);
-  return (int)cudaGetLastError();
+    return launch_pdl(A.pdl, k_hexgp<R, MAT, true, false>, nb, th, sm, s, A, pass);
+  if (gp == kLaunchInjury)
+    return launch_pdl(A.pdl, k_hexgp<R, MAT, false, true>, nb, th, sm, s, A, pass);
+  return launch_pdl(A.pdl, k_hexgp<R, MAT, false, false>, nb, th, sm, s, A, pass);
 }
 
 template <class R>

@@ -8,6 +8,25 @@
 
 namespace ftgpu {
 
+// kernel<<<blocks, threads, smem, s>>>(args...), with pdl as a programmatic
+// dependent of its predecessor in the stream (step_wait / step_release in
+// ft_common.h).  Returns a cudaError_t value.
+template <class... P, class... Args>
+inline int launch_pdl(int pdl, void (*kernel)(P...), long long blocks, int threads, size_t smem,
+                      cudaStream_t s, const Args &...args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)blocks);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = pdl ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Launch modes of the element kernel (argument gp of launch_elem_*)
 enum { kLaunchPlain = 0, kLaunchGaussPoints = 1, kLaunchInjury = 2 };
 

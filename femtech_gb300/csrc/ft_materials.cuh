@@ -25,12 +25,12 @@ struct Sym6 {
   R xx, yy, zz, yz, xz, xy;
 };
 
-// Terms of the small-strain Ogden series: FP32 always sums 9; FP64 the
-// smallest of the listed counts that reaches its rounding at the strain at hand
+// Terms of the small-strain Ogden series: the smallest of the listed counts
+// that reaches the type's rounding at the strain at hand
 template <class R> struct OgdenSeries;
 template <> struct OgdenSeries<float> {
-  static constexpr int kMax = 9, kSteps = 1;
-  static constexpr int n[kSteps] = {9};
+  static constexpr int kMax = 20, kSteps = 2;
+  static constexpr int n[kSteps] = {9, 20};
 };
 template <> struct OgdenSeries<double> {
   static constexpr int kMax = 32, kSteps = 5;
@@ -86,7 +86,7 @@ inline MatP<R> make_matp(int mat, const double *pr) {
     const int n = k + 1;
     if (n != OgdenSeries<R>::n[step]) continue;
     // n terms while the spectral radius of 2E is below r, r the largest (at
-    // most 0.3 in FP32, 0.5 in FP64) whose truncation bound
+    // most 0.5) whose truncation bound
     // sum_{j > n} |b_j| (3 + 2 r) r^j stays below eps r (rounding of the leading
     // term; the 1 + 2 (1 + r) weighs A itself and tr B = tr(A + M + M A))
     auto tail = [&](double r) {
@@ -98,7 +98,7 @@ inline MatP<R> make_matp(int mat, const double *pr) {
       }
       return t;
     };
-    double lo = 0.0, hi = sizeof(R) == 4 ? 0.3 : 0.5;
+    double lo = 0.0, hi = 0.5;
     if (tail(hi) <= eps * hi) {
       lo = hi;
     } else {
@@ -109,6 +109,12 @@ inline MatP<R> make_matp(int mat, const double *pr) {
     }
     q.ser_r[step++] = float(lo * (1.0 - 1e-6));
   }
+  // FP32: the stress is a difference of terms 1/alpha larger.  For |alpha| >= 2
+  // the longer series is as exact as the eigen-decomposition (5e-8 to 9e-8
+  // against 7e-8 to 1.2e-7 of the stress, median over states at the bound);
+  // for smaller ones it would not be (alpha = 0.5: 2e-7 against 8e-8).
+  if (sizeof(R) == 4 && std::fabs(a) < 2.0)
+    for (int k = 1; k < OgdenSeries<R>::kSteps; ++k) q.ser_r[k] = q.ser_r[0];
   // J^(-alpha/3): |J - 1| up to 1/32, less where the tail would show
   double c = 1.0;
   const int nj = JPowSeries<R>::kMax;
@@ -284,9 +290,9 @@ struct CGreen {
   R I1, trM2, I2, I3, jj, Ca, Cb, Cg;
 };
 template <class R>
-__device__ __forceinline__ CGreen<R> cgreen(const R (&D)[3][3], R Jm1) {
+__device__ __forceinline__ CGreen<R> cgreen_of(const Sym6<R> &M, R Jm1) {
   CGreen<R> g;
-  g.M = two_E(D);
+  g.M = M;
   g.M2 = sym_mul(g.M, g.M);
   g.I1 = g.M.xx + g.M.yy + g.M.zz;
   g.trM2 = g.M2.xx + g.M2.yy + g.M2.zz;
@@ -302,6 +308,10 @@ __device__ __forceinline__ CGreen<R> cgreen(const R (&D)[3][3], R Jm1) {
   g.Ca = -g.I3 * g.Cg;
   g.Cb = -(1 + g.I1) * g.Cg;
   return g;
+}
+template <class R>
+__device__ __forceinline__ CGreen<R> cgreen(const R (&D)[3][3], R Jm1) {
+  return cgreen_of(two_E(D), Jm1);
 }
 // a I + b M + c M^2
 template <class R>
@@ -649,6 +659,13 @@ __device__ __forceinline__ void ogden_horner(const MatP<R> &m, const CGreen<R> &
     c = nc;
   }
 }
+// The spectral radius of M, at most |I1|/3 + sqrt(2/3 tr M^2), is within the
+// bound of step k's count of terms
+template <class R>
+__device__ __forceinline__ bool ogden_within(const MatP<R> &m, const CGreen<R> &g, int k) {
+  const float t = m.ser_r[k] - approx_abs(g.I1) * (1.f / 3.f);
+  return t > 0.f && approx_abs(g.trM2) * (2.f / 3.f) < t * t;
+}
 
 // ---- 6: small strain: with M = 2E = C - I the isochoric stress is
 //   S_iso = (2 mu/alpha) J^{-alpha/3} [C^{alpha/2-1} - tr(C^{alpha/2})/3 C^{-1}]
@@ -660,26 +677,10 @@ __device__ __forceinline__ void ogden_horner(const MatP<R> &m, const CGreen<R> &
 // Horner's scheme on the three coefficients of I, M and M^2 (three FMAs per
 // term; carrying the powers themselves takes six), and
 //   tr B = I1 + tr A + tr(M A),  tr M^3 = I1 (tr M^2 - I2) + 3 I3.
-// The spectral radius is at most |I1|/3 + sqrt(2/3 tr M^2).
+// ogden_series: the stress from X = a I + b M + c M^2, A = M X.
 template <class R>
-__device__ __forceinline__ Sym6<R> mat_ogden(const MatP<R> &m, const R (&D)[3][3], R Jm1) {
-  const CGreen<R> g = cgreen(D, Jm1);
-  const float i1 = approx_abs(g.I1) * (1.f / 3.f), f2 = approx_abs(g.trM2) * (2.f / 3.f);
-  auto within = [&](int k) {
-    const float t = m.ser_r[k] - i1;
-    return t > 0.f && f2 < t * t;
-  };
-  if (!within(OgdenSeries<R>::kSteps - 1)) return ogden_eigen(m, g.M, Jm1);
-  R a = 0, b = 0, c = 0;
-  if constexpr (sizeof(R) == 4) {
-    ogden_horner<0, 9>(m, g, a, b, c);
-  } else {
-    if (!within(3)) ogden_horner<24, 32>(m, g, a, b, c);
-    if (!within(2)) ogden_horner<16, 24>(m, g, a, b, c);
-    if (!within(1)) ogden_horner<12, 16>(m, g, a, b, c);
-    if (!within(0)) ogden_horner<8, 12>(m, g, a, b, c);
-    ogden_horner<0, 8>(m, g, a, b, c);
-  }
+__device__ __forceinline__ Sym6<R> ogden_series(const MatP<R> &m, const CGreen<R> &g, R Jm1, R a,
+                                                R b, R c) {
   const R Aa = c * g.I3, Ab = a - c * g.I2, Ag = b + c * g.I1;  // A = M X
   const R trM3 = g.I1 * (g.trM2 - g.I2) + R(3) * g.I3;
   const R trB = g.I1 + Aa * (R(3) + g.I1) + Ab * (g.I1 + g.trM2) + Ag * (g.trM2 + trM3);
@@ -699,6 +700,65 @@ __device__ __forceinline__ Sym6<R> mat_ogden(const MatP<R> &m, const R (&D)[3][3
   const R Jp = R(0.5) * m.K * g.jj;
   const R w = Jp - k0 * (1 + t);
   return cg_combine(g, k0 * (Aa - t) + Jp + w * g.Ca, k0 * Ab + w * g.Cb, k0 * Ag + w * g.Cg);
+}
+
+// A global load where it stands: the longer FP32 series' coefficients, and the
+// part they belong to, must not be loaded ahead of the branch and kept in
+// registers through the Gauss loop
+__device__ __forceinline__ float load_here(const float *p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int load_here(const int *p) {
+  int v;
+  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+// Where the longer series finds its coefficients
+template <class R>
+struct PartAt {  // a part in hand
+  const MatP<R> *mp;
+  __device__ __forceinline__ const R *ser() const { return mp->ser_a; }
+};
+template <class R>
+struct PartOfThread {  // the part of element (patch, thread), found again
+  const MatP<R> *mats;
+  const int *epid, *patch_elem_off;
+  int patch_begin;
+  __device__ __forceinline__ const R *ser() const {
+    const int e = load_here(patch_elem_off + patch_begin + (int)blockIdx.x) + (int)threadIdx.x;
+    return mats[load_here(epid + e) & 0x7fffffff].ser_a;
+  }
+};
+
+template <class R, class PART>
+__device__ __forceinline__ Sym6<R> mat_ogden(const MatP<R> &m, const R (&D)[3][3], R Jm1,
+                                             const PART &part) {
+  const CGreen<R> g = cgreen(D, Jm1);
+  R a = 0, b = 0, c = 0;
+  if constexpr (sizeof(R) == 4) {
+    if (!ogden_within(m, g, 0)) {
+      if (!ogden_within(m, g, 1)) return ogden_eigen(m, g.M, Jm1);
+      const R *ser = part.ser();
+#pragma unroll
+      for (int k = 19; k >= 9; --k) {
+        const R na = c * g.I3 + load_here(ser + k), nb = a - c * g.I2, nc = b + c * g.I1;
+        a = na;
+        b = nb;
+        c = nc;
+      }
+    }
+    ogden_horner<0, 9>(m, g, a, b, c);
+  } else {
+    if (!ogden_within(m, g, 4)) return ogden_eigen(m, g.M, Jm1);
+    if (!ogden_within(m, g, 3)) ogden_horner<24, 32>(m, g, a, b, c);
+    if (!ogden_within(m, g, 2)) ogden_horner<16, 24>(m, g, a, b, c);
+    if (!ogden_within(m, g, 1)) ogden_horner<12, 16>(m, g, a, b, c);
+    if (!ogden_within(m, g, 0)) ogden_horner<8, 12>(m, g, a, b, c);
+    ogden_horner<0, 8>(m, g, a, b, c);
+  }
+  return ogden_series(m, g, Jm1, a, b, c);
 }
 
 }  // namespace ftgpu

@@ -62,7 +62,13 @@ __device__ __forceinline__ void bc_value(const BcFn &b, int d, double t, const d
   switch (b.kind) {
     case kBckFixed: u = b.p[0]; v = 0.0; break;
     case kBckRamp: u = t * b.p[0]; v = b.p[0]; break;
-    case kBckSine: u = b.p[0] * sin(b.p[1] * t); v = b.p[0] * b.p[1] * cos(b.p[1] * t); break;
+    case kBckSine: {
+      double sn, cs;
+      sincos(b.p[1] * t, &sn, &cs);
+      u = b.p[0] * sn;
+      v = b.p[0] * b.p[1] * cs;
+      break;
+    }
     default: {  // rigid rotation about a fixed axis
       double th, om;
       rot_angle(b.p, t, th, om);
@@ -472,20 +478,29 @@ __global__ void __launch_bounds__(512, 2) k_node(const NodeArgs A) {
 
 }
 
+// First function thread of k_step_scalars: the instances' warps come before
+__host__ __device__ inline int step_scalar_fn0(int ninst) { return (ninst + 31) / 32 * 32; }
+
 // Step scalars of every instance for one end-of-step launch: the new dt from
 // the dt minimum, the time levels, the velocity coefficients, the done flags
 // and the trigonometry of the rigid-rotation functions at the new time.  One
 // thread per instance, launched between the element pass and k_node_step, so
 // that the FP64 divisions and sin/cos run once per instance and step rather
 // than once per node block (FP64 issue is slow on this GPU).
-// With the node-pass split, thread i also evaluates boundary function i once
-// for the step when its value is the same for every node (fixed, ramp, sine)
+// With the node-pass split, further threads evaluate each boundary function
+// once for the step when its value is the same for every node (fixed, ramp, sine)
 // and one instance owns it (BcFn::pad): u and v at that instance's t_{n+2},
 // the values node_step's bc_value would compute per DOF.
+// Warps of instances first, then warps of functions, so that one thread's
+// sine does not stand before its clock.
 __global__ void k_step_scalars(const NodeArgs A) {
+  step_wait();  // the dt minimum is the element pass'
+  step_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (A.fnval && i < A.nfns) {
-    const BcFn &b = A.fns[i];
+  const int f = i - step_scalar_fn0(A.ninst);
+  if (f >= 0) {
+    if (!A.fnval || f >= A.nfns) return;
+    const BcFn &b = A.fns[f];
     if (b.kind <= kBckSine && b.pad >= 0) {
       const int o = b.pad;
       const Clock co = A.clock[A.parity * A.ninst + o];
@@ -494,9 +509,10 @@ __global__ void k_step_scalars(const NodeArgs A) {
       if (so.advance && !co.done) {
         double u, v;
         bc_value(b, 0, so.t_np2, A.X, A.N, 0, u, v);
-        A.fnval[i] = make_double2(u, v);
+        A.fnval[f] = make_double2(u, v);
       }
     }
+    return;
   }
   if (i >= A.ninst) return;
   const Clock ck = A.clock[A.parity * A.ninst + i];
@@ -674,6 +690,8 @@ __device__ __forceinline__ void node_step(const NodeArgs &A, long long n, R &eke
     u0[d] = A.u[d * N + n];
     vh0[d] = A.vh[d * N + n];
   }
+  step_wait();  // the partial forces and the step scalars are its predecessors'
+  step_release();
   const bool anybc = nbc[0] != kBcFree || nbc[1] != kBcFree || nbc[2] != kBcFree;
   if (anybc && A.skip_driven) {  // handled by the driven-node branch of the step
 #pragma unroll
@@ -860,6 +878,8 @@ __global__ void __launch_bounds__(512, 2) k_node_free(const NodeArgs A) {
     vh0[d] = A.vh[d * N + n];
   }
   const float minv = __ldg(A.minv + n);
+  step_wait();  // the partial forces and the step scalars are its predecessors'
+  step_release();
   if (kind & kNodeRest) return;
   int fn[3] = {kBcFree, kBcFree, kBcFree};
   if (kind & kNodeBcCached) {
