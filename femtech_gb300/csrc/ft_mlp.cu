@@ -415,30 +415,35 @@ __global__ void __launch_bounds__(256) k_mlp_infer(const bf16 *__restrict__ X, l
 }
 
 // ---------------- fused inference on the 5th-generation tensor cores ----------------
-// A persistent, warp-specialised kernel: one CTA per SM stages the weights
-// once and keeps three 128-row tiles in flight, one per *slot* (13 warps: the
-// register file is split over the SM's four schedulers, and 4 warps of 128
-// registers fill one scheduler's share).  Slot s owns an
-// input image, an activation image and TMEM columns [128 s, 128 s + 128); row r
-// of its tile is TMEM lane r.  Warps 4s .. 4s+3 are the slot's epilogue (warp
-// 4s + q reaches lanes 32 q .. 32 q + 31); warp 12 issues every MMA from one
-// thread.  Per layer the slot's epilogue makes its operand visible and
-// arrives on full[s]; the MMA thread waits on full[s], issues the layer
-// (tcgen05.mma, M = 128, K = 16 per instruction, BF16 x BF16 -> FP32) and
-// commits to done[s]; the epilogue waits on done[s], reads the accumulator
-// (tcgen05.ld), applies SiLU and writes the BF16 activations as the next
-// layer's A operand.  While one slot runs its epilogue the tensor core serves
-// the others.  The biases ride in the MMAs: every activation image carries
-// two constant columns of ones (columns 128, 129 of a K = 144 image; input
-// columns 14, 15, unused features) against the bias split into a BF16 high
-// part and the BF16 rounding of the rest (b = hi + lo to 2^-16) in the weight
-// images -- one more K = 16 MMA per hidden layer (the tensor core is mostly
-// idle) instead of a 128-column TMEM store per row and layer.  W0..W2 and
-// b0..b2 are staged times 1/2 (exact), so an accumulator holds h = z / 2 and
-// SiLU(z) = z sigmoid(z) = h + h tanh(h) is evaluated on BF16 pairs: one
-// MUFU tanh and one FMA per two values.
-// Every wait is bounded; a wait that gives
-// up raises a shared abort flag that ends all roles, and the error word.
+// A persistent kernel: one CTA per SM loads the weights once, as the operand
+// images that k_infer_image laid out when they last changed (one bulk copy),
+// and keeps four 128-row tiles in flight, one per *slot* of four warps.  Slot s
+// owns an activation image and TMEM columns [128 s, 128 s + 128); row r of its
+// tile is TMEM lane r (warp q of the slot reaches lanes 32 q .. 32 q + 31).
+// Per layer the slot's warps write its operand (the input rows, then the
+// activations over them), make it visible and arrive on full[s]; the slot's
+// first thread waits on full[s], issues the layer (tcgen05.mma, M = 128,
+// K = 16 per instruction, BF16 x BF16 -> FP32) and commits to done[s]; all
+// wait on done[s], read the accumulator (tcgen05.ld) and apply SiLU.  The slots share nothing but the
+// weights, so while one runs its epilogue the tensor core serves whichever is
+// ready.  The biases ride in the MMAs: one more K = 16 step per hidden layer
+// multiplies a constant image of two columns of ones (input columns 14, 15,
+// unused features, for the first layer) by the bias split into a BF16 high
+// part and the BF16 rounding of the rest (b = hi + lo to 2^-16).  W0..W2 and
+// b0..b2 are laid out times 1/2 (exact), so an accumulator holds h = z / 2 and
+// SiLU(z) = z sigmoid(z) = h + h tanh(h) is evaluated on BF16 pairs: one MUFU
+// tanh and one FMA per two values.
+// Every wait is bounded; a wait that gives up raises a shared abort flag that
+// ends all slots, and the error word.
+//
+// What bounds it: the chain of a layer (operand fence, arrival, nine MMAs,
+// commit, TMEM loads, SiLU), 5,600 SM cycles per tile with four in flight
+// against 1,536 of MUFU and 1,360 of the tensor core; chunks of 16 columns with
+// the next on its way measured the same.  Three slots with a thirteenth warp
+// issuing for all of them in turn (a slot behind an unfinished one waited for
+// it), 128 arrivals per operand and the weights laid out by every CTA at every
+// launch took 33 us for 165,000 rows, this 29 us; in-loop steps of 30,000 /
+// 200,000 / 2,000,000 tetrahedra 41.1 / 67.9 / 398.6 -> 34.8 / 65.6 / 371.8 us.
 //
 // Shared-memory operand images are K-major without swizzle: 8-row x 16-byte
 // core matrices, element (r, k) of an image with K columns at byte
@@ -446,21 +451,23 @@ __global__ void __launch_bounds__(256) k_mlp_infer(const bf16 *__restrict__ X, l
 // i.e. leading-dimension (K-direction) byte offset 128 and stride-dimension
 // (8-row group) byte offset 16 K in the matrix descriptors.
 namespace tc {
-constexpr int kSlots = 3;
-constexpr int kMmaWarp = 4 * kSlots;               // warp 12
-constexpr int kThreads = 32 * (kMmaWarp + 1);      // 416: at most 4 warps per SMSP
-constexpr int kKH = kMlpHid + 16;                  // hidden K plus the bias columns (144)
-constexpr uint32_t kSBOH = 16 * kKH;               // 8-row group stride of a K = 144 image
-constexpr uint32_t kW0 = 0;                        // [128 x 16]     4 KB (bias in columns 14, 15)
-constexpr uint32_t kW1 = kW0 + 128 * 16 * 2;       // [128 x 144]   36 KB
-constexpr uint32_t kW2 = kW1 + 128 * kKH * 2;      // [128 x 144]   36 KB
-constexpr uint32_t kW3 = kW2 + 128 * kKH * 2;      // [16 x 144]   4.5 KB (rows 8..15 zero)
-constexpr uint32_t kXs = kW3 + 16 * kKH * 2;       // per slot [128 x 16]    4 KB
-constexpr uint32_t kHs = kXs + kSlots * 4096;      // per slot [128 x 144]  36 KB
-constexpr uint32_t kBar = kHs + kSlots * 128 * kKH * 2;  // full[], done[], TMEM base, abort
-constexpr uint32_t kSmem = kBar + 72 + 128;        // + alignment slack of the base
-constexpr uint32_t kTmemCols = 512;               // 128 per slot, rounded to a power of 2
+constexpr int kSlots = 4;
+constexpr int kThreads = 128 * kSlots;
+constexpr uint32_t kW0 = 0;                        // [128 x 16]   4 KB (bias in columns 14, 15)
+constexpr uint32_t kW1 = kW0 + 128 * 16 * 2;       // [128 x 128] 32 KB
+constexpr uint32_t kW2 = kW1 + 128 * 128 * 2;      // [128 x 128] 32 KB
+constexpr uint32_t kW3 = kW2 + 128 * 128 * 2;      // [16 x 128]   4 KB (rows 8..15 zero)
+constexpr uint32_t kB1 = kW3 + 16 * 128 * 2;       // [128 x 16]   4 KB (hi, lo, zeros)
+constexpr uint32_t kB2 = kB1 + 128 * 16 * 2;       // [128 x 16]   4 KB
+constexpr uint32_t kB3 = kB2 + 128 * 16 * 2;       // [16 x 16]   0.5 KB
+constexpr uint32_t kOne = kB3 + 16 * 16 * 2;       // [128 x 16]   4 KB (ones in columns 0, 1)
+constexpr uint32_t kImage = kOne + 128 * 16 * 2;   // the weights' images (84.5 KB)
+constexpr uint32_t kHs = kImage;                   // per slot [128 x 128] 32 KB; first [128 x 16]
+constexpr uint32_t kBar = kHs + kSlots * 128 * 128 * 2;  // full[], done[], weights, TMEM, abort
+constexpr uint32_t kSmem = kBar + 80 + 128;        // + alignment slack of the base
+constexpr uint32_t kTmemCols = 128 * kSlots;
 constexpr int kWaitLimit = 1 << 21;                // try_wait rounds before giving up
+static_assert(kSmem <= 232448, "fits an SM's shared memory");
 }  // namespace tc
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -534,14 +541,12 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-      "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
       "tcgen05.wait::ld.sync.aligned;\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr)
       : "memory");
 #pragma unroll
@@ -563,224 +568,205 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// A row-major BF16 weight matrix [rows x Ks] (times `scale`) into a K-major
-// core-matrix image with K = Ks + 16 whose columns Ks, Ks + 1 hold the bias
-// (times `scale`) as a BF16 high part and the BF16 rounding of the rest; rows
-// up to rows_pad zero.  For the K = 16 input layer (Ks = 16) the bias goes
-// into columns 14, 15 instead (bcol), replacing weights of unused features.
-__device__ __forceinline__ void stage_kmajor_bias(unsigned char *img, const bf16 *src,
-                                                  const float *b, int rows, int rows_pad, int Ks,
-                                                  int Ki, int bcol, float scale) {
-  // chunk d of the image (16 bytes) is row 8 g + rr, columns 8 q .. 8 q + 7,
-  // with d = (g * (Ki / 8) + q) * 8 + rr: consecutive threads write
-  // consecutive chunks, rows_pad * Ki / 8 chunks in all
-  const int per_group = Ki;  // chunks per 8-row group: (Ki / 8) * 8
-  for (int d = threadIdx.x; d < rows_pad * (Ki / 8); d += blockDim.x) {
-    const int g = d / per_group, rem = d - g * per_group;
-    const int q = rem >> 3, r = 8 * g + (rem & 7), k0 = 8 * q;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (r < rows) {
-      bf16 *e = reinterpret_cast<bf16 *>(&v);
-      if (k0 + 8 <= Ks && (bcol >= k0 + 8 || bcol + 1 < k0)) {
-        v = *reinterpret_cast<const uint4 *>(src + (long long)r * Ks + k0);
-        if (scale != 1.f) {
+// The weights' operand images for k_mlp_infer_tc, one thread per 16-byte chunk
+// (8 columns of a row); launched when the parameters change.
+__global__ void k_infer_image(const bf16 *__restrict__ Wg, const float *__restrict__ P,
+                              unsigned char *__restrict__ out) {
+  const uint32_t o = 16 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (o >= tc::kImage) return;
+  // image, its columns, the chunk's row and first column
+  const uint32_t start[9] = {tc::kW0, tc::kW1, tc::kW2, tc::kW3, tc::kB1, tc::kB2, tc::kB3, tc::kOne,
+                             tc::kImage};
+  int im = 0;
+  while (o >= start[im + 1]) ++im;
+  const int K = im >= 1 && im <= 3 ? 128 : 16, d = (int)(o - start[im]) / 16;
+  const int g = d / K, q = (d - g * K) >> 3, r = 8 * g + (d & 7), k0 = 8 * q;
+  const int woff[4] = {kOffW0, kOffW1, kOffW2, kOffW3}, boff[4] = {kOffB0, kOffB1, kOffB2, kOffB3};
+  auto bias = [&](int l, int part) {  // BF16 high part, and the rest
+    const float b = (l == 3 && r >= kMlpOut) ? 0.f : P[boff[l] + r] * (l == 3 ? 1.f : 0.5f);
+    const float hi = __bfloat162float(__float2bfloat16_rn(b));
+    return part == 0 ? hi : b - hi;
+  };
+  bf16 e[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) e[j] = __float2bfloat16_rn(__bfloat162float(e[j]) * scale);
-        }
-      } else {
-        const float bs = b[r] * scale;
-        const bf16 hi = __float2bfloat16_rn(bs);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int k = k0 + j;
-          float w = 0.f;
-          if (k == bcol)
-            w = __bfloat162float(hi);
-          else if (k == bcol + 1)
-            w = bs - __bfloat162float(hi);
-          else if (k < Ks)
-            w = __bfloat162float(src[(long long)r * Ks + k]) * scale;
-          e[j] = __float2bfloat16_rn(w);
-        }
-      }
-    }
-    *reinterpret_cast<uint4 *>(img + 16 * d) = v;
+  for (int j = 0; j < 8; ++j) {
+    const int k = k0 + j;
+    float v = 0.f;
+    if (im == 7)
+      v = k < 2 ? 1.f : 0.f;
+    else if (im >= 4)
+      v = k < 2 ? bias(im - 3, k) : 0.f;
+    else if (im == 0 && k >= kMlpIn - 2)
+      v = bias(0, k - (kMlpIn - 2));
+    else if (im < 3 || r < kMlpOut)
+      v = __bfloat162float(Wg[woff[im] + r * K + k]) * (im == 3 ? 1.f : 0.5f);
+    e[j] = __float2bfloat16_rn(v);
   }
+  *reinterpret_cast<uint4 *>(out + o) = *reinterpret_cast<const uint4 *>(e);
 }
 
-// SiLU of one 32-column accumulator chunk of this thread's lane into row r of
-// the activation image (columns c0 .. c0 + 31)
-__device__ __forceinline__ void tc_silu_chunk(uint32_t taddr, unsigned char *hs, int r, int c0) {
+// SiLU of 32 accumulator columns of this thread's lane into the row's
+// activation image (row address hs, columns c0 .. c0 + 31)
+__device__ __forceinline__ void tc_silu_chunk(uint32_t taddr, unsigned char *hs, int c0) {
   float v[32];
   tmem_ld32(taddr, v);
   uint32_t pk[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) pk[j] = silu_h_bf16x2(v[2 * j], v[2 * j + 1]);
-  unsigned char *dst = hs + (r / 8) * tc::kSBOH + (r % 8) * 16 + (c0 / 8) * 128;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    *reinterpret_cast<uint4 *>(dst + i * 128) =
+    *reinterpret_cast<uint4 *>(hs + (c0 / 8 + i) * 128) =
         make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
 }
 
-// issue one layer of a slot: D (+)= A B^T over K = 16 steps
-__device__ __forceinline__ void tc_issue_layer(int layer, uint32_t tmem_d, uint32_t sX,
-                                               uint32_t sH, uint32_t sW0, uint32_t sW1,
-                                               uint32_t sW2, uint32_t sW3) {
+// issue one layer of a slot: D = A W^T over K = 16 steps, then + ones x bias
+__device__ __forceinline__ void tc_issue_layer(int layer, uint32_t tmem_d, uint32_t sH, uint32_t sI) {
   constexpr uint32_t id128 = umma_idesc_bf16(128, 128), id16 = umma_idesc_bf16(128, 16);
   if (layer == 0) {  // the bias comes with the input's constant columns
-    umma_bf16(tmem_d, umma_sdesc(sX, 128, 256), umma_sdesc(sW0, 128, 256), id128, 0u);
+    umma_bf16(tmem_d, umma_sdesc(sH, 128, 256), umma_sdesc(sI + tc::kW0, 128, 256), id128, 0u);
     return;
   }
-  const uint32_t sW = layer == 1 ? sW1 : (layer == 2 ? sW2 : sW3);
+  const uint32_t sW = sI + (layer == 1 ? tc::kW1 : (layer == 2 ? tc::kW2 : tc::kW3));
+  const uint32_t sB = sI + (layer == 1 ? tc::kB1 : (layer == 2 ? tc::kB2 : tc::kB3));
   const uint32_t id = layer == 3 ? id16 : id128;
 #pragma unroll
-  for (int kk = 0; kk < tc::kKH / 16; ++kk)  // 8 steps of weights, 1 of bias columns
-    umma_bf16(tmem_d, umma_sdesc(sH + 256 * kk, 128, tc::kSBOH),
-              umma_sdesc(sW + 256 * kk, 128, tc::kSBOH), id, kk > 0 ? 1u : 0u);
+  for (int kk = 0; kk < 8; ++kk)
+    umma_bf16(tmem_d, umma_sdesc(sH + 256 * kk, 128, 2048), umma_sdesc(sW + 256 * kk, 128, 2048), id,
+              kk > 0 ? 1u : 0u);
+  umma_bf16(tmem_d, umma_sdesc(sI + tc::kOne, 128, 256), umma_sdesc(sB, 128, 256), id, 1u);
 }
 
-__global__ void __maxnreg__(128)
-    k_mlp_infer_tc(const bf16 *__restrict__ X, long long n, const bf16 *__restrict__ Wg,
-                   const float *__restrict__ P, float *__restrict__ Y, int *err) {
+// One contiguous global -> shared copy (16-byte multiples) counted on `bar`
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes,
+                                          uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          dst),
+      "l"(src), "r"(bytes), "r"(bar)
+      : "memory");
+}
+
+__global__ void __launch_bounds__(tc::kThreads, 1)
+    k_mlp_infer_tc(const bf16 *__restrict__ X, long long n, const unsigned char *__restrict__ image,
+                   float *__restrict__ Y, int *err) {
   extern __shared__ __align__(128) unsigned char tc_raw[];
   unsigned char *sm = tc_raw + ((128 - (smem_u32(tc_raw) & 127)) & 127);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const uint32_t full0 = smem_u32(sm + tc::kBar), done0 = full0 + 8 * tc::kSlots;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + tc::kBar + 64);
-  volatile int *abort = reinterpret_cast<volatile int *>(sm + tc::kBar + 68);
-
-  // weights with their biases, once per CTA (layers 0..2 times 1/2, see above)
-  stage_kmajor_bias(sm + tc::kW0, Wg + kOffW0, P + kOffB0, kMlpHid, kMlpHid, kMlpIn, kMlpIn,
-                    kMlpIn - 2, 0.5f);
-  stage_kmajor_bias(sm + tc::kW1, Wg + kOffW1, P + kOffB1, kMlpHid, kMlpHid, kMlpHid, tc::kKH,
-                    kMlpHid, 0.5f);
-  stage_kmajor_bias(sm + tc::kW2, Wg + kOffW2, P + kOffB2, kMlpHid, kMlpHid, kMlpHid, tc::kKH,
-                    kMlpHid, 0.5f);
-  stage_kmajor_bias(sm + tc::kW3, Wg + kOffW3, P + kOffB3, kMlpOut, 16, kMlpHid, tc::kKH,
-                    kMlpHid, 1.f);
-  // the constant columns of every slot's activation image: ones in columns
-  // 128, 129, zeros in 130..143 (the epilogues write columns 0..127 only)
-  for (int d = t; d < tc::kSlots * 128; d += blockDim.x) {
-    const int sl = d / 128, r = d - sl * 128;
-    unsigned char *row = sm + tc::kHs + sl * 128 * tc::kKH * 2 + (r / 8) * tc::kSBOH + (r % 8) * 16;
-    *reinterpret_cast<uint4 *>(row + 16 * 128) = make_uint4(0x3F803F80u, 0u, 0u, 0u);
-    *reinterpret_cast<uint4 *>(row + 17 * 128) = make_uint4(0u, 0u, 0u, 0u);
-  }
+  const uint32_t wbar = done0 + 8 * tc::kSlots;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + tc::kBar + 72);
+  volatile int *abort = reinterpret_cast<volatile int *>(sm + tc::kBar + 76);
   if (t == 0) {
     for (int sl = 0; sl < tc::kSlots; ++sl) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" ::"r"(full0 + 8 * sl) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(full0 + 8 * sl) : "memory");
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(done0 + 8 * sl) : "memory");
     }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbar) : "memory");
     *abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(wbar), "r"(tc::kImage)
+                 : "memory");
+    bulk_load(smem_u32(sm), image, tc::kImage, wbar);
   }
   if (warp == 0) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
                  "r"(tc::kTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  fence_proxy_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = *tmem_slot;
-  const uint32_t sW0 = smem_u32(sm + tc::kW0), sW1 = smem_u32(sm + tc::kW1);
-  const uint32_t sW2 = smem_u32(sm + tc::kW2), sW3 = smem_u32(sm + tc::kW3);
+  // tile b + grid (s + 4 j), j = 0, 1, ..: an SM's share differs by one tile at most
   const long long tiles = (n + 127) / 128, stride = (long long)tc::kSlots * gridDim.x;
-
-  if (warp < tc::kMmaWarp) {
-    // ---- epilogue of slot s: tiles first, first + stride, ...
-    const int s = warp >> 2, q = warp & 3, r = 32 * q + lane;
-    const uint32_t tl = tbase + ((uint32_t)(32 * q) << 16) + 128u * s;
-    const uint32_t full = full0 + 8 * s, done = done0 + 8 * s;
-    unsigned char *xs = sm + tc::kXs + 4096 * s, *hs = sm + tc::kHs + 128 * tc::kKH * 2 * s;
-    const long long first = (long long)tc::kSlots * blockIdx.x + s;
-    uint32_t j = 0;  // steps (layers) completed: the parity of the next wait
-    uint4 xa = make_uint4(0u, 0u, 0u, 0u), xb = xa;
-    if (first < tiles && first * 128 + r < n) {
-      const uint4 *src = reinterpret_cast<const uint4 *>(X + (first * 128 + r) * kMlpIn);
-      xa = src[0];
-      xb = src[1];
-    }
-    bool ok = true;
-    for (long long tile = first; tile < tiles && ok; tile += stride) {
-      const long long row = tile * 128 + r;
-      // layer 0 operand: the input row with ones in the bias columns 14, 15
-      unsigned char *xd = xs + (r / 8) * 256 + (r % 8) * 16;
-      *reinterpret_cast<uint4 *>(xd) = xa;
-      *reinterpret_cast<uint4 *>(xd + 128) = make_uint4(xb.x, xb.y, xb.z, 0x3F803F80u);
-      {  // the next tile's rows, loaded while this one runs
-        const long long nrow = (tile + stride) * 128 + r;
-        xa = make_uint4(0u, 0u, 0u, 0u);
-        xb = xa;
-        if (tile + stride < tiles && nrow < n) {
-          const uint4 *src = reinterpret_cast<const uint4 *>(X + nrow * kMlpIn);
-          xa = src[0];
-          xb = src[1];
-        }
-      }
-      fence_proxy_async_smem();
-      tc_fence_before();
-      mbar_arrive(full);
-      for (int l = 0; l < 4; ++l) {
-        ok = mbar_wait(done, j & 1u, abort);
-        ++j;
+  const int s = warp >> 2, q = warp & 3, r = 32 * q + lane;
+  const uint32_t td = tbase + 128u * s, tl = td + ((uint32_t)(32 * q) << 16);
+  const uint32_t full = full0 + 8 * s, done = done0 + 8 * s;
+  unsigned char *hs = sm + tc::kHs + 128 * 128 * 2 * s;
+  unsigned char *xrow = hs + (r / 8) * 256 + (r % 8) * 16, *hrow = hs + (r / 8) * 2048 + (r % 8) * 16;
+  const bool issuer = q == 0 && lane == 0;
+  const long long first = blockIdx.x + (long long)s * gridDim.x;
+  uint32_t j = 0;  // layers completed: the parity of the slot's barriers
+  uint4 xa = make_uint4(0u, 0u, 0u, 0u), xb = xa;
+  if (first < tiles && first * 128 + r < n) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(X + (first * 128 + r) * kMlpIn);
+    xa = src[0];
+    xb = src[1];
+  }
+  bool ok = mbar_wait(wbar, 0u, abort);  // the weights (every thread: nobody leaves before)
+  ok = __all_sync(0xffffffffu, ok);
+  // publish the slot's operand, issue the layer, wait for its accumulator
+  auto layer = [&](int l) {
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(full);  // (one arrival per warp)
+    bool got = true;
+    if (issuer) {
+      got = mbar_wait(full, j & 1u, abort);
+      if (got) {
         tc_fence_after();
-        ok = __all_sync(0xffffffffu, ok);  // warp-uniform before the .sync.aligned TMEM ops
-        if (!ok) break;
-        if (l < 3) {
+        tc_issue_layer(l, td, smem_u32(hs), smem_u32(sm));
+        umma_commit(done);
+      }
+    }
+    __syncwarp();
+    if (got) got = mbar_wait(done, j & 1u, abort);
+    ++j;
+    tc_fence_after();
+    return (bool)__all_sync(0xffffffffu, got);  // warp-uniform before the .sync.aligned TMEM ops
+  };
+  for (long long tile = first; tile < tiles && ok; tile += stride) {
+    const long long row = tile * 128 + r;
+    // layer 0 operand: the input row with ones in the bias columns 14, 15
+    *reinterpret_cast<uint4 *>(xrow) = xa;
+    *reinterpret_cast<uint4 *>(xrow + 128) = make_uint4(xb.x, xb.y, xb.z, 0x3F803F80u);
+    {  // the next tile's rows, loaded while this one runs
+      const long long nrow = (tile + stride) * 128 + r;
+      xa = make_uint4(0u, 0u, 0u, 0u);
+      xb = xa;
+      if (tile + stride < tiles && nrow < n) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(X + nrow * kMlpIn);
+        xa = src[0];
+        xb = src[1];
+      }
+    }
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) tc_silu_chunk(tl + 32 * c, hs, r, 32 * c);
-          fence_proxy_async_smem();
-          tc_fence_before();
-          mbar_arrive(full);
-        } else {
-          float o[16];
-          tmem_ld16(tl, o);
-          if (row < n) {
-            float4 *yd = reinterpret_cast<float4 *>(Y + row * kMlpOut);
-            yd[0] = make_float4(o[0], o[1], o[2], o[3]);
-            yd[1] = make_float4(o[4], o[5], o[6], o[7]);
-          }
-        }
+    for (int l = 0; l < 3 && ok; ++l) {
+      ok = layer(l);
+      if (!ok) break;
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) tc_silu_chunk(tl + 32 * c, hrow, 32 * c);
+    }
+    if (ok) ok = layer(3);
+    if (!ok) break;
+    float o[16];
+    tmem_ld16(tl, o);
+    if (row < n) {
+      float4 *yd = reinterpret_cast<float4 *>(Y + row * kMlpOut);
+      yd[0] = make_float4(o[0], o[1], o[2], o[3]);
+      yd[1] = make_float4(o[4], o[5], o[6], o[7]);
+    }
+  }
+  if (!ok) {
+    if (lane == 0) atomicOr(err, kErrWait);
+    // the MMAs already issued and the weights' copy (bounded waits of their own)
+    if (issuer)
+      for (int w = 0; w < tc::kWaitLimit; ++w) {
+        uint32_t a, b;
+        asm volatile(
+            "{\n\t.reg .pred p, r;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%2], %4;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 r, [%3], %5;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\tselp.u32 %1, 1, 0, r;\n\t}\n"
+            : "=r"(a), "=r"(b)
+            : "r"(done), "r"(wbar), "r"((j - 1) & 1u), "r"(0u)
+            : "memory");
+        if (a && b) break;
       }
-    }
-    if (!ok && lane == 0) atomicOr(err, kErrWait);
-  } else if (lane == 0) {
-    // ---- the MMA issuer: slots round-robin, one layer per visit
-    long long nt[tc::kSlots];
-    uint32_t js[tc::kSlots];
-    for (int sl = 0; sl < tc::kSlots; ++sl) {
-      const long long f = (long long)tc::kSlots * blockIdx.x + sl;
-      nt[sl] = f < tiles ? (tiles - 1 - f) / stride + 1 : 0;
-      js[sl] = 0;
-    }
-    bool ok = true, any = true;
-    while (ok && any) {
-      any = false;
-      for (int sl = 0; sl < tc::kSlots && ok; ++sl) {
-        if ((long long)js[sl] >= 4 * nt[sl]) continue;
-        any = true;
-        ok = mbar_wait(full0 + 8 * sl, js[sl] & 1u, abort);
-        if (!ok) break;
-        tc_fence_after();
-        tc_issue_layer((int)(js[sl] & 3u), tbase + 128u * sl,
-                       smem_u32(sm + tc::kXs + 4096 * sl),
-                       smem_u32(sm + tc::kHs + 128 * tc::kKH * 2 * sl),
-                       sW0, sW1, sW2, sW3);
-        umma_commit(done0 + 8 * sl);
-        ++js[sl];
-      }
-    }
-    if (!ok) {
-      atomicOr(err, kErrWait);
-      // the MMAs already issued (bounded): the last commit of every slot
-      for (int sl = 0; sl < tc::kSlots; ++sl)
-        if (js[sl] > 0) mbar_wait(done0 + 8 * sl, (js[sl] - 1) & 1u, abort);
-    }
   }
   // every MMA has completed (or a wait gave up): free TMEM
   tc_fence_before();
@@ -821,6 +807,7 @@ struct ftgpu_surrogate {
   bf16 *H1 = nullptr, *H2 = nullptr, *H3 = nullptr, *dY = nullptr, *dZ1 = nullptr, *dZ2 = nullptr,
        *dZ3 = nullptr;
   long long adam_t = 0;
+  unsigned char *image = nullptr;  // operand images of the current parameters (k_infer_image)
   int *derr = nullptr;  // device error word of standalone inference calls
   // tcgen05 path: transposed operand images per 128-row tile, weight-gradient slices
   unsigned char *tiles = nullptr;
@@ -832,7 +819,7 @@ struct ftgpu_surrogate {
     for (void *p : {(void *)P, (void *)G, (void *)Mo, (void *)V, (void *)Wb, (void *)X, (void *)T,
                     (void *)Z1, (void *)Z2, (void *)Z3, (void *)Y, (void *)rowloss, (void *)loss,
                     (void *)H1, (void *)H2, (void *)H3, (void *)dY, (void *)dZ1, (void *)dZ2,
-                    (void *)dZ3, (void *)derr, (void *)tiles, (void *)part})
+                    (void *)dZ3, (void *)image, (void *)derr, (void *)tiles, (void *)part})
       if (p) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -990,6 +977,12 @@ int train_attrs(const ftgpu_surrogate *s) {
   return 0;
 }
 
+// The inference kernel's operand images, after the parameters changed (queued
+// on the surrogate's stream; every caller waits for it before it returns)
+void refresh_image(ftgpu_surrogate *s) {
+  k_infer_image<<<(tc::kImage / 16 + 255) / 256, 256, 0, s->stream>>>(s->Wb, s->P, s->image);
+}
+
 // Y of B rows of X
 int forward(ftgpu_surrogate *s, const bf16 *X, long long B) {
   if (!s->tensor_cores) return forward_mma(s, X, B);
@@ -1046,10 +1039,9 @@ int surrogate_infer(ftgpu_surrogate *s, const uint16_t *X, long long n, float *Y
   }
   const int sms = sm_count(s->device);
   const long long tiles = (n + 127) / 128;
-  const long long grid =
-      std::max<long long>(1, std::min<long long>((long long)sms, (tiles + tc::kSlots - 1) / tc::kSlots));
+  const long long grid = std::min<long long>(sms, tiles);
   k_mlp_infer_tc<<<(unsigned)grid, tc::kThreads, tc::kSmem, st>>>(reinterpret_cast<const bf16 *>(X), n,
-                                                          s->Wb, s->P, Y, err);
+                                                                  s->image, Y, err);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return record_error(FTGPU_ERR_CUDA, (std::string("tensor-core inference launch: ") +
@@ -1109,7 +1101,8 @@ int ftgpu_surrogate_create(ftgpu_surrogate **out, int device, const double *prop
   s->law.out_scale = 1.0;
   s->law.trust_e2 = 0.04;
   int r = dalloc(&s->P, kMlpParams) | dalloc(&s->G, kMlpParams) | dalloc(&s->Mo, kMlpParams) |
-          dalloc(&s->V, kMlpParams) | dalloc(&s->Wb, kMlpParams) | dalloc(&s->derr, 1);
+          dalloc(&s->V, kMlpParams) | dalloc(&s->Wb, kMlpParams) | dalloc(&s->derr, 1) |
+          dalloc(&s->image, tc::kImage);
   if (r) return FTGPU_ERR_ALLOC;
   // Kaiming-uniform-style init (fan-in scaled), seeded, on the host
   std::vector<float> p(kMlpParams, 0.f);
@@ -1132,6 +1125,8 @@ int ftgpu_surrogate_create(ftgpu_surrogate **out, int device, const double *prop
   SCK(cudaMemset(s->Mo, 0, kMlpParams * 4));
   SCK(cudaMemset(s->V, 0, kMlpParams * 4));
   k_to_bf16<<<(kMlpParams + 255) / 256, 256, 0, s->stream>>>(s->P, kMlpParams, s->Wb);
+  refresh_image(s.get());
+  SCK(cudaGetLastError());
   SCK(cudaStreamSynchronize(s->stream));
   *out = s.release();
   return FTGPU_OK;
@@ -1201,7 +1196,10 @@ int ftgpu_surrogate_train(ftgpu_surrogate *s, int epochs, int batch, double lr,
       const float b1 = 0.9f, b2 = 0.999f;
       const float c1 = 1.f - powf(b1, (float)at), c2 = 1.f - powf(b2, (float)at);
       r = train_batch(s, X, T, batch, AdamArgs{1, lr_t, b1, b2, 1e-8f, c1, c2});
-      if (r) return r;
+      if (r) {
+        refresh_image(s);
+        return r;
+      }
       s->adam_t = at;
       if (b == nb - 1) {
         float hl = 0.f;
@@ -1212,6 +1210,8 @@ int ftgpu_surrogate_train(ftgpu_surrogate *s, int epochs, int batch, double lr,
     }
     last = acc;
   }
+  refresh_image(s);
+  SCK(cudaGetLastError());
   SCK(cudaStreamSynchronize(s->stream));
   int e = 0;
   SCK(cudaMemcpy(&e, s->derr, sizeof(int), cudaMemcpyDeviceToHost));
@@ -1319,6 +1319,8 @@ int ftgpu_surrogate_params(ftgpu_surrogate *s, float *get, const float *set) {
   if (set) {
     SCK(cudaMemcpy(s->P, set, kMlpParams * 4, cudaMemcpyHostToDevice));
     k_to_bf16<<<(kMlpParams + 255) / 256, 256, 0, s->stream>>>(s->P, kMlpParams, s->Wb);
+    refresh_image(s);
+    SCK(cudaGetLastError());
     SCK(cudaStreamSynchronize(s->stream));
   }
   if (get) SCK(cudaMemcpy(get, s->P, kMlpParams * 4, cudaMemcpyDeviceToHost));

@@ -313,16 +313,6 @@ __global__ void __launch_bounds__(trn::kThreads, 1)
                  : "memory");
 }
 
-// One contiguous global -> shared copy (16-byte multiples) counted on `bar`
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes,
-                                          uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          dst),
-      "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
-
 // dW_l of one batch slice: dW = dZ^T H, both operands transposed images as
 // k_train_rows left them, so a tile is two bulk copies and eight MMAs.
 // blockIdx.y: layer 0..3 (operand rows dZ1, dZ2, dZ3, dY; columns X, H1, H2,
