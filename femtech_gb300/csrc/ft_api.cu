@@ -1176,7 +1176,7 @@ int setup_t(ftgpu_model *m) {
     }
     CKI(m->fib.upload(fb.data(), fb.size()));
   }
-  // viscoelastic history per group: [ncomp][NGP][nelem], zero
+  // viscoelastic history per group in whole blocks of 32, zero
   m->hist.clear();
   for (auto &g : ps.groups) {
     int nc = g.mat == 5 ? 18 : (g.mat == 7 ? 12 : 0);
@@ -1184,7 +1184,9 @@ int setup_t(ftgpu_model *m) {
       m->hist.emplace_back(nullptr);
       continue;
     }
-    const size_t n = (size_t)nc * (g.etype == 0 ? 8 : 1) * g.nelem;
+    const int ngp = g.etype == 0 ? 8 : 1;
+    const size_t n = (size_t)nc * kLaneBlk *
+                     (m->hexgp && g.etype == 0 ? blk_up(8ll * g.nelem) : ngp * blk_up(g.nelem));
     auto b = std::make_unique<DBuf>();
     CKI(b->alloc(n * sizeof(R)));
     CK(cudaMemset(b->p, 0, n * sizeof(R)));
@@ -1239,7 +1241,8 @@ int setup_t(ftgpu_model *m) {
       continue;
     }
     auto b = std::make_unique<DBuf>();
-    CKI(b->alloc((size_t)80 * g.nelem * sizeof(R)));
+    // (whole blocks of 32 elements, or of 32 of their points)
+    CKI(b->alloc((m->hexgp ? 10 * blk_up(8ll * g.nelem) : 80 * blk_up(g.nelem)) * kLaneBlk * sizeof(R)));
     m->geo.push_back(std::move(b));
     const ElemArgs<R> A = elem_args<R>(m, g, (int)gi);
     if (m->hexgp)

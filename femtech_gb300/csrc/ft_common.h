@@ -13,6 +13,18 @@ constexpr int kMaxPatchElems = 256;   // elements per patch (thread block) upper
 constexpr int kMaxLocalNodes = 320;   // local nodes per patch (shared memory bound)
 constexpr int kElemThreads = 256;     // upper bound of threads per element block
 
+// Per-element (and per-Gauss-point) arrays of one group that a thread walks
+// component by component are kept in blocks of 32 elements, [element / 32]
+// [component][32]: a warp's access stays one line, and a component's address
+// is a constant offset from the first one's (as [component][element] each took
+// two integer operations: 48 of a tetrahedron's 1,285 instructions).
+constexpr int kLaneBlk = 32;
+__host__ __device__ constexpr long long blk_up(long long n) { return (n + kLaneBlk - 1) / kLaneBlk; }
+// first component of item i of `comps` (stride kLaneBlk)
+__host__ __device__ constexpr long long blk_at(long long i, int comps) {
+  return (i >> 5) * (comps * kLaneBlk) + (i & (kLaneBlk - 1));
+}
+
 // Shared memory of an element block's staged local CSR (the in-block
 // assembly's offsets and corner entries, 16-bit): kMaxLocalNodes + 1 offsets
 // padded to 8, then NC entries per element.
@@ -99,11 +111,13 @@ struct ElemArgs {
   const Real *sU;             // [S] Slot4: displacement replicas
   Real *sF;                   // [S] Slot4: patch-partial internal forces
   // material state
-  Real *hist;                 // [ncomp][NGP][nelem] of this group
-  // FP32 C3D8 groups: the reference geometry, written once at set-up -- per
-  // element 80 values (Gauss point g: A^{-1} row major, then det A, at
-  // 10 g .. 10 g + 9) in 20 rows of 4, value v at [4 (v/4 * nelem + e) + v%4]
-  // (null for C3D4 groups and in FP64 mode)
+  // history of this group: [nelem/32][NGP][ncomp][32]; on the eight-lane pass
+  // [8 nelem/32][ncomp][32] of points 8 element + lane
+  Real *hist;
+  // C3D8 groups: the reference geometry, written once at set-up -- per element
+  // 80 values (Gauss point g: A^{-1} row major, then det A, at 10 g ..
+  // 10 g + 9) as 20 rows of 4, [nelem/32][20][32][4]; on the eight-lane pass ten
+  // values per point, [8 nelem/32][10][32] (null for C3D4 groups)
   const Real *geo;
   const MatP<Real> *mats;
   // clock

@@ -105,7 +105,7 @@ __device__ __forceinline__ void adj3(const R (&A)[3][3], R (&J)[3][3], R &det) {
 }
 
 // Per-Gauss-point material update on the displacement gradient D = F - I.
-// hist points at this element's first history component (stride hs per
+// hist points at this Gauss point's first history component (stride kLaneBlk per
 // component, gstride per Gauss point).
 // Green strain (Voigt, tensor shear) from D
 template <class R>
@@ -173,8 +173,7 @@ __device__ __forceinline__ void goh_parts_surrogate(const MatP<R> &mp, const R (
 template <class R>
 struct HistGlobal {
   const R *p;
-  long long stride;
-  __device__ __forceinline__ R operator()(int k) const { return p[k * stride]; }
+  __device__ __forceinline__ R operator()(int k) const { return p[k * kLaneBlk]; }
 };
 template <class R>
 struct HistShared {
@@ -189,7 +188,7 @@ __host__ __device__ constexpr int hist_comps(int mat) { return mat == 5 ? 18 : (
 // FFORM: the HGO family through F (FP32 tetrahedra, see mat_hgo_parts_f)
 template <class R, int MAT, bool FFORM = false, class HIN, class PART>
 __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][3], R Jm1,
-                                             const R (&a0)[3], R *hist, long long hs,
+                                             const R (&a0)[3], R *hist,
                                              const R (&pc)[4], const float *sy,
                                              const SurrogateLaw &law, const HIN &hin,
                                              const PART &part) {
@@ -234,14 +233,14 @@ __device__ __forceinline__ Sym6<R> stress_at(const MatP<R> &mp, const R (&D)[3][
     for (int c = 0; c < 6; ++c) {
       const R dS = sd[c] - h[NT * 6 + c];
       const R h1 = pc[0] * h[c] + pc[1] * dS;
-      hist[c * hs] = h1;
+      hist[c * kLaneBlk] = h1;
       R acc = sd[c] + sv[c] + h1;
       if (NT == 2) {
         const R h2 = pc[2] * h[6 + c] + pc[3] * dS;
-        hist[(6 + c) * hs] = h2;
+        hist[(6 + c) * kLaneBlk] = h2;
         acc += h2;
       }
-      hist[(NT * 6 + c) * hs] = sd[c];
+      hist[(NT * 6 + c) * kLaneBlk] = sd[c];
       out[c] = acc;
     }
     S = Sym6<R>{out[0], out[1], out[2], out[3], out[4], out[5]};
@@ -412,24 +411,28 @@ __device__ __forceinline__ float face_pair_area_max(const float (&h)[7][3], int 
 // history one point ahead (two buffers), so that no point waits for memory and
 // four blocks still fit an SM (238k elements of material 5: step 156 us with
 // the history loaded at each point's start, 114 us streamed).
+// Rows are stored side by side, [row][elements][4], as the copies deliver them
+// (a thread's 80 values contiguous, with constant offsets and no more bank
+// conflicts, took 921 instead of 794 us: a copied line then falls apart into
+// eight places).
 struct HexStream {
-  float *geo;        // shared: [pairs held][5 rows][elements] x 4, this thread's first value
+  float *geo;        // shared: [pairs held][5 rows][elements][4], this thread's first value
   float *hist;       // shared: [2][components][elements], this thread's value
   const float *src;  // global: this element's value 0 of row 0
-  long long nelem;
-  int rs;            // 4 x elements per patch: row stride in shared memory
-  int mask;          // pairs held - 1 (3: all four, 1: two)
+  int pe;            // elements per patch
+  // pair q of Gauss points: rows 5 q .. 5 q + 4; held: pairs kept (2 or 4)
+  template <int HELD>
   __device__ __forceinline__ void geo_pair(int q) const {
-    const float *s = src + 20ll * q * nelem;
-    float *d = geo + (q & mask) * 5 * rs;
+    const float *s = src + 5 * q * 4 * kLaneBlk;
+    float *d = geo + (q % HELD) * 20 * pe;
 #pragma unroll
-    for (int r = 0; r < 5; ++r) cp_async16(d + r * rs, s + 4ll * r * nelem);
+    for (int r = 0; r < 5; ++r) cp_async16(d + 4 * r * pe, s + r * 4 * kLaneBlk);
   }
   template <int NH>
-  __device__ __forceinline__ void hist_point(int g, const float *h, long long hs) const {
-    float *d = hist + (g & 1) * NH * (rs / 4);
+  __device__ __forceinline__ void hist_point(int g, const float *h) const {
+    float *d = hist + (g & 1) * NH * pe;
 #pragma unroll
-    for (int k = 0; k < NH; ++k) cp_async_small<4>(d + k * (rs / 4), h + k * hs);
+    for (int k = 0; k < NH; ++k) cp_async_small<4>(d + k * pe, h + k * kLaneBlk);
   }
 };
 
@@ -437,13 +440,13 @@ template <int MAT, bool GP>
 __device__ __forceinline__ void hex_gauss_loop_x2(const float2 (&hp)[7], const float (&hz)[7],
                                                   const MatP<float> &mp,
                                                   const float (&pc)[4], const float (&a0)[3],
-                                                  float *hist, long long hs, long long gs,
-                                                  int pass, float &vol, float2 (&mc)[7],
+                                                  float *hist, int pass, float &vol, float2 (&mc)[7],
                                                   float (&mz)[7], int &bad,
                                                   const ElemArgs<float> &A, long long gpo,
                                                   const HexStream &st) {
   const bool dt_only = pass == kPassDt;
-  const int rs = st.rs;
+  constexpr int NH = hist_comps(MAT);
+  const int rs = 4 * st.pe;  // row stride
   const float *gn = st.geo;  // the next point's values (all rows staged)
 #pragma unroll
   for (int k = 0; k < 7; ++k) {
@@ -455,23 +458,21 @@ __device__ __forceinline__ void hex_gauss_loop_x2(const float2 (&hp)[7], const f
     float xi, et, ze;
     hex_gauss_point(g, xi, et, ze);
     const float ez = et * ze, xz = xi * ze, xe = xi * et;
-    if (hist_comps(MAT) > 0) {
+    if (NH > 0) {
       if (g > 0) cp_async_wait_all();  // this point's inputs, on their way since the last one
-      if (!(g & 1) && g < 6) st.geo_pair(g / 2 + 1);
+      if (!(g & 1) && g < 6) st.template geo_pair<2>(g / 2 + 1);
       if (g < 7 && pass == kPassForce)
-        st.template hist_point<hist_comps(MAT)>(g + 1, hist + (g + 1) * gs, hs);
+        st.template hist_point<NH>(g + 1, hist + (g + 1) * (NH * kLaneBlk));
     }
     // A^{-1} (Q) and det A: values 10g .. 10g+9 as five pairs
-    const float *gb = hist_comps(MAT) > 0
-                          ? st.geo + ((g >> 1) & 1) * 5 * rs + ((g & 1) ? 2 * rs + 2 : 0)
-                          : gn;
+    const float *gb = NH > 0 ? st.geo + ((g >> 1) & 1) * 5 * rs + ((g & 1) ? 2 * rs + 2 : 0) : gn;
     const int o1 = (g & 1) ? rs - 2 : 2;
     const float2 q0 = *reinterpret_cast<const float2 *>(gb),
                  q1 = *reinterpret_cast<const float2 *>(gb + o1),
                  q2 = *reinterpret_cast<const float2 *>(gb + rs),
                  q3 = *reinterpret_cast<const float2 *>(gb + rs + o1),
                  q4 = *reinterpret_cast<const float2 *>(gb + 2 * rs);
-    if (hist_comps(MAT) == 0) gn += (g & 1) ? 3 * rs - 2 : 2 * rs + 2;
+    if (NH == 0) gn += (g & 1) ? 3 * rs - 2 : 2 * rs + 2;
     const float Q[3][3] = {{q0.x, q0.y, q1.x}, {q1.y, q2.x, q2.y}, {q3.x, q3.y, q4.x}};
     const float detA = q4.y;
     // H[d][i] = du_d / dxi_i: column i, rows 0-1 paired, row 2 scalar
@@ -502,8 +503,8 @@ __device__ __forceinline__ void hex_gauss_loop_x2(const float2 (&hp)[7], const f
     }
     const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
     const Sym6<float> S = stress_at<float, MAT>(
-        mp, D, Jm1, a0, hist + g * gs, hs, pc, sy, A.law,
-        HistShared<float>{st.hist + (g & 1) * hist_comps(MAT) * (rs / 4), rs / 4},
+        mp, D, Jm1, a0, hist + g * (NH * kLaneBlk), pc, sy, A.law,
+        HistShared<float>{st.hist + (g & 1) * NH * st.pe, st.pe},
         PartOfThread<float>{A.mats, A.epid, A.patch_elem_off, A.patch_begin});
     if (GP) {
       const long long q = gpo + g;
@@ -596,9 +597,8 @@ __device__ __forceinline__ void hex_inverse_transform(const T (&m)[7], T (&f)[8]
 template <int MAT, bool GP>
 __device__ __forceinline__ void hex_element_f32(const float (&x)[8][3], const float (&u)[8][3],
                                                 const MatP<float> &mp, const float (&pc)[4],
-                                                const float (&a0)[3], float *hist, long long hs,
-                                                long long gs, int pass, float (&f)[8][3],
-                                                float &le, int &bad, const ElemArgs<float> &A,
+                                                const float (&a0)[3], float *hist, int pass,
+                                                float (&f)[8][3], float &le, int &bad, const ElemArgs<float> &A,
                                                 long long gpo, const HexStream &st) {
   float vol = 0;
   // FP32: corners as (x, y) pairs + z; the current geometry's Hadamard
@@ -637,7 +637,7 @@ __device__ __forceinline__ void hex_element_f32(const float (&x)[8][3], const fl
     mc[k] = make_float2(0.f, 0.f);
     mz[k] = 0.f;
   }
-  hex_gauss_loop_x2<MAT, GP>(hp, hz, mp, pc, a0, hist, hs, gs, pass, vol, mc, mz, bad, A, gpo,
+  hex_gauss_loop_x2<MAT, GP>(hp, hz, mp, pc, a0, hist, pass, vol, mc, mz, bad, A, gpo,
                              st);
   le = vol / amax;
   if (pass == kPassForce) {
@@ -659,9 +659,8 @@ __device__ __forceinline__ void hex_element_f32(const float (&x)[8][3], const fl
 template <class R, int MAT, bool GP>
 __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][3],
                                             const MatP<R> &mp, const R (&pc)[4],
-                                            const R (&a0)[3], R *hist, long long hs,
-                                            long long gs, int pass, R (&f)[8][3], R &le,
-                                            int &bad, const ElemArgs<R> &A, long long gpo) {
+                                            const R (&a0)[3], R *hist, int pass, R (&f)[8][3],
+                                            R &le, int &bad, const ElemArgs<R> &A, long long gpo) {
   const bool dt_only = pass == kPassDt;
   R vol = 0;
   R m[7][3];
@@ -731,8 +730,8 @@ __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][
       continue;
     }
     const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
-    Sym6<R> S = stress_at<R, MAT>(mp, D, Jm1, a0, hist + g * gs, hs, pc, sy, A.law,
-                                  HistGlobal<R>{hist + g * gs, hs}, PartAt<R>{&mp});
+    Sym6<R> S = stress_at<R, MAT>(mp, D, Jm1, a0, hist, pc, sy, A.law, HistGlobal<R>{hist},
+                                  PartAt<R>{&mp});
     if (GP) {
       long long q = gpo + g;
 #pragma unroll
@@ -799,8 +798,7 @@ __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][
 template <class R, int MAT, bool GP>
 __device__ __forceinline__ void tet_element(const R (&x)[4][3], const R (&u)[4][3],
                                             const MatP<R> &mp, const R (&pc)[4],
-                                            const R (&a0)[3], R *hist, long long hs,
-                                            int pass, R (&f)[4][3], R &le, int &bad,
+                                            const R (&a0)[3], R *hist, int pass, R (&f)[4][3], R &le, int &bad,
                                             const ElemArgs<R> &A, long long gpo,
                                             const HistShared<R> &hin) {
   const bool dt_only = pass != kPassForce;
@@ -850,7 +848,7 @@ __device__ __forceinline__ void tet_element(const R (&x)[4][3], const R (&u)[4][
   if (!dt_only) {
     const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
     Sym6<R> S =
-        stress_at<R, MAT, sizeof(R) == 4>(mp, D, Jm1, a0, hist, hs, pc, sy, A.law, hin,
+        stress_at<R, MAT, sizeof(R) == 4>(mp, D, Jm1, a0, hist, pc, sy, A.law, hin,
                                           PartOfThread<R>{A.mats, A.epid, A.patch_elem_off, A.patch_begin});
     if (GP) {
 #pragma unroll
@@ -1038,7 +1036,8 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
   // last read from the first corner-force write)
   R *shF = PACK ? reinterpret_cast<R *>(shU + kMaxLocalNodes) : shUs + 3 * kMaxLocalNodes;
   constexpr bool GEO = ET == 0;  // (FP32: FP64 C3D8 elements run on k_hexgp)
-  constexpr int kStream = hist_comps(MAT) > 0 ? 40 + 2 * hist_comps(MAT) : 80;  // per element
+  constexpr bool kHist = hist_comps(MAT) > 0;
+  constexpr int kStream = kHist ? 40 + 2 * hist_comps(MAT) : 80;  // per element
   const int PE = blockDim.x;
   // the local CSR of the in-block assembly: offsets, then entries
   uint16_t *shLp = reinterpret_cast<uint16_t *>(shF + (GEO ? kStream : NC * 3) * PE);
@@ -1053,18 +1052,18 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
   const bool act = t < ne;
   const int e = e0 + (act ? t : 0);
   const long long el = e - A.elem_begin;
-  const long long gs = A.nelem, hs = (long long)NGP * A.nelem;
+  // this element's first history component (Gauss point g: NH * kLaneBlk on)
+  R *const hist = hist_comps(MAT) > 0 && A.hist ? A.hist + blk_at(el, NGP * hist_comps(MAT)) : nullptr;
   // the first Gauss points' geometry (and the first one's history), landing
   // while the per-element loads and the slot staging below are in flight
   HexStream stream;
   if constexpr (GEO) {
-    constexpr bool kHist = hist_comps(MAT) > 0;
-    stream = HexStream{shF + 4 * t, shF + 40 * PE + t, A.geo + 4 * el, gs, 4 * PE, kHist ? 1 : 3};
+    stream = HexStream{shF + 4 * t, shF + 40 * PE + t,
+                       A.geo + (el >> 5) * (80 * kLaneBlk) + (el & (kLaneBlk - 1)) * 4, PE};
     if (act) {
 #pragma unroll
-      for (int q = 0; q < (kHist ? 1 : 4); ++q) stream.geo_pair(q);
-      if (kHist && pass == kPassForce)
-        stream.template hist_point<hist_comps(MAT)>(0, A.hist + el, hs);
+      for (int q = 0; q < (kHist ? 1 : 4); ++q) stream.template geo_pair<kHist ? 2 : 4>(q);
+      if (kHist && pass == kPassForce) stream.template hist_point<hist_comps(MAT)>(0, hist);
     }
   }
   uint4 cv = make_uint4(0u, 0u, 0u, 0u);
@@ -1090,7 +1089,7 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
     }
     if (NH > 1 && pass == kPassForce) {
 #pragma unroll
-      for (int k = 0; k < NH; ++k) hin[k] = A.hist[el + k * hs];
+      for (int k = 0; k < NH; ++k) hin[k] = hist[k * kLaneBlk];
     }
   }
   const Clock *ck = A.clock + A.parity * A.ninst + inst;
@@ -1171,13 +1170,12 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
     const MatP<R> mp = A.mats[pw & 0x7fffffff];
     R pc[4];
     prony_consts<R, MAT>(mp, dt, pc);
-    R *hist = A.hist ? A.hist + el : nullptr;
     R le;
     const long long gpo = A.gpbase + el * NGP;
     if constexpr (ET == 0)
-      hex_element_f32<MAT, GP>(x, u, mp, pc, a0, hist, hs, gs, pass, f, le, bad, A, gpo, stream);
+      hex_element_f32<MAT, GP>(x, u, mp, pc, a0, hist, pass, f, le, bad, A, gpo, stream);
     else
-      tet_element<R, MAT, GP>(x, u, mp, pc, a0, hist, hs, pass, f, le, bad, A, gpo,
+      tet_element<R, MAT, GP>(x, u, mp, pc, a0, hist, pass, f, le, bad, A, gpo,
                               HistShared<R>{hin, 1});
     if (!GEO && pass == kPassForce) {
 #pragma unroll
@@ -1242,7 +1240,7 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
 // evaluated once as in ShapeFunctions.cpp:197-215), computed in FP64 from the
 // slot coordinates.  Per element an 80-value record, value 10 g + k of Gauss
 // point g = (Q00 Q01 Q02 Q10 Q11 Q12 Q20 Q21 Q22 det A)[k], stored as 20 rows
-// of 4 values: value v at geo[4 (v/4 * nelem + element) + v%4].
+// of 4 values, [nelem/32][20][32][4].
 template <class R>
 __global__ void __launch_bounds__(kElemThreads) k_elem_geo(const ElemArgs<R> A, float *geo) {
   static_assert(sizeof(R) == 4, "the geometry table serves the FP32 element kernels");
@@ -1254,7 +1252,6 @@ __global__ void __launch_bounds__(kElemThreads) k_elem_geo(const ElemArgs<R> A, 
 #pragma unroll
     for (int d = 0; d < 3; ++d) shX[d][i] = double(A.sX[d * A.S + s0 + i]);
   __syncthreads();
-  const long long gs = A.nelem;
   int bad = 0;
   for (int t = threadIdx.x; t < ne; t += blockDim.x) {
     const long long el = e0 + t - A.elem_begin;
@@ -1288,7 +1285,8 @@ __global__ void __launch_bounds__(kElemThreads) k_elem_geo(const ElemArgs<R> A, 
       for (int k = 0; k < 10; ++k) {
         const int v = 10 * g + k;
         const double q = k < 9 ? Ad[k / 3][k % 3] * id : det;
-        geo[4 * ((v >> 2) * gs + el) + (v & 3)] = float(q);
+        geo[(el >> 5) * (80 * kLaneBlk) + (v >> 2) * (4 * kLaneBlk) + (el & (kLaneBlk - 1)) * 4 + (v & 3)] =
+            float(q);
       }
     }
   }

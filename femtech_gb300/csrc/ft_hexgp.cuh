@@ -23,7 +23,7 @@
 // 1,000 Neo-Hookean 159 -> 22 us, 32,000 Ogden 1,004 -> 239 us (with the laws'
 // series, ft_materials.cuh); FP32 3,927 Ogden 18.9 -> 8.5 us.
 // Geometry: A^{-1} / 8 and det A of every Gauss point from a set-up table
-// [10][8 nelem] (the 1/8 of both transforms, exact).
+// [8 nelem/32][10][32] (the 1/8 of both transforms, exact).
 #pragma once
 
 #include "ft_elem.cuh"
@@ -183,7 +183,6 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
   const R cx = bx ? c : -c, cy = by ? c : -c, cz = bz ? c : -c;
   const int bits = __popc(l8);
   const R cp = bits < 2 ? R(1) : (bits == 2 ? c : c * c);
-  const long long GS = 8ll * A.nelem;
   cp_async_wait_all();
   if (A.use_clock && ck->done) return;  // past its end time: the whole block
   const R dt = A.use_clock ? R(ck->dt) : R(A.dt_direct);
@@ -198,10 +197,11 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
     const bool act = i < ne;
     const int e = e0 + (act ? i : 0);
     const long long el = e - A.elem_begin, sg = 8 * el + l8;
+    const R *geo = A.geo + blk_at(sg, 10);
     R Q[3][3];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) Q[k / 3][k % 3] = A.geo[k * GS + sg];
-    const R detA = A.geo[9 * GS + sg];
+    for (int k = 0; k < 9; ++k) Q[k / 3][k % 3] = geo[k * kLaneBlk];
+    const R detA = geo[9 * kLaneBlk];
     int ln = A.lconn[8 * el + corner];
     const int pw = A.epid[e];
     if (ln >= ns) {
@@ -281,12 +281,13 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
       R pc[4];
       prony_consts<R, MAT>(mp, dt, pc);
       const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + (8 * el + gp) * kMlpOut : nullptr;
+      R *hist = hist_comps(MAT) > 0 ? A.hist + blk_at(sg, hist_comps(MAT)) : nullptr;
       Sym6<R> S;
       if ((MAT == 5 || MAT == 7) && !act)  // (its history is another element's)
         S = Sym6<R>{0, 0, 0, 0, 0, 0};
       else
-        S = stress_at<R, MAT>(mp, D, Jm1, a0, A.hist + sg, GS, pc, sy, A.law,
-                              HistGlobal<R>{A.hist + sg, GS}, PartAt<R>{&mp});
+        S = stress_at<R, MAT>(mp, D, Jm1, a0, hist, pc, sy, A.law, HistGlobal<R>{hist},
+                              PartAt<R>{&mp});
       if (GP && act) {
         const long long q = A.gpbase + 8 * el + gp;
 #pragma unroll
@@ -371,7 +372,8 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
 
 // Set-up pass of a group that k_hexgp runs: A^{-1} / 8 (row major) and det A
 // of the reference geometry at each Gauss point (ShapeFunction_C3D8.cpp:35-120),
-// in FP64 from the slot coordinates, as [10][8 nelem], point 8 element + lane.
+// in FP64 from the slot coordinates, as [8 nelem/32][10][32] of points 8
+// element + lane.
 template <class R>
 __global__ void __launch_bounds__(kHexGpThreads) k_hexgp_geo(const ElemArgs<R> A, R *geo) {
   __shared__ double shX[3][kMaxLocalNodes];
@@ -382,7 +384,6 @@ __global__ void __launch_bounds__(kHexGpThreads) k_hexgp_geo(const ElemArgs<R> A
 #pragma unroll
     for (int d = 0; d < 3; ++d) shX[d][i] = double(A.sX[d * A.S + s0 + i]);
   __syncthreads();
-  const long long GS = 8ll * A.nelem;
   int bad = 0;
   for (int q = threadIdx.x; q < 8 * ne; q += blockDim.x) {
     const long long el = e0 + (q >> 3) - A.elem_begin;
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(kHexGpThreads) k_hexgp_geo(const ElemArgs<R> A
     adj3(Am, Ad, det);
     const double id = 0.125 / det;  // det = 0: non-finite entries, flagged by the force pass
 #pragma unroll
-    for (int k = 0; k < 10; ++k) geo[k * GS + 8 * el + l8] = R(k < 9 ? Ad[k / 3][k % 3] * id : det);
+    for (int k = 0; k < 10; ++k) geo[blk_at(8 * el + l8, 10) + k * kLaneBlk] = R(k < 9 ? Ad[k / 3][k % 3] * id : det);
   }
   if (bad) atomicOr(A.err, bad);
 }

@@ -61,11 +61,11 @@ inline int launch_strain<double>(int etype, int nblocks, int threads, size_t sme
 }
 
 // Setup pass of an FP32 C3D8 group (k_elem_geo): the Gauss points' inverse
-// reference Jacobians and determinants into geo ([20][nelem] x 4 values).
+// reference Jacobians and determinants into geo ([nelem/32][20][32][4]).
 // Returns a cudaError_t value.
 int launch_geo_f32(int nblocks, cudaStream_t s, const ElemArgs<float> &A, float *geo);
 
-// The eight-lane C3D8 pass (ft_hexgp.cuh) and its set-up table ([10][8 nelem])
+// The eight-lane C3D8 pass (ft_hexgp.cuh) and its set-up table (ten values per point)
 int launch_hexgp(int mat, int gp, int nblocks, int threads, size_t smem, cudaStream_t s,
                  const ElemArgs<float> &A, int pass);
 int launch_hexgp(int mat, int gp, int nblocks, int threads, size_t smem, cudaStream_t s,
