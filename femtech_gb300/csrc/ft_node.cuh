@@ -369,85 +369,203 @@ __device__ __forceinline__ float d2f_bits(double d) {
   return __uint_as_float(((t - (384u << 23)) & 0x7fffffffu) | (hi & 0x80000000u));
 }
 
+// f(slot) for the slots of node n in slot order: from its 16-byte records
+// (one round trip), or its list when it has more
+template <class F>
+__device__ __forceinline__ void for_slots(const NodeArgs &A, long long n, const int4 &sr,
+                                          const int4 &sr2, F f) {
+  if (sr.x == kSlotCsr) {
+    for (int k = A.slot_off[n]; k < A.slot_off[n + 1]; ++k) f(A.slots[k]);
+    return;
+  }
+  const int s[8] = {sr.x, sr.y, sr.z, sr.w, sr2.x, sr2.y, sr2.z, sr2.w};
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (s[j] >= 0) f(s[j]);
+}
+// f(partial force) for the slots of node n in slot order, four loads in
+// flight at a time
+template <class R, class F>
+__device__ __forceinline__ void for_partials(const NodeArgs &A, const Slot4<R> *sF, long long n,
+                                             const int4 &sr, const int4 &sr2, F f) {
+  if (sr.x == kSlotCsr) {
+    for (int k = A.slot_off[n]; k < A.slot_off[n + 1]; ++k) f(sF[A.slots[k]]);
+    return;
+  }
+  auto four = [&](const int4 &r) {
+    const int s[4] = {r.x, r.y, r.z, r.w};
+    Slot4<R> q[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (s[j] >= 0) q[j] = sF[s[j]];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (s[j] >= 0) f(q[j]);
+  };
+  four(sr);
+  if (A.slot4b) four(sr2);
+}
+// To and from the element precision by integer arithmetic: the hardware
+// conversions take slots of the FP64 pipe, one warp instruction in 16 cycles
+// (the first accelerations of 4.08 M nodes, 24 conversions a node: 515 us
+// with them, 369 without)
+template <class R> __device__ __forceinline__ R to_real(double x);
+template <> __device__ __forceinline__ float to_real<float>(double x) { return d2f_bits(x); }
+template <> __device__ __forceinline__ double to_real<double>(double x) { return x; }
+__device__ __forceinline__ double to_fp64(float x) { return f2d_bits(x); }
+__device__ __forceinline__ double to_fp64(double x) { return x; }
+
+// The rigid-rotation functions' trigonometry at time t, once per block that
+// holds a node with such a DOF (`driven`; every thread of the block calls):
+// per DOF it was nine FP64 sines and cosines a node (2 M tetrahedra with a
+// rotating skull: the boundary values 111 -> 26 us, the half-step that opens
+// a run 95 -> 29 us)
+__device__ __forceinline__ void block_rot_trig(const NodeArgs &A, bool driven, double t,
+                                               double (*trig)[3]) {
+  if (!__syncthreads_or(driven)) return;
+  if (threadIdx.x < A.nrot) {
+    double *r = trig[threadIdx.x];
+    rot_trig(A.fns[A.rot_ids[threadIdx.x]], t, r[0], r[1], r[2]);
+  }
+  __syncthreads();
+}
+// bc_value for the three DOFs of one node; trig: block_rot_trig's at t, null
+// where the block has them for another time
+struct NodeBc {
+  int of = -1;  // the rotation that ur, vr are of
+  double ur[3], vr[3];
+  __device__ __forceinline__ void value(const NodeArgs &A, int fn, int d, double t, long long n,
+                                        const double (*trig)[3], double &u, double &v) {
+    const BcFn &b = A.fns[fn];
+    if (trig && b.kind == kBckRot && b.pad >= 0 && b.pad < A.nrot) {
+      if (of != fn) {
+        const double *r = trig[b.pad];
+        rot_apply(b, r[0], r[1], r[2], A.X, A.N, n, ur, vr);
+        of = fn;
+      }
+      u = ur[d];
+      v = vr[d];
+    } else {
+      bc_value(b, d, t, A.X, A.N, n, u, v);
+    }
+  }
+};
+__device__ __forceinline__ bool is_rot(const NodeArgs &A, int fn) {
+  return fn >= 0 && A.fns[fn].kind == kBckRot;
+}
+
+// The node passes outside a fused step: the half-step that opens a run, the
+// first accelerations, and the scatter and gather of the single primitives.
 template <class R>
 __global__ void __launch_bounds__(512, 2) k_node(const NodeArgs A) {
-  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long n0 = (long long)blockIdx.x * blockDim.x, n = n0 + threadIdx.x;
+  // kNodeBegin: the block's first instance's step coefficients, formed once
+  // (four FP64 operations; the pipe takes one warp instruction in 16 cycles)
+  __shared__ double s_h, s_dt, s_t;
+  __shared__ double s_trig[kMaxRotFns][3];
+  __shared__ int s_inst;
+  if (A.mode == kNodeBegin) {
+    if (threadIdx.x == 0) {
+      s_inst = A.node_inst ? A.node_inst[n0] : 0;
+      const Clock &ck = A.clock[A.parity * A.ninst + s_inst];
+      const double t_np1 = ck.time + ck.dt;
+      s_t = t_np1;
+      s_dt = ck.dt;
+      s_h = 0.5 * (t_np1 + ck.time) - ck.time;
+    }
+    __syncthreads();
+    if (A.nrot) {
+      bool driven = false;
+      if (n < A.N)
+        for (int d = 0; d < 3; ++d) driven |= is_rot(A, A.nbc[d * A.N + n]);
+      block_rot_trig(A, driven, s_t, s_trig);
+    }
+  }
   if (n >= A.N) return;
   const int inst = A.node_inst ? A.node_inst[n] : 0;
-  const InstParams &ip = A.inst[inst];
-  const bool leader = (n == ip.node_begin);
   const Slot4<R> *sF = reinterpret_cast<const Slot4<R> *>(A.sF);
   Slot4<R> *sU = reinterpret_cast<Slot4<R> *>(A.sU);
-  const int sb = A.slot_off[n], se = A.slot_off[n + 1];
+  const int4 sr = A.slot4[n];
+  int4 sr2 = make_int4(-1, -1, -1, -1);
+  if (A.slot4b) sr2 = A.slot4b[n];
   const long long N = A.N;
 
   if (A.mode == kNodeScatterU) {  // replicate u into the patch slots
-    const Slot4<R> r{R(A.u[n]), R(A.u[N + n]), R(A.u[2 * N + n]), R(0)};
-    for (int k = sb; k < se; ++k) sU[A.slots[k]] = r;
+    const Slot4<R> r{to_real<R>(A.u[n]), to_real<R>(A.u[N + n]), to_real<R>(A.u[2 * N + n]), R(0)};
+    for_slots(A, n, sr, sr2, [&](int k) { sU[k] = r; });
     return;
   }
   if (A.mode == kNodeGather) {  // assembled internal force fi = sum of partials
     double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-    for (int k = sb; k < se; ++k) {
-      const Slot4<R> q = sF[A.slots[k]];
-      f0 += double(q.x);
-      f1 += double(q.y);
-      f2 += double(q.z);
-    }
+    for_partials(A, sF, n, sr, sr2, [&](const Slot4<R> &q) {
+      f0 += to_fp64(q.x);
+      f1 += to_fp64(q.y);
+      f2 += to_fp64(q.z);
+    });
     A.fi_out[n] = f0;
     A.fi_out[N + n] = f1;
     A.fi_out[2 * N + n] = f2;
     return;
   }
 
-  const Clock ck = A.clock[A.parity * A.ninst + inst];
+  const Clock &ck = A.clock[A.parity * A.ninst + inst];
   if (A.mode == kNodeBegin) {
     // first half of a step: v_half, u update, BCs at t_{n+1} (ex9.cpp:109-138)
     if (ck.done) return;
-    const double t_n = ck.time, dt = ck.dt, t_np1 = t_n + dt, t_half = 0.5 * (t_np1 + t_n);
+    double h = s_h, dt = s_dt, t_np1 = s_t;
+    if (inst != s_inst) {
+      dt = ck.dt;
+      t_np1 = ck.time + dt;
+      h = 0.5 * (t_np1 + ck.time) - ck.time;
+    }
+    int fn[3];
+    double uo[3], vo[3], ao[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      fn[d] = A.nbc[d * N + n];
+      uo[d] = A.u[d * N + n];
+      vo[d] = A.v[d * N + n];
+      ao[d] = A.a[d * N + n];
+    }
     double un[3];
     // rigid-body DOFs: the motion at t_{n+1} (k_rigid_begin advanced it)
     double ru[3] = {0.0, 0.0, 0.0}, rv[3] = {0.0, 0.0, 0.0}, ra[3] = {0.0, 0.0, 0.0};
     if (A.rbstep) {
       bool rig = false;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const int fn = A.nbc[d * N + n];
-        if (fn >= 0 && A.fns[fn].kind == kBckRigid) rig = true;
-      }
+      for (int d = 0; d < 3; ++d)
+        if (fn[d] >= 0 && A.fns[fn[d]].kind == kBckRigid) rig = true;
       if (rig) rigid_node(A.rbstep + inst, A.X, N, n, ru, rv, ra);
     }
+    NodeBc bc;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const int fn = A.nbc[d * N + n];
-      const double uold = A.u[d * N + n];
-      double u = uold;
-      if (fn == kBcFree) {
-        const double vh = A.v[d * N + n] + (t_half - t_n) * A.a[d * N + n];
+      double u = uo[d];
+      if (fn[d] == kBcFree) {
+        const double vh = vo[d] + h * ao[d];
         u = u + dt * vh;
         A.vh[d * N + n] = vh;
         A.u[d * N + n] = u;
-      } else if (fn >= 0 && A.fns[fn].kind == kBckRigid) {
+      } else if (fn[d] >= 0 && A.fns[fn[d]].kind == kBckRigid) {
         // v_half of a constrained DOF is unused: it keeps a_n + a_{n+1}, the
         // inertia term of the DOF's reaction in the energy balance
-        const double aold = A.a[d * N + n];
         u = ru[d];
         A.u[d * N + n] = u;
         A.v[d * N + n] = rv[d];
         A.a[d * N + n] = ra[d];
-        A.vh[d * N + n] = aold + ra[d];
-      } else if (fn >= 0) {
+        A.vh[d * N + n] = ao[d] + ra[d];
+      } else if (fn[d] >= 0) {
         double vb;
-        bc_value(A.fns[fn], d, t_np1, A.X, N, n, u, vb);
+        bc.value(A, fn[d], d, t_np1, n, inst == s_inst ? s_trig : nullptr, u, vb);
         A.u[d * N + n] = u;
         A.v[d * N + n] = vb;
         A.a[d * N + n] = 0.0;
       }
-      if (A.du) reinterpret_cast<R *>(A.du)[d * N + n] = R(u - uold);  // energy: this step's du
+      if (A.du) reinterpret_cast<R *>(A.du)[d * N + n] = R(u - uo[d]);  // energy: this step's du
       un[d] = u;
     }
-    const Slot4<R> r{R(un[0]), R(un[1]), R(un[2]), R(0)};
-    for (int k = sb; k < se; ++k) sU[A.slots[k]] = r;
+    const Slot4<R> r{to_real<R>(un[0]), to_real<R>(un[1]), to_real<R>(un[2]), R(0)};
+    for_slots(A, n, sr, sr2, [&](int k) { sU[k] = r; });
     return;
   }
   if (A.mode == kNodeInit) {
@@ -456,15 +574,16 @@ __global__ void __launch_bounds__(512, 2) k_node(const NodeArgs A) {
     // k_node_step sums them) and in FP64
     R fr[3] = {0, 0, 0};
     double fd[3] = {0.0, 0.0, 0.0};
-    for (int k = sb; k < se; ++k) {
-      const Slot4<R> q = sF[A.slots[k]];
-      fr[0] += q.x;
-      fr[1] += q.y;
-      fr[2] += q.z;
-      fd[0] += double(q.x);
-      fd[1] += double(q.y);
-      fd[2] += double(q.z);
-    }
+    for_partials(A, sF, n, sr, sr2, [&](const Slot4<R> &q) {
+      if (A.fprev) {
+        fr[0] += q.x;
+        fr[1] += q.y;
+        fr[2] += q.z;
+      }
+      fd[0] += to_fp64(q.x);
+      fd[1] += to_fp64(q.y);
+      fd[2] += to_fp64(q.z);
+    });
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       if (A.fprev) reinterpret_cast<R *>(A.fprev)[d * N + n] = fr[d];
@@ -472,10 +591,8 @@ __global__ void __launch_bounds__(512, 2) k_node(const NodeArgs A) {
       const double f = fd[d];
       A.a[d * N + n] = A.fp64 ? -f / A.mass[n] : -f * A.minv[n];
     }
-    if (leader) A.dtmin[A.parity * A.ninst + inst] = kDtHugeBits;
-    return;
+    if (n == A.inst[inst].node_begin) A.dtmin[A.parity * A.ninst + inst] = kDtHugeBits;
   }
-
 }
 
 // First function thread of k_step_scalars: the instances' warps come before
@@ -1079,13 +1196,20 @@ __global__ void k_clock_init(Clock *clock, unsigned long long *dtmin, const Inst
 template <class R>
 __global__ void k_apply_bc(const NodeArgs A, double t) {
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= A.N) return;
   const long long N = A.N;
+  __shared__ double s_trig[kMaxRotFns][3];
+  int fns[3] = {kBcFree, kBcFree, kBcFree};
+  if (n < N)
+    for (int d = 0; d < 3; ++d) fns[d] = A.nbc[d * N + n];
+  if (A.nrot)
+    block_rot_trig(A, is_rot(A, fns[0]) || is_rot(A, fns[1]) || is_rot(A, fns[2]), t, s_trig);
+  if (n >= N) return;
   const int inst = A.node_inst ? A.node_inst[n] : 0;
   double un[3];
+  NodeBc bc;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const int fn = A.nbc[d * N + n];
+    const int fn = fns[d];
     un[d] = A.u[d * N + n];
     if (fn < 0) continue;
     double u, v, a = 0.0;
@@ -1096,16 +1220,19 @@ __global__ void k_apply_bc(const NodeArgs A, double t) {
       v = rv[d];
       a = ra[d];
     } else {
-      bc_value(A.fns[fn], d, t, A.X, N, n, u, v);
+      bc.value(A, fn, d, t, n, s_trig, u, v);
     }
     A.u[d * N + n] = u;
     A.v[d * N + n] = v;
     A.a[d * N + n] = a;
     un[d] = u;
   }
-  const Slot4<R> r{R(un[0]), R(un[1]), R(un[2]), R(0)};
+  const Slot4<R> r{to_real<R>(un[0]), to_real<R>(un[1]), to_real<R>(un[2]), R(0)};
   Slot4<R> *sU = reinterpret_cast<Slot4<R> *>(A.sU);
-  for (int k = A.slot_off[n]; k < A.slot_off[n + 1]; ++k) sU[A.slots[k]] = r;
+  const int4 sr = A.slot4[n];
+  int4 sr2 = make_int4(-1, -1, -1, -1);
+  if (A.slot4b) sr2 = A.slot4b[n];
+  for_slots(A, n, sr, sr2, [&](int k) { sU[k] = r; });
 }
 
 }  // namespace ftgpu
