@@ -21,7 +21,7 @@
 // way back (Gauss points -> moments -> corners) takes 30 + 9.
 // Measured (element pass, one thread per element -> eight lanes): FP64
 // 1,000 Neo-Hookean 159 -> 22 us, 32,000 Ogden 1,004 -> 239 us (with the laws'
-// series, ft_materials.cuh); FP32 3,927 Ogden 18.9 -> 8.5 us.
+// series, ft_materials.cuh; 195 us with the step bounds); FP32 3,927 Ogden 18.9 -> 8.5 us.
 // Geometry: A^{-1} / 8 and det A of every Gauss point from a set-up table
 // [8 nelem/32][10][32] (the 1/8 of both transforms, exact).
 #pragma once
@@ -79,13 +79,19 @@ __device__ __forceinline__ bool is_zero(double x) {
 // The element's stable step l / c, l = volume / largest face area of the
 // current geometry (CalculateCharacteristicLength_C3D8.cpp:6-29, the face rule
 // of Geometry.cpp:29-64 with its signed parallelogram test), from the lane's
-// current corner y and its share detJ of the volume.  A lane takes the three
+// current corner y and vol, its share of the volume (SHARE) or the volume.  A lane takes the three
 // faces that meet in its corner, and on each the quadrature point next to it:
 // the face's tangents there are butterflies of the patterns (+-1 on the face's
 // axis, +-1/sqrt 3 or, for a parallelogram, 0 on the others).  All values in
 // units of 8 x the patterns.  Same on all eight lanes.
 template <class R>
-__device__ __forceinline__ R hexgp_dt(const R (&y)[3], R detJ, const MatP<R> &mp, bool bx, bool by,
+__device__ __forceinline__ R hexgp_volume(R detJ) {
+  detJ += shx(detJ, 1);
+  detJ += shx(detJ, 2);
+  return detJ + shx(detJ, 4);
+}
+template <bool SHARE, class R>
+__device__ __forceinline__ R hexgp_dt(const R (&y)[3], R vol, const MatP<R> &mp, bool bx, bool by,
                                       bool bz) {
   R h[3], w1[3], w2[3], w4[3];
   const int lane = threadIdx.x & 31;
@@ -138,18 +144,94 @@ __device__ __forceinline__ R hexgp_dt(const R (&y)[3], R detJ, const MatP<R> &mp
     const auto o = __shfl_xor_sync(0xffffffffu, am, m);
     am = o > am ? o : am;
   }
-  R vol = detJ;
-  vol += shx(vol, 1);
-  vol += shx(vol, 2);
-  vol += shx(vol, 4);
+  if (SHARE) vol = hexgp_volume(vol);
   if constexpr (sizeof(R) == 4) return R(64) * vol / from_ubits(am) * mp.inv_ce;
   return R(64) * vol / (from_ubits(am) * R(mp.ce));
+}
+
+// Bounds of the same step for FP64, in FP32: only the elements whose lower
+// bound is not above the block's least upper one (nor above the minimum so far)
+// take hexgp_dt, a quarter to a third of the pass' FP64 operations, on a pipe that issues one
+// warp instruction in 16 cycles (32,000 Ogden elements 245 -> 201 us a step,
+// 42,000 of material 7 362 -> 305; 86 % of the pipe then).  r: the current corner relative to the
+// element's first one; vol: the volume (FP64, rounded).  The arithmetic is
+// hexgp_dt's.  Errors, with eps = 2^-24 and Rm the largest |r|: the patterns
+// carry at most 32 eps Rm (inputs and three sums of up to 8 Rm), the face's
+// tangents 160 eps Rm, so a point's area sqrt 3 160 eps Rm (|a| + |b|) and the
+// face's sum four times that; 1200 takes in the roundings of the product, the
+// root and the sums.  A twist within its own error of the parallelogram test,
+// values outside FP32's comfortable range and NaNs leave the element undecided:
+// lo = 0, hi = inf.
+__device__ __forceinline__ void hexgp_dt_bounds(const float (&r)[3], float vol, float inv_ce, bool bx,
+                                                bool by, bool bz, float &lo, float &hi) {
+  constexpr float kEps = 1.f / 16777216.f;
+  const float inf = r_inf<float>();
+  const int lane = threadIdx.x & 31;
+  float rm = fmaxf(fmaxf(fabsf(r[0]), fabsf(r[1])), fabsf(r[2]));
+#pragma unroll
+  for (int m = 1; m <= 4; m <<= 1) rm = fmaxf(rm, shx(rm, m));
+  float h[3], w1[3], w2[3], w4[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    h[d] = had(had(had(r[d], 1, bx), 2, by), 4, bz);
+    w1[d] = __shfl_sync(0xffffffffu, h[d], lane | 1);
+    w2[d] = __shfl_sync(0xffffffffu, h[d], lane | 2);
+    w4[d] = __shfl_sync(0xffffffffu, h[d], lane | 4);
+  }
+  const float ox = bx ? 1.f : -1.f, oy = by ? 1.f : -1.f, oz = bz ? 1.f : -1.f;
+  const float t = 0.57735026918962576451f, tol = 8e-6f, dtw = 100.f * kEps * rm;
+  float size = rm >= 1e-8f && rm <= 1e8f ? 0.f : inf;  // largest |a| + |b|
+  auto face = [&](const float (&p)[3], const float (&q)[3], int m0, bool b0, float o0, int mA,
+                  bool bA, float oA, int mB, bool bB, float oB) {
+    float a[3], b[3], cD[3];
+    bool flat = true, open = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      a[d] = ev(p[d], m0, b0, o0);
+      b[d] = ev(q[d], m0, b0, o0);
+      const float x = shx(a[d], mB);
+      cD[d] = bB ? a[d] : x;
+      flat = flat && cD[d] < tol;
+      open = open || !(fabsf(cD[d] - tol) > dtw);
+      a[d] = bB ? x : a[d];
+      const float z = shx(b[d], mA);
+      b[d] = bA ? z : b[d];
+    }
+    const float kA = flat ? 0.f : t * oB, kB = flat ? 0.f : t * oA;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      a[d] += kA * cD[d];
+      b[d] += kB * cD[d];
+    }
+    const float nx = a[1] * b[2] - a[2] * b[1], ny = a[2] * b[0] - a[0] * b[2],
+                nz = a[0] * b[1] - a[1] * b[0];
+    size = fmaxf(size, open ? inf
+                            : (fabsf(a[0]) + fabsf(a[1]) + fabsf(a[2])) +
+                                  (fabsf(b[0]) + fabsf(b[1]) + fabsf(b[2])));
+    float s = sqrtf(nx * nx + ny * ny + nz * nz);
+    s += shx(s, mA);
+    return s + shx(s, mB);
+  };
+  float am = face(w1, w2, 4, bz, oz, 1, bx, ox, 2, by, oy);
+  am = fmaxf(am, face(w1, w4, 2, by, oy, 1, bx, ox, 4, bz, oz));
+  am = fmaxf(am, face(w2, w4, 1, bx, ox, 2, by, oy, 4, bz, oz));
+#pragma unroll
+  for (int m = 1; m <= 4; m <<= 1) {
+    am = fmaxf(am, shx(am, m));
+    size = fmaxf(size, shx(size, m));
+  }
+  const float err = 1200.f * kEps * rm * size;
+  const float v = 64.f * vol * inv_ce;
+  const float l = v / (am + err) * (1.f - 1e-6f), u = v / (am - err) * (1.f + 1e-6f);
+  lo = l > 1e-30f && l < 1e30f ? l : 0.f;
+  hi = am > err && u > 1e-30f && u < 1e30f ? u : inf;
 }
 
 // FP64: at most 128 registers (two blocks per SM, 16 warps); the pipe takes
 // one instruction in 16 cycles, so more warps would not help.  FP32: the small
 // meshes it serves put one block on an SM.
-template <class R, int MAT, bool GP, bool INJ>
+// BOUND: stable steps by hexgp_dt_bounds first (FP64 force passes).
+template <class R, int MAT, bool GP, bool INJ, bool BOUND = false>
 __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A, int pass) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Slot4<R> *shX = reinterpret_cast<Slot4<R> *>(smem_raw);
@@ -177,6 +259,11 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
   // lane l of the element: bits, corner and Gauss point of these signs
   const int l8 = t & 7;
   const bool bx = l8 & 1, by = l8 & 2, bz = l8 & 4;
+  // the elements' step bounds and volumes (BOUND)
+  R *shVol = shF + 24 * ne;
+  float *shLo = reinterpret_cast<float *>(shVol + ne);
+  __shared__ unsigned cut;  // least upper bound, as bits
+  if (BOUND && t == 0) cut = ubits(r_inf<float>());
   const int corner = (bz ? 4 : 0) + (by ? (bx ? 2 : 3) : (bx ? 1 : 0));
   const int gp = (bz ? 0 : 4) + (by ? (bx ? 2 : 3) : (bx ? 1 : 0));
   const R c = R(0.577350269189626);
@@ -245,8 +332,22 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
     }
     {
       const R y[3] = {xs.x + u[0], xs.y + u[1], xs.z + u[2]};
-      const auto b = ubits(hexgp_dt(y, J * detA, mp, bx, by, bz));
-      if (act && pw >= 0 && b < dmin) dmin = b;
+      if constexpr (BOUND) {
+        const R vol = hexgp_volume(J * detA);
+        float r[3], lo, hi;
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          r[d] = d2f_bits(y[d] - __shfl_sync(0xffffffffu, y[d], lane & 24));
+        hexgp_dt_bounds(r, d2f_bits(vol), d2f_bits(mp.inv_ce), bx, by, bz, lo, hi);
+        if (act && l8 == 0) {
+          shVol[i] = vol;
+          shLo[i] = pw >= 0 ? lo : r_inf<float>();
+          if (pw >= 0) atomicMin(&cut, ubits(hi));
+        }
+      } else {
+        const auto b = ubits(hexgp_dt<true>(y, J * detA, mp, bx, by, bz));
+        if (act && pw >= 0 && b < dmin) dmin = b;
+      }
     }
     if (pass == kPassDt) continue;
     if (act && (bad_j(J) || is_zero(detA))) bad |= 1;
@@ -339,6 +440,27 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
   if (pass == kPassSurrogateFeatures) return;  // features only (uniform per block)
   if (INJ && pass == kPassForce)
     injury_block_extremes<kHexGpThreads>(iv, ij, ic, reinterpret_cast<InjuryPart *>(A.inj_part) + p);
+  if constexpr (BOUND) {
+    // the exact steps of the elements that the bounds leave
+    __syncthreads();
+    unsigned long long *gmin = A.dtmin + A.parity * A.ninst + inst;
+    const float cutf = from_ubits(cut);
+    const unsigned long long seen = *reinterpret_cast<volatile unsigned long long *>(gmin);
+    for (int i0 = 0; i0 < ne; i0 += T >> 3) {
+      const int i = i0 + (t >> 3);
+      const float lo = i < ne ? shLo[i] : r_inf<float>();
+      const bool mine = lo <= cutf && lo < r_inf<float>() && ubits(f2d_bits(lo)) <= seen;
+      if (!__any_sync(0xffffffffu, mine)) continue;
+      const int e = e0 + (i < ne ? i : 0);
+      int ln = A.lconn[8ll * (e - A.elem_begin) + corner];
+      if (ln >= ns) ln = 0;
+      const Slot4<R> us = shU[ln], xs = shX[ln];
+      const R y[3] = {xs.x + us.x, xs.y + us.y, xs.z + us.z};
+      const auto b = ubits(hexgp_dt<false>(y, mine ? shVol[i] : R(1),
+                                           A.mats[A.epid[e] & 0x7fffffff], bx, by, bz));
+      if (mine && b < dmin) dmin = b;
+    }
+  }
   // block minimum of the time steps as bits (positive values order like them;
   // a negative or NaN step of an inverted element is larger than any)
 #pragma unroll
@@ -429,6 +551,9 @@ int hexgp_go(int gp, int nb, int th, size_t sm, cudaStream_t s, const ElemArgs<R
     return launch_pdl(A.pdl, k_hexgp<R, MAT, true, false>, nb, th, sm, s, A, pass);
   if (gp == kLaunchInjury)
     return launch_pdl(A.pdl, k_hexgp<R, MAT, false, true>, nb, th, sm, s, A, pass);
+  if constexpr (sizeof(R) == 8)
+    if (A.dt_bounds)
+      return launch_pdl(A.pdl, k_hexgp<R, MAT, false, false, true>, nb, th, sm, s, A, pass);
   return launch_pdl(A.pdl, k_hexgp<R, MAT, false, false>, nb, th, sm, s, A, pass);
 }
 

@@ -77,7 +77,8 @@ int launch_hexgp_geo(int nblocks, cudaStream_t s, const ElemArgs<double> &A, dou
 inline int hexgp_threads(int PE) { return PE >= 32 ? 256 : (8 * PE + 31) / 32 * 32; }
 template <class R>
 inline size_t hexgp_smem_bytes(int PE) {
-  return sizeof(R) * (8 * (size_t)kMaxLocalNodes + 24 * (size_t)PE);
+  return sizeof(R) * (8 * (size_t)kMaxLocalNodes + 24 * (size_t)PE) +
+         (sizeof(R) == 8 ? 12 * (size_t)PE : 0);
 }
 
 // Dynamic shared memory of one element block: node X and u records (4 values

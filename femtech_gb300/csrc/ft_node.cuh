@@ -340,35 +340,6 @@ __device__ __forceinline__ StepScalars step_scalars(const Clock &ck, const InstP
   return s;
 }
 
-// FP32 <-> FP64 conversions of the mixed nodal update by integer bit
-// arithmetic.  This GPU converts between FP32 and FP64 on its FP64 pipe (two
-// lanes per SM and cycle); a handful of integer operations give the same
-// bits for every normal number, and the rare others (zero, subnormal,
-// overflow, inf, NaN) take the hardware conversion.
-// float -> double: exact (rebias the exponent by 1023 - 127 = 896, widen the
-// mantissa).
-__device__ __forceinline__ double f2d_bits(float f) {
-  const unsigned b = __float_as_uint(f);
-  const unsigned ex = b & 0x7f800000u;
-  if (ex == 0u || ex == 0x7f800000u) return (double)f;
-  const unsigned hi = (b & 0x80000000u) | (((b >> 3) & 0x0fffffffu) + (896u << 20));
-  return __hiloint2double((int)hi, (int)(b << 29));
-}
-// double -> float, round to nearest even: the top 9 bits of (hi:lo) << 3 hold
-// the low exponent bits, the next 23 the kept mantissa; the 29 bits shifted
-// out decide the rounding (a carry into the exponent is the correct result,
-// up to infinity at the top of the range); the exponent is rebiased modulo
-// 512, exact for results in the normal FP32 range.
-__device__ __forceinline__ float d2f_bits(double d) {
-  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
-  const unsigned e11 = (hi >> 20) & 0x7ffu;
-  if (e11 <= 896u || e11 >= 1151u) return __double2float_rn(d);
-  unsigned t = __funnelshift_l(lo, hi, 3);
-  const unsigned rem = lo << 3;
-  t += (rem > 0x80000000u || (rem == 0x80000000u && (t & 1u))) ? 1u : 0u;
-  return __uint_as_float(((t - (384u << 23)) & 0x7fffffffu) | (hi & 0x80000000u));
-}
-
 // f(slot) for the slots of node n in slot order: from its 16-byte records
 // (one round trip), or its list when it has more
 template <class F>

@@ -78,3 +78,37 @@ def test_laws(mat, prec, tol):
 def test_ogden_series_and_eigen(strain, alpha, prec, tol):
     """Every count of series terms and the eigen-decomposition beyond them."""
     check(*case((4, 4, 4), 6, strain, seed=3, alpha=alpha), prec, tol)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(14, 14, 13), (43, 9, 8)])
+@pytest.mark.parametrize("scale,shift", [(1.0, 0.0), (1.0, 1e3), (5e3, 0.0), (1e-6, 0.0)])
+@pytest.mark.parametrize("kind", ["jitter", "box", "sliver"])
+def test_fp64_step_bounds(kind, scale, shift, shape):
+    """Meshes large enough for the FP32 bounds in front of the FP64 stable step:
+    no two elements alike, all alike (parallelogram faces, every bound equal),
+    and thin ones; far from the origin, and sizes at which the bounds leave the
+    twist test open (edges of 5 m) or their range (1e-9 m).  The step is that of
+    the FP64 evaluation of every element: its rounding, 1e-12, plus the
+    coordinates' own, 1e-16 of their size over an edge."""
+    from oracle.oracle import Oracle
+    mesh, mats, u = case(shape, 1, 0.05 if kind == "jitter" else 0.0, seed=5)
+    h = 1.0e-3
+    if kind != "jitter":
+        mesh = mg.hex_block(*shape, shape[0] * h, shape[1] * h, shape[2] * h)
+        u = np.zeros_like(u)
+    X = mesh["coordinates"].copy()
+    if kind == "sliver":
+        rng = np.random.default_rng(2)
+        X[:, 2] *= 1e-3
+        X += rng.uniform(-1, 1, X.shape) * [0.1 * h, 0.1 * h, 1e-4 * h]
+    mesh["coordinates"] = X * scale + shift
+    u = u * scale
+    m = ft.Model(mesh, mats, precision=ft.FP64)
+    ref = Oracle(mesh, mats).stable_time_step(u, np.zeros(len(u), np.int32))
+    tol = 1e-12 + 1e-16 * shift / (h * scale * (1e-3 if kind == "sliver" else 1.0)) * 8
+    assert abs(m.StableTimeStep(u) - ref) <= tol * ref
+    m.set_state(u, np.zeros_like(u), None, 0.0)
+    m.init_explicit(1.0, 0.0, 1.0e9)
+    assert abs(m.state()["dt"] - ref) <= tol * ref
+    m.close()
