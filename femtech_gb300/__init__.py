@@ -186,7 +186,7 @@ class Model:
     # ---- symbol-compatible primitives ----
     def GetForce(self, u, dt=0.0):
         """Internal force fi (and f_net = -fi) on displacements u, like GetForce()."""
-        fi = np.zeros(3 * self.nNodes)
+        fi = np.empty(3 * self.nNodes)
         _check(lib().ftgpu_get_force(self.h, np.ascontiguousarray(u, np.float64).ravel(),
                                      float(dt), fi.ctypes.data, None))
         return fi

@@ -357,7 +357,7 @@ struct ftgpu_model {
   std::vector<int> fn_owner;  // instance owning each boundary function, -1 none / shared
   DBuf nkind, fnval, rest_list;
   long long rest_n = 0;
-  DBuf dX, u, v, a, vh, mass, minv, fi;
+  DBuf dX, u, v, a, vh, mass, minv;
   DBuf gpF, gpJ, gpS;
   // graph of one chunk of steps (plain, and with timing events): the first
   // chunk of a run opens with the half-step of ex9.cpp:109-138 from (u, v,
@@ -374,6 +374,8 @@ struct ftgpu_model {
   std::vector<cudaEvent_t> prof_ev;
   Clock *h_clock = nullptr;  // pinned
   int *h_err = nullptr;          // [2] pinned
+  size_t h_io_bytes = 0;
+  double *h_io = nullptr;        // pinned: dt, error flags, a primitive's arrays in and out
   cudaEvent_t run_ev[2] = {};    // the clocks of a run's last two graphs are in h_clock
   // learned surrogate for material-7 groups
   ftgpu_surrogate *surr = nullptr;
@@ -391,6 +393,7 @@ struct ftgpu_model {
     for (cudaEvent_t e : prof_ev) cudaEventDestroy(e);
     if (h_clock) cudaFreeHost(h_clock);
     if (h_err) cudaFreeHost(h_err);
+    if (h_io) cudaFreeHost(h_io);
     for (cudaEvent_t e : run_ev)
       if (e) cudaEventDestroy(e);
     if (ev_fork) cudaEventDestroy(ev_fork);
@@ -527,7 +530,6 @@ NodeArgs node_args(ftgpu_model *m, int mode, int parity) {
   A.dtmin = m->dtmin.as<unsigned long long>();
   A.inst = m->instp.as<InstParams>();
   A.err = m->err.as<int>();
-  A.fi_out = m->fi.as<double>();
   A.N = m->nNodes;
   A.S = m->S;
   A.ninst = m->ninst;
@@ -823,32 +825,52 @@ int download_state3(ftgpu_model *m, DBuf *const d[3], double *const h[3]) {
 }
 
 // AoS [3N] host -> SoA [3][N] device (h == NULL: zero)
-int upload_aos(ftgpu_model *m, const double *h, DBuf &d) {
-  const long long N = m->nNodes;
-  if (!h) {
-    CK(cudaMemsetAsync(d.p, 0, 3 * N * sizeof(double), m->stream));
-    CK(cudaStreamSynchronize(m->stream));
-    return 0;
+// Displacements of one primitive (null: zero) into u and the patch slots.
+// Up to kIoDirect bytes the kernels read and write page-locked memory of the
+// model in place, and the caller's arrays are copied by the host; above, the
+// copies are the link's, which one host thread does not keep up with (internal
+// force in place / by copies: 28 KB 57 / 86 us, 283 KB 130 / 140 us, 460 KB
+// 196 / 191 us).
+constexpr size_t kIoDirect = 384 << 10;
+size_t io_bytes(const ftgpu_model *m) { return 3 * (size_t)m->nNodes * sizeof(double); }
+bool io_direct(const ftgpu_model *m) { return io_bytes(m) <= kIoDirect; }
+int ensure_io(ftgpu_model *m) {
+  const size_t need = 16 + (io_direct(m) ? 2 * io_bytes(m) : 0);
+  if (m->h_io_bytes < need) {
+    if (m->h_io) CK(cudaFreeHost(m->h_io));
+    m->h_io = nullptr;
+    m->h_io_bytes = 0;
+    CK(cudaMallocHost((void **)&m->h_io, need));
+    m->h_io_bytes = need;
   }
-  CKI(ensure_stage(m));
-  CK(cudaMemcpyAsync(m->stage.p, h, 3 * N * sizeof(double), cudaMemcpyHostToDevice, m->stream));
-  k_aos_to_soa<<<(unsigned)((N + 255) / 256), 256, 0, m->stream>>>(m->stage.as<double>(),
-                                                                    d.as<double>(), N);
-  CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(m->stream));
-  return 0;
+  return io_direct(m) ? 0 : ensure_stage(m);
 }
+double *io_dt(ftgpu_model *m) { return m->h_io; }
+int *io_err(ftgpu_model *m) { return reinterpret_cast<int *>(m->h_io + 1); }
+double *io_in(ftgpu_model *m) { return io_direct(m) ? m->h_io + 2 : m->stage.as<double>(); }
+double *io_out(ftgpu_model *m) {
+  return io_direct(m) ? m->h_io + 2 + 3 * (size_t)m->nNodes : m->stage.as<double>();
+}
+unsigned io_blocks(const ftgpu_model *m) { return (unsigned)((m->nNodes + kIoThreads - 1) / kIoThreads); }
 
-int download_aos(ftgpu_model *m, const DBuf &d, double *h) {
-  if (!h) return 0;
-  const long long N = m->nNodes;
-  CKI(ensure_stage(m));
-  k_soa_to_aos<<<(unsigned)((N + 255) / 256), 256, 0, m->stream>>>(d.as<double>(),
-                                                                    m->stage.as<double>(), N);
-  CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(h, m->stage.p, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, m->stream));
-  CK(cudaStreamSynchronize(m->stream));
-  return 0;
+int scatter_in(ftgpu_model *m, const double *u) {
+  CKI(ensure_io(m));
+  if (io_direct(m)) {
+    if (u)
+      memcpy(io_in(m), u, io_bytes(m));
+    else
+      memset(io_in(m), 0, io_bytes(m));
+  } else if (u) {
+    CK(cudaMemcpyAsync(io_in(m), u, io_bytes(m), cudaMemcpyHostToDevice, m->stream));
+  } else {
+    CK(cudaMemsetAsync(io_in(m), 0, io_bytes(m), m->stream));
+  }
+  const NodeArgs A = node_args(m, kNodeScatterU, 0);
+  if (is_fp64(m))
+    k_scatter_in<double><<<io_blocks(m), kIoThreads, 0, m->stream>>>(A, io_in(m));
+  else
+    k_scatter_in<float><<<io_blocks(m), kIoThreads, 0, m->stream>>>(A, io_in(m));
+  return (int)cudaGetLastError();
 }
 
 // Reference layout and principal strains of the averaged Green strain of
@@ -922,14 +944,16 @@ int strain_groups_t(ftgpu_model *m, double *E6) {
   return 0;
 }
 
-int check_err(ftgpu_model *m) {
-  CK(cudaMemcpyAsync(m->h_err, m->err.p, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
-  CK(cudaStreamSynchronize(m->stream));
-  int e = *m->h_err;
+int check_flags(int e) {
   if (e & kErrInverted) return fail(FTGPU_ERR_INVERTED, "non-positive or non-finite Jacobian");
   if (e & kErrIndex) return fail(FTGPU_ERR_INPUT, "local node index out of range");
   if (e & kErrWait) return fail(FTGPU_ERR_CUDA, "tensor-core inference gave up waiting");
   return 0;
+}
+int check_err(ftgpu_model *m) {
+  CK(cudaMemcpyAsync(m->h_err, m->err.p, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+  CK(cudaStreamSynchronize(m->stream));
+  return check_flags(*m->h_err);
 }
 
 // Per-element part word: part | (1 << 31) when every node of the element has
@@ -1207,7 +1231,7 @@ int setup_t(ftgpu_model *m) {
       for (int d = 0; d < 3; ++d) xs[d * N + n] = m->X[3 * n + d];
     CKI(m->dX.upload(xs.data(), xs.size()));
   }
-  for (DBuf *b : {&m->u, &m->v, &m->a, &m->vh, &m->fi}) {
+  for (DBuf *b : {&m->u, &m->v, &m->a, &m->vh}) {
     CKI(b->alloc(3 * N * sizeof(double)));
     CK(cudaMemset(b->p, 0, 3 * N * sizeof(double)));
   }
@@ -1738,40 +1762,40 @@ int ftgpu_num_gauss_points(ftgpu_model *m) {
 int ftgpu_get_force(ftgpu_model *m, const double *u, double dt, double *fi, double *f_net) {
   if (!m || !m->setup_done) return fail(FTGPU_ERR_STATE, "get_force before setup");
   CK(cudaSetDevice(m->device));
-  CKI(upload_aos(m, u, m->u));
-  CKI(launch_node(m, kNodeScatterU, 0));
   CKI(ensure_gp(m));
-  CKI(fill_dtmin(m));
+  CKI(scatter_in(m, u));
   CKI(launch_groups(m, 0, 0, dt, 1, 0));
-  CKI(launch_node(m, kNodeGather, 0));
-  CKI(check_err(m));
-  std::vector<double> h(3 * (size_t)m->nNodes);
-  CKI(download_aos(m, m->fi, h.data()));
-  if (fi) memcpy(fi, h.data(), h.size() * sizeof(double));
+  const NodeArgs A = node_args(m, kNodeScatterU, 0);
+  if (is_fp64(m))
+    k_gather_out<double><<<io_blocks(m), kIoThreads, 0, m->stream>>>(A, io_out(m), io_err(m));
+  else
+    k_gather_out<float><<<io_blocks(m), kIoThreads, 0, m->stream>>>(A, io_out(m), io_err(m));
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(m->stream));
+  CKI(check_flags(*io_err(m)));
+  double *out = fi ? fi : f_net;
+  if (!out) return FTGPU_OK;
+  if (io_direct(m)) {
+    memcpy(out, io_out(m), io_bytes(m));
+  } else {
+    const HostDrain::Part part = {out, io_out(m), io_bytes(m)};
+    CKI(m->drain.copy(m->device, m->stream, &part, 1));
+  }
   if (f_net)
-    for (size_t i = 0; i < h.size(); ++i) f_net[i] = -h[i];
+    for (size_t i = 0; i < 3 * (size_t)m->nNodes; ++i) f_net[i] = -out[i];
   return FTGPU_OK;
 }
 
 int ftgpu_stable_time_step(ftgpu_model *m, const double *u, double *dt_min) {
   if (!m || !m->setup_done || !dt_min) return fail(FTGPU_ERR_STATE, "stable_time_step before setup");
   CK(cudaSetDevice(m->device));
-  CKI(upload_aos(m, u, m->u));
-  CKI(launch_node(m, kNodeScatterU, 0));
-  CKI(fill_dtmin(m));
+  CKI(scatter_in(m, u));
   CKI(launch_groups(m, 0, 0, 0.0, 0, 1));
-  std::vector<unsigned long long> h(2 * m->ninst);
-  CK(cudaMemcpyAsync(h.data(), m->dtmin.p, h.size() * 8, cudaMemcpyDeviceToHost, m->stream));
+  k_dt_out<<<1, kIoThreads, 0, m->stream>>>(node_args(m, kNodeScatterU, 0), io_dt(m), io_err(m));
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(m->stream));
-  double mn = 1e20;  // "huge" of GlobalVariables.h:15
-  for (int i = 0; i < m->ninst; ++i) {
-    double v;
-    memcpy(&v, &h[i], 8);
-    mn = std::min(mn, v);
-  }
-  *dt_min = mn;
-  CKI(fill_dtmin(m));
-  return check_err(m);
+  *dt_min = std::min(1e20, *io_dt(m));  // "huge" of GlobalVariables.h:15
+  return check_flags(*io_err(m));
 }
 
 int ftgpu_get_gauss_points(ftgpu_model *m, double *F, double *detF, double *pk2) {

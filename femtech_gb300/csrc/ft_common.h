@@ -235,7 +235,6 @@ struct NodeArgs {
   unsigned long long *dtmin;
   const InstParams *inst;
   int *err;
-  double *fi_out;             // optional [3][N] assembled internal force
   long long N, S;
   int ninst, parity;
   int mode;                   // kNodeBegin / kNodeFused / kNodeFinish / kNodeInit
@@ -263,8 +262,7 @@ struct NodeArgs {
   long long epart_off;
 };
 
-enum { kNodeBegin = 0, kNodeFused = 1, kNodeFinish = 2, kNodeInit = 3, kNodeGather = 4,
-       kNodeScatterU = 5 };
+enum { kNodeBegin = 0, kNodeFused = 1, kNodeFinish = 2, kNodeInit = 3, kNodeScatterU = 4 };
 
 #ifdef __CUDACC__
 // FP32 <-> FP64 conversions by integer bit arithmetic.  This GPU converts between FP32 and FP64 on its FP64 pipe (two

@@ -829,16 +829,39 @@ __device__ __forceinline__ void tet_element(const R (&x)[4][3], const R (&u)[4][
 #pragma unroll
     for (int d = 0; d < 3; ++d) xc[a][d] = x[a][d] + u[a][d];
   R six_v = fabs((1 + Jm1) * detA);
-  constexpr int fc[4][3] = {{1, 2, 3}, {2, 3, 0}, {3, 0, 1}, {0, 1, 2}};
-  R nmax = 0;
+  // the root of the largest square: the roots' maximum, bit for bit
+  R n2 = 0;
+  if (sizeof(R) == 8) {
+    // the edges from corner 3, three cross products, and the opposite face's
+    // normal as their sum: half the FP64 operations that the faces take one by
+    // one
+    R e[3][3];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int p1 = fc[k][0], p2 = fc[k][1], p3 = fc[k][2];
-    R v1x = xc[p2][0] - xc[p1][0], v1y = xc[p2][1] - xc[p1][1], v1z = xc[p2][2] - xc[p1][2];
-    R v2x = xc[p3][0] - xc[p1][0], v2y = xc[p3][1] - xc[p1][1], v2z = xc[p3][2] - xc[p1][2];
-    R n = norm3(v1y * v2z - v1z * v2y, v1z * v2x - v1x * v2z, v1x * v2y - v1y * v2x);
-    nmax = fmax(nmax, n);
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) e[r][d] = xc[r][d] - xc[3][d];
+    R s[3] = {0, 0, 0};
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const R(&p)[3] = e[r], (&q)[3] = e[(r + 1) % 3];
+      const R n[3] = {p[1] * q[2] - p[2] * q[1], p[2] * q[0] - p[0] * q[2], p[0] * q[1] - p[1] * q[0]};
+      n2 = fmax(n2, n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) s[d] += n[d];
+    }
+    n2 = fmax(n2, s[0] * s[0] + s[1] * s[1] + s[2] * s[2]);
+  } else {
+    constexpr int fc[4][3] = {{1, 2, 3}, {2, 3, 0}, {3, 0, 1}, {0, 1, 2}};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int p1 = fc[k][0], p2 = fc[k][1], p3 = fc[k][2];
+      R v1x = xc[p2][0] - xc[p1][0], v1y = xc[p2][1] - xc[p1][1], v1z = xc[p2][2] - xc[p1][2];
+      R v2x = xc[p3][0] - xc[p1][0], v2y = xc[p3][1] - xc[p1][1], v2z = xc[p3][2] - xc[p1][2];
+      const R nx = v1y * v2z - v1z * v2y, ny = v1z * v2x - v1x * v2z, nz = v1x * v2y - v1y * v2x;
+      n2 = fmax(n2, nx * nx + ny * ny + nz * nz);
+    }
   }
+  const R nmax = d_sqrt(n2);
   le = six_v / nmax;
   const long long sg = gpo - A.gpbase;  // Gauss point within the group
   if (MAT == 7 && pass == kPassSurrogateFeatures) {
