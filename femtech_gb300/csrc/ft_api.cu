@@ -599,6 +599,16 @@ int launch_node(ftgpu_model *m, int mode, int parity) {
   };
   const bool fork = step && m->rig_nodes > 0 && m->stream2;
   const int pdl = m->step_pdl;
+  if (fork) {
+    // fork: the driven nodes' motion (rigid bodies' integrator, rotation
+    // trigonometry) and, when the step scalars are there too, those nodes on
+    // the second stream, every other node on the first; join before what
+    // follows
+    CK(cudaEventRecord(m->ev_fork, m->stream));
+    CK(cudaStreamWaitEvent(m->stream2, m->ev_fork, 0));
+    k_driven_step<<<(unsigned)m->ninst, 32, 0, m->stream2>>>(A);
+    CK(cudaGetLastError());
+  }
   if (step) {  // (with the fork, the rotation trigonometry moves to k_driven_step)
     NodeArgs S = A;
     if (fork) S.nrot = 0;
@@ -606,9 +616,6 @@ int launch_node(ftgpu_model *m, int mode, int parity) {
     CKI(launch_pdl(pdl, k_step_scalars, (nth + 127) / 128, 128, 0, m->stream, S));
   }
   if (fork) {
-    // fork: the driven nodes' motion (rigid bodies' integrator, rotation
-    // trigonometry) and then those nodes on the second stream, every other
-    // node on the first; join before what follows
     const long long nbr = (m->rig_nodes + th - 1) / th;
     NodeArgs B = A;
     B.node_list = m->rig_list.as<int>();
@@ -617,7 +624,6 @@ int launch_node(ftgpu_model *m, int mode, int parity) {
     A.skip_driven = 1;
     CK(cudaEventRecord(m->ev_fork, m->stream));
     CK(cudaStreamWaitEvent(m->stream2, m->ev_fork, 0));
-    k_driven_step<<<(unsigned)m->ninst, 32, 0, m->stream2>>>(B);
     CKI(node_step(0, nbr, m->stream2, B));
     if (!f64 && !en && A.nkind) {  // every other node: the split, as below
       k_node_free<<<(unsigned)nb, th, 0, m->stream>>>(A);

@@ -702,19 +702,22 @@ __global__ void k_step_scalars(const NodeArgs A) {
     }
 }
 
-// The driven nodes' motion at t_{n+2} for the next step, after
-// k_step_scalars, one warp per instance: the rigid body's integrator step
-// (ex5.cpp:344 with Time = t_{n+2}, dt = the new dt) and the trigonometry of
-// the rigid-rotation functions (lane k: function k).  It runs on a second
-// stream beside k_node_step over the nodes without such DOFs: the integrator
-// and sin/cos are latency-bound FP64 chains, the free-node update is
-// bandwidth-bound, and only the driven nodes (k_node_step over their list,
-// after this kernel) need the result.
+// The driven nodes' motion at t_{n+2} for the next step, one warp per
+// instance: the rigid body's integrator step (ex5.cpp:344 with Time = t_{n+2},
+// dt = the new dt) and the trigonometry of the rigid-rotation functions (lane
+// k: function k).  It runs on a second stream beside k_step_scalars and
+// k_node_step over the nodes without such DOFs: the integrator and sin/cos are
+// latency-bound FP64 chains, the free-node update is bandwidth-bound, and only
+// the driven nodes (k_node_step over their list, after this kernel) need the
+// result.  It forms the instance's step scalars itself, from the same values:
+// waiting for k_step_scalars' put that kernel on the branch's chain (300,000
+// tetrahedra with a rigid skull 51.9 -> 50.4 us a step, 200,000 with a rotation
+// and the surrogate 64.0 -> 62.7).
 __global__ void __launch_bounds__(32) k_driven_step(const NodeArgs A) {
   __shared__ double sacc[5][6];
   const int i = blockIdx.x;
   const Clock ck = A.clock[A.parity * A.ninst + i];
-  const StepScalars sc = A.stepsc[i];
+  const StepScalars sc = step_scalars(ck, A.inst[i], A.dtmin[A.parity * A.ninst + i], A.mode);
   if (!sc.advance || ck.done) return;
   const int k = threadIdx.x;
   if (k < A.nrot) {
