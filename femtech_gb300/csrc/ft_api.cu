@@ -1268,7 +1268,6 @@ int setup_t(ftgpu_model *m) {
     CKI(b->alloc(3 * N * sizeof(double)));
     CK(cudaMemset(b->p, 0, 3 * N * sizeof(double)));
   }
-  CKI(upload_bc(m));
   // instances
   if (!m->inst_set) {
     m->ninst = 1;
