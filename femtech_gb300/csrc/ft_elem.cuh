@@ -962,6 +962,23 @@ __device__ __forceinline__ void injury_element(const ElemArgs<R> &A, int c, cons
   above[1] = psxsr > inj_run<R>(q, 1);
 }
 
+// One element's values v into its thread's extremes.  Only through the
+// comparison: a shear that is NaN (the trigonometric roots just outside acos'
+// domain) never wins one and stays out, while taken as the thread's value it
+// would stand for the warp's others in the butterfly below, none of them
+// comparing better.
+template <class R>
+__device__ __forceinline__ void injury_take(const R (&v)[4], const int (&vj)[4], const int (&vc)[4],
+                                            R (&best)[4], int (&jj)[4], int (&cc)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (inj_better(k, v[k], vj[k], best[k], jj[k])) {
+      best[k] = v[k];
+      jj[k] = vj[k];
+      cc[k] = vc[k];
+    }
+}
+
 // A warp's values above a running percentile into the step's candidates (in
 // any order: only the values are selected from).  Every lane calls it.
 template <class R>
@@ -1207,7 +1224,12 @@ __global__ void __launch_bounds__(kElemThreads, (ET == 0 || sizeof(R) == 8) ? 2 
         for (int d = 0; d < 3; ++d) shF[(a * 3 + d) * PE + t] = f[a][d];
     }
     if (!skip) dte = dt_of<R>(le, mp);
-    if (INJ && ci >= 0) injury_element<R>(A, ci, Es, dt, iv, ij, ic, above);
+    if (INJ && ci >= 0) {
+      R v[4];
+      int vj[4], vc[4];
+      injury_element<R>(A, ci, Es, dt, v, vj, vc, above);
+      injury_take<R>(v, vj, vc, iv, ij, ic);
+    }
   }
   if (INJ && pass == kPassForce) {
     injury_append<R>(A, 0, above[0], iv[0]);

@@ -366,13 +366,7 @@ __global__ void __launch_bounds__(kHexGpThreads, 2) k_hexgp(const ElemArgs<R> A,
       if (ci >= 0) {
         int vj[4], vc[4];
         injury_element<R>(A, ci, Es, dt, v, vj, vc, above);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (inj_better(k, v[k], vj[k], iv[k], ij[k])) {
-            iv[k] = v[k];
-            ij[k] = vj[k];
-            ic[k] = vc[k];
-          }
+        injury_take<R>(v, vj, vc, iv, ij, ic);
       }
       injury_append<R>(A, 0, above[0], v[0]);
       injury_append<R>(A, 1, above[1], v[3]);

@@ -272,10 +272,7 @@ __device__ __forceinline__ void injury_extremes(const InjuryArgs<R> &A, double t
     const InjuryPart p = A.part[b];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      // (a NaN -- the trigonometric roots just outside acos' domain -- is no extreme)
-      const uint64_t a = (uint64_t)__double_as_longlong(p.v[k]) & 0x7fffffffffffffffull;
-      if (a > 0x7ff0000000000000ull) continue;
-      const uint64_t x = fkey(p.v[k]);
+      const uint64_t x = fkey(p.v[k]);  // (never a NaN: injury_take)
       take(k, k == 1 ? ~x : x, p.j[k], p.c[k]);
     }
   }
