@@ -583,7 +583,7 @@ int beside_begin(ftgpu_model *m, cudaStream_t &st) {
   return 0;
 }
 
-int launch_node(ftgpu_model *m, int mode, int parity) {
+int launch_node(ftgpu_model *m, int mode, int parity, bool seam = false) {
   NodeArgs A = node_args(m, mode, parity);
   const int th = m->node_threads;
   long long nb = (m->nNodes + th - 1) / th;
@@ -613,7 +613,8 @@ int launch_node(ftgpu_model *m, int mode, int parity) {
     NodeArgs S = A;
     if (fork) S.nrot = 0;
     const long long nth = step_scalar_fn0(m->ninst) + (A.nkind ? (long long)m->fns.size() : 0);
-    CKI(launch_pdl(pdl, k_step_scalars, (nth + 127) / 128, 128, 0, m->stream, S));
+    CKI(launch_pdl(pdl, seam ? k_step_scalars<true> : k_step_scalars<false>, (nth + 127) / 128, 128,
+                   0, m->stream, S));
   }
   if (fork) {
     const long long nbr = (m->rig_nodes + th - 1) / th;
@@ -1463,7 +1464,7 @@ int capture_chunk(ftgpu_model *m, int K, bool prof, bool open = true) {
       r = (int)cudaEventRecordWithFlags(m->prof_ev[2 * k + 1], m->stream, cudaEventRecordExternal);
     if (!r && m->injury_on) r = launch_injury(m, k & 1);
     if (!r && k > 0) r = join(m->energy_on, m->ev_en);
-    if (!r) r = launch_node(m, prof && k == K - 1 ? kNodeFinish : kNodeFused, k & 1);
+    if (!r) r = launch_node(m, prof && k == K - 1 ? kNodeFinish : kNodeFused, k & 1, !prof && k == K - 1);
   }
   if (prof && !r) r = (int)cudaEventRecordWithFlags(m->prof_ev[2 * K], m->stream, cudaEventRecordExternal);
   if (!r) r = join(m->injury_on, m->ev_inj);
@@ -1509,7 +1510,7 @@ int run_impl(ftgpu_model *m, int max_steps, int *steps_done, bool prof, double *
   CK(cudaStreamSynchronize(m->stream));
   const long long start0 = m->h_clock[0].step;
   for (int i = 0; i < ni; ++i) {
-    m->h_clock[i].done &= ~2;  // a new run lifts the previous step limit
+    m->h_clock[i].done &= ~(2 | kDoneHalt);  // a new run lifts the previous one's limit and halt
     m->inst[i].step_limit = m->h_clock[i].step + max_steps;
   }
   CK(cudaMemcpyAsync(m->clock.p, m->h_clock, sizeof(Clock) * ni, cudaMemcpyHostToDevice, m->stream));
@@ -1526,9 +1527,9 @@ int run_impl(ftgpu_model *m, int max_steps, int *steps_done, bool prof, double *
   }
   // Every launch advances each running instance by its steps (or ends it).  Up
   // to two graphs are on their way: the next one is launched before the host
-  // has read the clocks of the one before (a graph of an ended run moves
-  // nothing), so the GPU does not wait for the host between graphs.  The
-  // timing graph is read back one at a time.
+  // has read the clocks of the one before (a graph of an ended run, or behind
+  // one with an error, moves nothing), so the GPU does not wait for the host
+  // between graphs.  The timing graph is read back one at a time.
   const int deep = prof ? 1 : 2;
   for (int k = 0; k < 2; ++k)
     if (!m->run_ev[k]) CK(cudaEventCreateWithFlags(&m->run_ev[k], cudaEventDisableTiming));
@@ -1577,7 +1578,7 @@ int run_impl(ftgpu_model *m, int max_steps, int *steps_done, bool prof, double *
       }
     }
     prev = ck[0].step;
-    if (stop) continue;  // (a graph behind the one that ended the run)
+    if (stop) continue;  // (a graph behind the one that ended the run: the same clocks)
     bool all = true, dterr = false;
     long long most = 0;
     for (int i = 0; i < ni; ++i) {
@@ -2037,7 +2038,7 @@ int ftgpu_get_instance_clock(ftgpu_model *m, double *time, double *dt, long long
     if (time) time[i] = c[i].time;
     if (dt) dt[i] = c[i].dt;
     if (step) step[i] = c[i].step;
-    if (done) done[i] = c[i].done;
+    if (done) done[i] = c[i].done & ~kDoneHalt;
   }
   return FTGPU_OK;
 }

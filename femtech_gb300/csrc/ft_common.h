@@ -38,9 +38,12 @@ struct Clock {
   double time;     // t_n
   double dt;       // dt_n (the next step's increment)
   long long step;  // steps completed
-  int done;        // bit0 tMax reached, bit1 step limit, bit2 error
+  int done;        // bit0 tMax reached, bit1 step limit, bit2 error, kDoneHalt
   int err;
 };
+// An error ended the run with the graph that this clock closes: the graphs
+// queued behind it move nothing (k_step_scalars).  Cleared by the next run.
+constexpr int kDoneHalt = 8;
 
 struct InstParams {
   double tmax;

@@ -657,9 +657,27 @@ __host__ __device__ inline int step_scalar_fn0(int ninst) { return (ninst + 31) 
 // the values node_step's bc_value would compute per DOF.
 // Warps of instances first, then warps of functions, so that one thread's
 // sine does not stand before its clock.
+// SEAM: the last step of a graph that others may be queued behind.  An error
+// ends the run of every instance with the graph that it shows up in, as if the
+// host had read it before it launched the next: an element pass' error word,
+// final here, or another instance's failed step.  (A kernel of its own: with
+// the test in the other steps' code their launches took 0.12 us more.)
+template <bool SEAM>
 __global__ void k_step_scalars(const NodeArgs A) {
   step_wait();  // the dt minimum is the element pass'
   step_release();
+  const int err = SEAM ? *A.err : 0;
+  int halt = 0;
+  if (SEAM && A.ninst > 1) {
+    bool h = false;
+    for (int k = threadIdx.x; k < A.ninst; k += blockDim.x) {
+      const int done = A.clock[A.parity * A.ninst + k].done;
+      const double raw = __longlong_as_double((long long)A.dtmin[A.parity * A.ninst + k]);
+      const bool low = raw < A.inst[k].failure_dt;
+      h = h || (done ? (done & 4) != 0 : low);
+    }
+    halt = __syncthreads_or(h) ? kDoneHalt : 0;
+  }
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int f = i - step_scalar_fn0(A.ninst);
   if (f >= 0) {
@@ -680,7 +698,11 @@ __global__ void k_step_scalars(const NodeArgs A) {
   }
   if (i >= A.ninst) return;
   const Clock ck = A.clock[A.parity * A.ninst + i];
-  const StepScalars sc = step_scalars(ck, A.inst[i], A.dtmin[A.parity * A.ninst + i], A.mode);
+  StepScalars sc = step_scalars(ck, A.inst[i], A.dtmin[A.parity * A.ninst + i], A.mode);
+  if (SEAM) {
+    if (err & (kErrInverted | kErrWait)) halt = kDoneHalt;
+    sc.done |= halt;  // (sc.advance stands: this step is an ordinary one)
+  }
   A.stepsc[i] = sc;
   // the instance's clock for the next step and its fresh dt-minimum slot
   // (the other parity: nothing reads them before the next element pass).

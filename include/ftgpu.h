@@ -215,7 +215,9 @@ int ftgpu_init_explicit(ftgpu_model *m, double reduction, double failure_dt, dou
 /* Advance every instance by up to max_steps central-difference steps
  * (ex9.cpp:107-175) or until Time >= tMax; the loop runs on the device as
  * CUDA graphs of 16 steps and, at the end of the run, one of 2-14 steps.
- * *steps_done = steps taken by instance 0. */
+ * *steps_done = steps taken by instance 0.  An error (an inverted element, a
+ * step below FailureTimeStep) ends the run of all instances with the graph it
+ * occurs in, up to 15 steps later; the state read back is that graph's end. */
 int ftgpu_run(ftgpu_model *m, int max_steps, int *steps_done);
 
 /* ftgpu_run with CUDA events recorded on the model's stream around the whole
