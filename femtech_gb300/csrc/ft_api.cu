@@ -1529,18 +1529,31 @@ int run_impl(ftgpu_model *m, int max_steps, int *steps_done, bool prof, double *
   // to two graphs are on their way: the next one is launched before the host
   // has read the clocks of the one before (a graph of an ended run, or behind
   // one with an error, moves nothing), so the GPU does not wait for the host
-  // between graphs.  The timing graph is read back one at a time.
+  // between graphs.  Not where the graphs on their way should reach every
+  // tMax, at the instances' present steps: the next one would run empty
+  // (32,000 elements, the last 40 steps to tMax 968 -> 834 us, a run past its
+  // end 292 -> 160).  The estimate decides nothing else: where it ends too
+  // early, the next graph waits for the host's read.  The timing graph is read
+  // back one at a time.
   const int deep = prof ? 1 : 2;
+  auto to_end = [&](const Clock *ck) {  // most steps to an instance's tMax
+    double most = 0.0;
+    for (int i = 0; i < ni; ++i)
+      if (!ck[i].done) most = std::max(most, (m->inst[i].tmax - ck[i].time) / ck[i].dt);
+    return most;
+  };
   for (int k = 0; k < 2; ++k)
     if (!m->run_ev[k]) CK(cudaEventCreateWithFlags(&m->run_ev[k], cudaEventDisableTiming));
   int rc = FTGPU_OK;
   long long prev = start0;
   long long left = max_steps;  // most steps any running instance will still have
   long long launched = 0, read = 0;
+  double end = to_end(m->h_clock);  // steps behind the launched ones to the last tMax
+  int in_graph[2] = {0, 0};         // steps of the last two graphs
   bool stop = false;
   const Clock *last = m->h_clock;  // the newest clocks read
   while (true) {
-    while (!stop && left > 0 && launched - read < deep) {
+    while (!stop && left > 0 && launched - read < deep && (launched == read || end > 0.01)) {
       // the run's first graph opens with the half-step, the others continue
       const bool open = launched == 0;
       cudaGraphExec_t g = prof ? m->prof_exec : open ? m->chunk_exec : m->cont_exec;
@@ -1562,6 +1575,8 @@ int run_impl(ftgpu_model *m, int max_steps, int *steps_done, bool prof, double *
       CK(cudaEventRecord(m->run_ev[k], m->stream));
       ++launched;
       left -= steps;
+      end -= steps;
+      in_graph[k] = steps;
     }
     if (read == launched) break;
     const int k = (int)(read++ & 1);
@@ -1593,6 +1608,7 @@ int run_impl(ftgpu_model *m, int max_steps, int *steps_done, bool prof, double *
     else if (dterr)
       rc = fail(FTGPU_ERR_DT, "time step below FailureTimeStep");
     stop = rc != FTGPU_OK || all;
+    end = to_end(ck) - (launched == read ? 0 : in_graph[k ^ 1]);
     if (launched == read) left = most;
   }
   if (device_ms) {

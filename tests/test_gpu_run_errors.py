@@ -2,7 +2,9 @@
 the steps taken, the clocks and the fields are those of its 16th step, although
 further graphs may already be queued behind it.  An inverted element, and a step
 below FailureTimeStep in one instance of two (the other has nothing to do with
-it and runs to the same 16th step)."""
+it and runs to the same 16th step).  And a run that is past its end."""
+import time
+
 import numpy as np
 import pytest
 
@@ -94,3 +96,23 @@ def test_failed_step_of_one_instance_ends_the_run_with_its_graph(prec):
     assert c["step"][0] == 16 and 1 <= c["step"][1] < 16
     assert c["done"][0] == 0 and c["done"][1] == 4
     m.close()
+
+
+@pytest.mark.gpu
+def test_a_run_past_its_end_takes_one_empty_graph():
+    """Every graph of a run that is past its tMax is empty: it takes as long as a
+    run of one graph's 16 steps (a second graph ahead of the first one's clocks
+    took 1.6 times that; 1.3 lies between, over medians of 40 in turn)."""
+    mesh = mg.hex_block(40, 40, 20, 40 * H, 40 * H, 20 * H)
+    m = ft.Model(mesh, LAW)
+    m.set_state(time=0.0)
+    m.init_explicit(0.9, 0.0, 20.5 * 0.9 * m.StableTimeStep(np.zeros(mesh["coordinates"].size)))
+    assert m.run(10 ** 6) == 21
+    times = {16: [], 10 ** 6: []}
+    for _ in range(40):
+        for steps, t in times.items():
+            t0 = time.perf_counter()
+            assert m.run(steps) == 0
+            t.append(time.perf_counter() - t0)
+    m.close()
+    assert np.median(times[10 ** 6]) <= 1.3 * np.median(times[16])
