@@ -15,6 +15,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -60,6 +61,42 @@ struct MatP {  // per-part material parameters, precomputed on the host
   float jpow_x;
 };
 
+// The spectral radius of 2E up to which n terms of the Ogden series do (host):
+// the largest r (at most 0.5) whose truncation bound
+// sum_{j > n} |b_j| (3 + 2 r) r^j, b_j = binom(alpha/2 - 1, j), stays below
+// eps r (rounding of the leading term; the 1 + 2 (1 + r) weighs A itself and
+// tr B = tr(A + M + M A)).  The bound's logarithm is convex in x = ln r, so
+// Newton's steps from 0.5 come down to its zero from above, in four to eight;
+// each sum ends where the rest no longer shows (a geometric series bounds it:
+// a ratio is at most r times the larger of one and the last).  bn = |b_n|.
+// 0 (never) for an alpha whose sums leave FP64's range.
+// (Bisections with 400 terms each took half a millisecond a part, and the
+// allocation-free entry forms its part on every call.)
+inline double ogden_radius(double a, int n, double bn, double eps) {
+  if (bn == 0.0) return 0.5;  // (a finite series)
+  double x = std::log(0.5);
+  for (int it = 0; it < 50; ++it) {
+    const double r = std::exp(x);
+    double t = 1.0, s0 = 0.0, s1 = 0.0;  // |b_j| r^(j-1) over bn r^n, its sum and the sum of (j-1) times it
+    for (int j = n; j < n + 400; ++j) {
+      const double c = std::fabs(a / 2.0 - 1.0 - j) / (j + 1.0);
+      t *= j > n ? c * r : c;
+      s0 += t;
+      s1 += j * t;
+      const double g = std::max(c, 1.0) * r;
+      if (g < 1.0 && t * g <= 1e-12 * (1.0 - g) * s0) break;
+    }
+    if (s0 == 0.0) return 0.5;
+    const double h = std::log(bn / eps) + n * x + std::log((3.0 + 2.0 * r) * s0);
+    if (it == 0 && h <= 0.0) return 0.5;
+    if (!std::isfinite(h)) return 0.0;
+    const double d = h / (2.0 * r / (3.0 + 2.0 * r) + s1 / s0);
+    x -= d;
+    if (std::fabs(d) < 1e-10) return std::exp(x);
+  }
+  return 0.0;
+}
+
 // A part's parameters from the reference's property array (host)
 template <class R>
 inline MatP<R> make_matp(int mat, const double *pr) {
@@ -77,37 +114,13 @@ inline MatP<R> make_matp(int mat, const double *pr) {
   if (mat != 6) return q;
   const double a = pr[3];
   q.og_c = R(2.0 * mu / a);
-  const double eps = sizeof(R) == 4 ? 1e-7 : 5e-17;
   double ba = 1.0;
   int step = 0;
   for (int k = 0; k < OgdenSeries<R>::kMax; ++k) {
     ba *= (a / 2.0 - 1.0 - k) / (k + 1.0);
     q.ser_a[k] = R(ba);
-    const int n = k + 1;
-    if (n != OgdenSeries<R>::n[step]) continue;
-    // n terms while the spectral radius of 2E is below r, r the largest (at
-    // most 0.5) whose truncation bound
-    // sum_{j > n} |b_j| (3 + 2 r) r^j stays below eps r (rounding of the leading
-    // term; the 1 + 2 (1 + r) weighs A itself and tr B = tr(A + M + M A))
-    auto tail = [&](double r) {
-      double ca = ba, rk = std::pow(r, n), t = 0.0;
-      for (int j = n; j < n + 400; ++j) {
-        ca *= (a / 2.0 - 1.0 - j) / (j + 1.0);
-        rk *= r;
-        t += std::fabs(ca) * (3.0 + 2.0 * r) * rk;
-      }
-      return t;
-    };
-    double lo = 0.0, hi = 0.5;
-    if (tail(hi) <= eps * hi) {
-      lo = hi;
-    } else {
-      for (int it = 0; it < 60; ++it) {
-        const double mid = 0.5 * (lo + hi);
-        (tail(mid) <= eps * mid ? lo : hi) = mid;
-      }
-    }
-    q.ser_r[step++] = float(lo * (1.0 - 1e-6));
+    if (k + 1 != OgdenSeries<R>::n[step]) continue;
+    q.ser_r[step++] = float(ogden_radius(a, k + 1, std::fabs(ba), sizeof(R) == 4 ? 1e-7 : 5e-17) * (1.0 - 1e-6));
   }
   // FP32: the stress is a difference of terms 1/alpha larger.  For |alpha| >= 2
   // the longer series is as exact as the eigen-decomposition (5e-8 to 9e-8
