@@ -22,8 +22,11 @@
 // every column of du/dxi at a Gauss point costs 3 FMAs, and the B0^T S
 // contraction is accumulated as 7 moment vectors that one inverse transform
 // turns into the 8 nodal forces.  The reference Jacobian's inverse and
-// determinant at each Gauss point come from a table written at set-up (FP32
-// kernels) or from the same transform of the reference coordinates (FP64).
+// determinant at each Gauss point come from a table written at set-up (the
+// allocation-free entry point has none and transforms the reference
+// coordinates).  One thread per element serves the mixed-precision models of
+// more than 20,000 C3D8 elements and all C3D4; the other C3D8 models run on
+// ft_hexgp.cuh, eight lanes per element.
 // Mathematically this is the reference's
 //   F = sum_a x_a (x) dN_a/dX,  f_a = sum_gp w detJ B0_a^T S.
 #pragma once
@@ -74,10 +77,6 @@ __device__ __forceinline__ void cp_async_small(void *smem_dst, const void *gsrc)
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
-
-template <class R> struct Pair;
-template <> struct Pair<float> { using T = float2; };
-template <> struct Pair<double> { using T = double2; };
 
 // Gauss point g of the 2x2x2 rule in the order of GaussQuadrature3D.cpp:17-58
 // (the literal 0.577350269189626 as there): xi > 0 for g in {1,2,5,6},
@@ -264,45 +263,6 @@ __device__ __forceinline__ void prony_consts(const MatP<R> &mp, R dt, R (&pc)[4]
       pc[3] = mp.p[7] * (-d_expm1(-rt2)) / rt2;
     }
   }
-}
-
-template <class R>
-__device__ __forceinline__ R norm3(R x, R y, R z) {
-  return d_sqrt(x * x + y * y + z * z);
-}
-
-// areaHexahedronFace, src/math/Geometry.cpp:29-64 (signed tolerance test kept;
-// the 2x2 quadrature uses (q cD + c1) x (q' cD + c2) = c1 x c2 + q cD x c2 + q' c1 x cD).
-// (FP64 path; the FP32 C3D8 kernels take face_pair_area_max)
-template <class R>
-__device__ __forceinline__ R hex_face_area(const R (&xc)[8][3], int i1, int i2, int i3, int i4) {
-  R cD[3], c1[3], c2[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    R p1 = xc[i1][k], p2 = xc[i2][k], p3 = xc[i3][k], p4 = xc[i4][k];
-    cD[k] = R(0.25) * (p1 - p2 + p3 - p4);
-    c1[k] = R(0.25) * (-p1 + p2 + p3 - p4);
-    c2[k] = R(0.25) * (-p1 - p2 + p3 + p4);
-  }
-  R n0x = c1[1] * c2[2] - c1[2] * c2[1], n0y = c1[2] * c2[0] - c1[0] * c2[2],
-    n0z = c1[0] * c2[1] - c1[1] * c2[0];
-  const R tol = R(1e-6);
-  if (cD[0] < tol && cD[1] < tol && cD[2] < tol) return 4 * norm3(n0x, n0y, n0z);
-  R n1x = cD[1] * c2[2] - cD[2] * c2[1], n1y = cD[2] * c2[0] - cD[0] * c2[2],
-    n1z = cD[0] * c2[1] - cD[1] * c2[0];
-  R n2x = c1[1] * cD[2] - c1[2] * cD[1], n2y = c1[2] * cD[0] - c1[0] * cD[2],
-    n2z = c1[0] * cD[1] - c1[1] * cD[0];
-  const R t = R(0.57735026918962576451);
-  R area = 0;
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      R qj = j ? t : -t, qi = i ? t : -t;
-      area += norm3(n0x + qj * n1x + qi * n2x, n0y + qj * n1y + qi * n2y,
-                    n0z + qj * n1z + qi * n2z);
-    }
-  return area;
 }
 
 // FP32 Gauss loop of the C3D8 element with packed FP32 arithmetic: every
@@ -654,30 +614,15 @@ __device__ __forceinline__ void hex_element_f32(const float (&x)[8][3], const fl
   }
 }
 
-// The same in any precision with the Jacobian rebuilt at each Gauss point (the
-// allocation-free entry point, which keeps no table).
-template <class R, int MAT, bool GP>
-__device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][3],
-                                            const MatP<R> &mp, const R (&pc)[4],
-                                            const R (&a0)[3], R *hist, int pass, R (&f)[8][3],
-                                            R &le, int &bad, const ElemArgs<R> &A, long long gpo) {
-  const bool dt_only = pass == kPassDt;
-  R vol = 0;
+// The nodal forces alone, in any precision, with the Jacobian rebuilt at each
+// Gauss point: the allocation-free entry point, which keeps no table and takes
+// the laws without history.
+template <class R, int MAT>
+__device__ __forceinline__ void hex_force(const R (&x)[8][3], const R (&u)[8][3], const MatP<R> &mp,
+                                          R (&f)[8][3], int &bad) {
+  static_assert(hist_comps(MAT) == 0, "no history to read or write here");
+  const R a0[3] = {1, 0, 0}, pc[4] = {0, 0, 0, 0};
   R m[7][3];
-  R amax;
-  {
-    R xc[8][3];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) xc[a][d] = x[a][d] + u[a][d];
-    amax = hex_face_area(xc, 0, 1, 2, 3);
-    amax = fmax(amax, hex_face_area(xc, 4, 5, 6, 7));
-    amax = fmax(amax, hex_face_area(xc, 0, 3, 7, 4));
-    amax = fmax(amax, hex_face_area(xc, 1, 2, 6, 5));
-    amax = fmax(amax, hex_face_area(xc, 0, 1, 5, 4));
-    amax = fmax(amax, hex_face_area(xc, 3, 2, 6, 7));
-  }
   R hx[7][3], hu[7][3];
   hex_hadamard(x, hx);
   hex_hadamard(u, hu);
@@ -720,32 +665,9 @@ __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][
       for (int j = 0; j < 3; ++j)
         D[i][j] = H[i][0] * Q[j][0] + H[i][1] * Q[j][1] + H[i][2] * Q[j][2];
     const R Jm1 = jm1_of(D);
-    // det(dx/dxi) = det A det F
-    vol += (1 + Jm1) * detA;
-    if (dt_only) continue;
     if (!(Jm1 > R(-1)) || !(detA != 0)) bad = 1;
-    const long long sg = gpo - A.gpbase + g;  // Gauss point within the group
-    if (MAT == 7 && pass == kPassSurrogateFeatures) {
-      write_surrogate_features(D, a0, A.law, A.surr_x + sg * kMlpIn);
-      continue;
-    }
-    const float *sy = (MAT == 7 && A.surr_y) ? A.surr_y + sg * kMlpOut : nullptr;
-    Sym6<R> S = stress_at<R, MAT>(mp, D, Jm1, a0, hist, pc, sy, A.law, HistGlobal<R>{hist},
-                                  PartAt<R>{&mp});
-    if (GP) {
-      long long q = gpo + g;
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) A.gpF[9 * q + i + 3 * j] = double((i == j ? R(1) : R(0)) + D[i][j]);
-      A.gpJ[q] = double(1 + Jm1);
-      A.gpS[6 * q + 0] = S.xx;
-      A.gpS[6 * q + 1] = S.yy;
-      A.gpS[6 * q + 2] = S.zz;
-      A.gpS[6 * q + 3] = S.yz;
-      A.gpS[6 * q + 4] = S.xz;
-      A.gpS[6 * q + 5] = S.xy;
-    }
+    const Sym6<R> S = stress_at<R, MAT>(mp, D, Jm1, a0, nullptr, pc, nullptr, SurrogateLaw{},
+                                        HistGlobal<R>{nullptr}, PartAt<R>{&mp});
     // w detJ B0^T S with w = 1: P = det A F S = det A (S + D S), Gm = P A^{-1}
     const R sxx = detA * S.xx, syy = detA * S.yy, szz = detA * S.zz, syz = detA * S.yz,
             sxz = detA * S.xz, sxy = detA * S.xy;
@@ -770,26 +692,22 @@ __device__ __forceinline__ void hex_element(const R (&x)[8][3], const R (&u)[8][
       m[6][i] += ez * g0 + xz * g1 + xe * g2;
     }
   }
-  le = vol / amax;
-  if (pass == kPassForce) {
-    // inverse transform: f_a = 1/8 sum_k sign_k(a) m_k
+  // inverse transform: f_a = 1/8 sum_k sign_k(a) m_k
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const R q = R(0.125);
-      R t1 = m[0][i] + m[6][i], t2 = m[0][i] - m[6][i], t3 = m[3][i] + m[4][i],
-        t4 = m[3][i] - m[4][i];
-      R Pmm = t1 - t3, Ppp = t1 + t3, Ppm = t2 + t4, Pmp = t2 - t4;
-      R r1 = m[1][i] + m[2][i], r2 = m[1][i] - m[2][i];
-      R Qmm = m[5][i] - r1, Qpp = m[5][i] + r1, Qpm = r2 - m[5][i], Qmp = -r2 - m[5][i];
-      f[0][i] = q * (Qmm - Pmm);
-      f[1][i] = q * (Qmm + Pmm);
-      f[2][i] = q * (Qpm + Ppm);
-      f[3][i] = q * (Qpm - Ppm);
-      f[4][i] = q * (Qmp - Pmp);
-      f[5][i] = q * (Qmp + Pmp);
-      f[6][i] = q * (Qpp + Ppp);
-      f[7][i] = q * (Qpp - Ppp);
-    }
+  for (int i = 0; i < 3; ++i) {
+    const R q = R(0.125);
+    R t1 = m[0][i] + m[6][i], t2 = m[0][i] - m[6][i], t3 = m[3][i] + m[4][i], t4 = m[3][i] - m[4][i];
+    R Pmm = t1 - t3, Ppp = t1 + t3, Ppm = t2 + t4, Pmp = t2 - t4;
+    R r1 = m[1][i] + m[2][i], r2 = m[1][i] - m[2][i];
+    R Qmm = m[5][i] - r1, Qpp = m[5][i] + r1, Qpm = r2 - m[5][i], Qmp = -r2 - m[5][i];
+    f[0][i] = q * (Qmm - Pmm);
+    f[1][i] = q * (Qmm + Pmm);
+    f[2][i] = q * (Qpm + Ppm);
+    f[3][i] = q * (Qpm - Ppm);
+    f[4][i] = q * (Qmp - Pmp);
+    f[5][i] = q * (Qmp + Pmp);
+    f[6][i] = q * (Qpp + Ppp);
+    f[7][i] = q * (Qpp - Ppp);
   }
 }
 

@@ -41,7 +41,7 @@ static double *g_noalloc_ptr[kNoAllocMaxDevices];
 static int *g_noalloc_bad_ptr[kNoAllocMaxDevices];
 static std::mutex g_noalloc_mu;
 
-// One thread per element: the C3D8 element force of ft_elem.cuh in FP64,
+// One thread per element: hex_force of ft_elem.cuh in FP64,
 // reading coordinates/displacements straight from the caller's AoS arrays.
 template <int MAT>
 __global__ void k_noalloc_hex(int nelements, const double *X, const int *conn, const double *u,
@@ -58,13 +58,9 @@ __global__ void k_noalloc_hex(int nelements, const double *X, const int *conn, c
       uu[a][d] = u[3 * n + d];
     }
   }
-  ElemArgs<double> none;
-  memset(&none, 0, sizeof(none));
-  const double pc[4] = {0, 0, 0, 0};
-  const double a0[3] = {1, 0, 0};
-  double f[8][3], le;
+  double f[8][3];
   int bad = 0;
-  hex_element<double, MAT, false>(x, uu, mp, pc, a0, nullptr, kPassForce, f, le, bad, none, 0);
+  hex_force<double, MAT>(x, uu, mp, f, bad);
   if (bad) atomicOr(bad_out, 1);
 #pragma unroll
   for (int a = 0; a < 8; ++a)
