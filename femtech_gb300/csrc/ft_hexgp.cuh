@@ -535,8 +535,14 @@ __global__ void __launch_bounds__(kHexGpThreads) k_hexgp_geo(const ElemArgs<R> A
   if (bad) atomicOr(A.err, bad);
 }
 
-static_assert(8 * (8 * kMaxLocalNodes + 24 * 128) <= 48 * 1024,
+// The launches ask for no more than the default 48 KB: the largest patches of
+// each precision with the kernels' own static arrays (the injury extremes',
+// the block minima and the bounds' cut: 576 bytes)
+constexpr size_t kHexGpStatic = 1024;
+static_assert(hexgp_smem_bytes<double>(128) + kHexGpStatic <= 48 * 1024,
               "an FP64 patch of 128 elements fits the default shared memory");
+static_assert(hexgp_smem_bytes<float>(kMaxPatchElems) + kHexGpStatic <= 48 * 1024,
+              "the largest FP32 patch fits the default shared memory");
 
 // The launcher of one precision's instantiations (ft_hexgp_f32.cu, _f64.cu)
 template <class R, int MAT>

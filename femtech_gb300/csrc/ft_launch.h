@@ -76,7 +76,7 @@ int launch_hexgp_geo(int nblocks, cudaStream_t s, const ElemArgs<double> &A, dou
 // corner forces in shared memory
 inline int hexgp_threads(int PE) { return PE >= 32 ? 256 : (8 * PE + 31) / 32 * 32; }
 template <class R>
-inline size_t hexgp_smem_bytes(int PE) {
+constexpr size_t hexgp_smem_bytes(int PE) {
   return sizeof(R) * (8 * (size_t)kMaxLocalNodes + 24 * (size_t)PE) +
          (sizeof(R) == 8 ? 12 * (size_t)PE : 0);
 }
