@@ -858,7 +858,6 @@ int download_state3(ftgpu_model *m, DBuf *const d[3], double *const h[3]) {
   return 0;
 }
 
-// AoS [3N] host -> SoA [3][N] device (h == NULL: zero)
 // Displacements of one primitive (null: zero) into u and the patch slots.
 // Up to kIoDirect bytes the kernels read and write page-locked memory of the
 // model in place, and the caller's arrays are copied by the host; above, the

@@ -60,7 +60,7 @@ inline int launch_strain<double>(int etype, int nblocks, int threads, size_t sme
   return launch_strain_f64(etype, nblocks, threads, smem, s, A, Eout);
 }
 
-// Setup pass of an FP32 C3D8 group (k_elem_geo): the Gauss points' inverse
+// Setup pass of a C3D8 group that k_elem runs (k_elem_geo): the Gauss points' inverse
 // reference Jacobians and determinants into geo ([nelem/32][20][32][4]).
 // Returns a cudaError_t value.
 int launch_geo_f32(int nblocks, cudaStream_t s, const ElemArgs<float> &A, float *geo);
