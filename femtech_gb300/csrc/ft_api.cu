@@ -89,12 +89,17 @@ struct DBuf {
 // contiguous share, through their own page-locked piece and stream
 // (element_strain of 238k elements, 23 MB: 2.7 -> 1.05 ms with the results in
 // the caller's order from the device).  Page-locked destinations and results
-// below 4 MB are copied directly (2.9 MB: 0.15 ms, threads 0.55 ms).  The buffers belong to one model (one
-// host thread drives it) and go with it: 8 x 512 KB.
+// below 4 MB are copied directly (2.9 MB: 0.15 ms, threads 0.55 ms).  Results
+// of several parts, which lie together on the device, come in one copy up to
+// 512 KB and are parted by the host: every further copy costs 10 us
+// (element_strain, four parts, 20 KB 83 -> 54 us, 205 KB 94 -> 69, 360 KB 97 ->
+// 81, 750 KB 107 / 112; injury, three, 2 KB 50 -> 21).  The buffers belong to
+// one model (one host thread drives it) and go with it: 9 x 512 KB.
 struct HostDrain {
   static constexpr int kMax = 8;
-  static constexpr size_t kPiece = 512 << 10, kDirect = 4 << 20;
+  static constexpr size_t kPiece = 512 << 10, kDirect = 4 << 20, kJoin = 512 << 10;
   char *pin = nullptr;
+  std::vector<char> joined;
   cudaStream_t st[kMax] = {};
   HostDrain() = default;
   HostDrain(const HostDrain &) = delete;
@@ -109,8 +114,29 @@ struct HostDrain {
     const void *src;
     size_t bytes;
   };
-  // The parts' device data are complete when everything queued on `after` is.
+  // The parts' device data (of one buffer) are complete when everything queued
+  // on `after` is.
   int copy(int device, cudaStream_t after, const Part *parts, int n) {
+    if (n > 1) {
+      const char *lo = nullptr, *hi = nullptr;
+      int wanted = 0;
+      for (int i = 0; i < n; ++i) {
+        if (!parts[i].dst || !parts[i].bytes) continue;
+        const char *s = (const char *)parts[i].src;
+        lo = wanted ? std::min(lo, s) : s;
+        hi = wanted ? std::max(hi, s + parts[i].bytes) : s + parts[i].bytes;
+        ++wanted;
+      }
+      if (wanted > 1 && (size_t)(hi - lo) <= kJoin) {
+        if (joined.size() < (size_t)(hi - lo)) joined.resize(hi - lo);
+        CK(cudaMemcpyAsync(joined.data(), lo, hi - lo, cudaMemcpyDeviceToHost, after));
+        CK(cudaStreamSynchronize(after));
+        for (int i = 0; i < n; ++i)
+          if (parts[i].dst)
+            memcpy(parts[i].dst, joined.data() + ((const char *)parts[i].src - lo), parts[i].bytes);
+        return 0;
+      }
+    }
     size_t total = 0;
     bool direct = true;
     for (int i = 0; i < n; ++i) {
@@ -951,12 +977,14 @@ __global__ void k_principal_strain(const double *E6, const int *order, long long
   shear[el] = 0.5 * (mx - mn);
 }
 
-// The listed elements' flags (with the last step's percentile lists) and last
-// MPS in the caller's order
+// The record, and the listed elements' flags (with the last step's percentile
+// lists) and last MPS in the caller's order
 template <class R>
-__global__ void k_injury_out(const InjuryRun *run, const uint8_t *flags, const R *ps, const R *psxsr,
-                             const int *upos, int n, double *ps_out, int *flags_out) {
+__global__ void k_injury_out(const InjuryState *state, const InjuryRun *run, const uint8_t *flags,
+                             const R *ps, const R *psxsr, const int *upos, int n,
+                             InjuryState *state_out, double *ps_out, int *flags_out) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c == 0) *state_out = *state;
   if (c >= n) return;
   const int j = upos[c];
   flags_out[j] = inj_list_flags<R>(run, flags[c], ps[c], psxsr[c]);
@@ -2195,23 +2223,29 @@ int ftgpu_set_injury(ftgpu_model *m, int n, const int *element_ids) {
 int ftgpu_get_injury(ftgpu_model *m, ftgpu_injury *out, int *flags, double *ps) {
   if (!m || !m->injury_on) return fail(FTGPU_ERR_STATE, "injury criteria are off");
   CK(cudaSetDevice(m->device));
-  CK(cudaStreamSynchronize(m->stream));
-  if (out) CK(cudaMemcpy(out, m->inj_state.p, sizeof(ftgpu_injury), cudaMemcpyDeviceToHost));
+  if (!flags && !ps) {
+    if (!out) return FTGPU_OK;
+    CK(cudaStreamSynchronize(m->stream));
+    CK(cudaMemcpy(out, m->inj_state.p, sizeof(ftgpu_injury), cudaMemcpyDeviceToHost));
+    return FTGPU_OK;
+  }
   const int n = m->inj_n;  // device arrays are in group order: back to the caller's
-  if (!flags && !ps) return FTGPU_OK;
-  CKI(m->inj_out.bytes >= n * 12ull ? 0 : m->inj_out.alloc(n * 12ull));
-  double *po = m->inj_out.as<double>();
+  const size_t need = sizeof(InjuryState) + n * 12ull;
+  CKI(m->inj_out.bytes >= need ? 0 : m->inj_out.alloc(need));
+  InjuryState *so = m->inj_out.as<InjuryState>();
+  double *po = reinterpret_cast<double *>(so + 1);
   int *fo = reinterpret_cast<int *>(po + n);
   auto collect = [&](auto real) {
     typedef decltype(real) R;
     k_injury_out<R><<<(n + 255) / 256, 256, 0, m->stream>>>(
-        m->inj_run.as<InjuryRun>(), m->inj_flags.as<uint8_t>(), m->inj_ps_old.as<R>(),
-        m->inj_psxsr.as<R>(), m->inj_upos_d.as<int>(), n, po, fo);
+        m->inj_state.as<InjuryState>(), m->inj_run.as<InjuryRun>(), m->inj_flags.as<uint8_t>(),
+        m->inj_ps_old.as<R>(), m->inj_psxsr.as<R>(), m->inj_upos_d.as<int>(), n, so, po, fo);
   };
   is_fp64(m) ? collect(0.0) : collect(0.f);
   CK(cudaGetLastError());
-  const HostDrain::Part parts[] = {{flags, fo, n * sizeof(int)}, {ps, po, n * sizeof(double)}};
-  return m->drain.copy(m->device, m->stream, parts, 2);
+  const HostDrain::Part parts[] = {{out, so, sizeof(InjuryState)}, {ps, po, n * sizeof(double)},
+                                   {flags, fo, n * sizeof(int)}};
+  return m->drain.copy(m->device, m->stream, parts, 3);
 }
 
 int ftgpu_set_energy(ftgpu_model *m, int enable) {
