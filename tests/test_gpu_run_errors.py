@@ -102,7 +102,7 @@ def test_failed_step_of_one_instance_ends_the_run_with_its_graph(prec):
 def test_a_run_past_its_end_takes_one_empty_graph():
     """Every graph of a run that is past its tMax is empty: it takes as long as a
     run of one graph's 16 steps (a second graph ahead of the first one's clocks
-    took 1.6 times that; 1.3 lies between, over medians of 40 in turn)."""
+    took 1.6 times that; 1.3 lies between, the least of 40 each in turn)."""
     mesh = mg.hex_block(40, 40, 20, 40 * H, 40 * H, 20 * H)
     m = ft.Model(mesh, LAW)
     m.set_state(time=0.0)
@@ -115,4 +115,4 @@ def test_a_run_past_its_end_takes_one_empty_graph():
             assert m.run(steps) == 0
             t.append(time.perf_counter() - t0)
     m.close()
-    assert np.median(times[10 ** 6]) <= 1.3 * np.median(times[16])
+    assert min(times[10 ** 6]) <= 1.3 * min(times[16])
